@@ -116,7 +116,7 @@ typedef struct sdfgpu_stats {
   double ms_vote;                 /* vote + adaptive rays + winding */
   int64_t certified_nodes;        /* learned radius: nodes whose bounded search certified the result */
   double radius_loss;             /* final training loss of the radius network */
-  int64_t bvh_visits;             /* LBVH nodes visited by the unbounded search (one per warp and node) */
+  int64_t bvh_visits;             /* LBVH nodes opened by the unbounded search (one per warp and node) */
   double ms_train;                /* device time of the last sdfgpu_train_radius (coarse grid + training) */
   int64_t train_launches;         /* kernels of this library launched by the last sdfgpu_train_radius */
   int64_t sign_band_reruns;       /* axis-row ray-triangle tests decided in FP64 (FP32 result inside its error band) */

@@ -69,49 +69,68 @@ __device__ __forceinline__ float obox_d2(float3 p, const OBox& o) {
   return fmaf(u0, u0, fmaf(u1, u1, u2 * u2));
 }
 
-// Leaf-ordered FP32 record of one triangle for the unbounded searches (mesh-local; every field
-// rounded once from its FP64 value): vertex a, edges e0 = b - a and e1 = c - a, the inverse squared
-// lengths of e0, e1 and c - b, the unit normal n and, for each edge, the unit in-plane normal m_k
-// pointing into the triangle with its offset o_k (a point of the plane lies inside when
-// (p - a).m_k >= o_k for k = 0, 1, 2).  A triangle without area has m_k = 0 and o_k = 1 and
-// reduces to its three edges.
+// Leaf-ordered FP32 record of one triangle for the unbounded searches (mesh-local; every field rounded
+// once from its FP64 value): vertex a, the unit normal n and, for the edges a -> b, b -> c and c -> a,
+// the unit in-plane normals m_k pointing into the triangle and the lengths L_k.  With w = p - a the
+// in-plane distances of p inside the edge lines are f0 = w.m0, f1 = w.m1 - o1, f2 = w.m2, and the edge
+// directions are m_k x n.  A triangle without area is its longest edge: a, m0, n and L0 describe that
+// edge's line (n and m0 any normals of it), and the other two edges lie kFlat away (L2 < 0 marks it).
+constexpr float kFlat = 1.0e18f;
+constexpr int kWeakTri = 1 << 30;  // above every triangle index (at most 2^29)
 struct __align__(16) LeafTri {
-  float4 a;   // a.xyz, 1 / |e0|^2
-  float4 e0;  // e0.xyz, 1 / |e1|^2
-  float4 e1;  // e1.xyz, 1 / |c - b|^2
-  float4 n;   // n.xyz, triangle index (int bits)
-  float4 m0;  // edge a -> b: m0.xyz, o0 = 0
-  float4 m1;  // edge b -> c: m1.xyz, o1 = e0.m1
-  float4 m2;  // edge c -> a: m2.xyz, o2 = e1.m2
+  float4 a;   // a.xyz, triangle index | kWeakTri when it is not fit for FP32 decisions (int bits)
+  float4 n;   // n.xyz, L0
+  float4 m0;  // m0.xyz, L1
+  float4 m1;  // m1.xyz, o1
+  float4 m2;  // m2.xyz, L2
 };
 
-__device__ __forceinline__ float clamp01(float t) { return fminf(fmaxf(t, 0.f), 1.f); }
+// The records of all sorted leaves as five planes of float4 (the fields of LeafTri in order, n per
+// plane): the searches read runs of consecutive leaves, a lane per leaf.
+struct LeafTris {
+  const float4* p;
+  int64_t n;
+  __device__ __forceinline__ float4 at(int field, int leaf) const { return p[field * n + leaf]; }
+  __device__ __forceinline__ LeafTri load(int leaf) const {
+    return {at(0, leaf), at(1, leaf), at(2, leaf), at(3, leaf), at(4, leaf)};
+  }
+};
 
-// Squared distance from p to the triangle of T, without division or branch: the smallest squared
-// distance to the three edges, and the squared plane distance when p projects inside.  Every
-// rounding is relative to |w| <= d + |e| (w = p - a, d the distance, e the longest edge) or to
-// |e|, and the inside test compares physical distances to the edge lines (no barycentric
-// division), so for inputs within E of the origin the result is within about 7e-7 E + 4e-7 d of
-// the exact distance to the FP64 triangle, whatever its shape -- at least 5x inside the FP32 band
-// of the unbounded searches (4e-6 E + 4e-6 d).
-__device__ __forceinline__ float leaf_d2(float3 p, const LeafTri& T) {
-  const float wx = p.x - T.a.x, wy = p.y - T.a.y, wz = p.z - T.a.z;
-  const float t0 = clamp01(fmaf(wx, T.e0.x, fmaf(wy, T.e0.y, wz * T.e0.z)) * T.a.w);
-  const float t1 = clamp01(fmaf(wx, T.e1.x, fmaf(wy, T.e1.y, wz * T.e1.z)) * T.e0.w);
-  const float q0x = fmaf(-t0, T.e0.x, wx), q0y = fmaf(-t0, T.e0.y, wy), q0z = fmaf(-t0, T.e0.z, wz);
-  const float q1x = fmaf(-t1, T.e1.x, wx), q1y = fmaf(-t1, T.e1.y, wy), q1z = fmaf(-t1, T.e1.z, wz);
-  const float e2x = T.e1.x - T.e0.x, e2y = T.e1.y - T.e0.y, e2z = T.e1.z - T.e0.z;  // c - b
-  const float wbx = wx - T.e0.x, wby = wy - T.e0.y, wbz = wz - T.e0.z;              // p - b
-  const float t2 = clamp01(fmaf(wbx, e2x, fmaf(wby, e2y, wbz * e2z)) * T.e1.w);
-  const float q2x = fmaf(-t2, e2x, wbx), q2y = fmaf(-t2, e2y, wby), q2z = fmaf(-t2, e2z, wbz);
-  float d2 = fminf(fmaf(q0x, q0x, fmaf(q0y, q0y, q0z * q0z)),
-                   fminf(fmaf(q1x, q1x, fmaf(q1y, q1y, q1z * q1z)), fmaf(q2x, q2x, fmaf(q2y, q2y, q2z * q2z))));
-  const bool in0 = fmaf(wx, T.m0.x, fmaf(wy, T.m0.y, wz * T.m0.z)) >= T.m0.w;
-  const bool in1 = fmaf(wx, T.m1.x, fmaf(wy, T.m1.y, wz * T.m1.z)) >= T.m1.w;
-  const bool in2 = fmaf(wx, T.m2.x, fmaf(wy, T.m2.y, wz * T.m2.z)) >= T.m2.w;
-  const float dp = fmaf(wx, T.n.x, fmaf(wy, T.n.y, wz * T.n.z));
-  if (in0 && in1 && in2) d2 = fminf(d2, dp * dp);
-  return d2;
+// The triangle of T as seen from points p0 + d: its plane distance, the distances inside its three edge
+// lines and the coordinates along its edges as linear functions of d.
+struct LeafView {
+  float3 n, m0, m1, m2, u0, u1, u2;
+  float bn, f0, f1, f2, g0, g1, g2;  // values at p0
+  float L0, L1, L2;
+};
+__device__ __forceinline__ LeafView leaf_view(const LeafTri& T, float3 p0) {
+  LeafView V;
+  V.n = f3(T.n); V.m0 = f3(T.m0); V.m1 = f3(T.m1); V.m2 = f3(T.m2);
+  V.L0 = T.n.w; V.L1 = T.m0.w; V.L2 = T.m2.w;
+  V.u0 = cross3f(V.m0, V.n); V.u1 = cross3f(V.m1, V.n); V.u2 = cross3f(V.m2, V.n);
+  const float3 w = p0 - f3(T.a);
+  V.bn = dot3f(w, V.n);
+  V.f0 = dot3f(w, V.m0); V.f1 = dot3f(w, V.m1) - T.m1.w; V.f2 = dot3f(w, V.m2);
+  V.g0 = dot3f(w, V.u0); V.g1 = dot3f(w, V.u1) - V.L0 * dot3f(V.u0, V.u1); V.g2 = dot3f(w, V.u2) + V.L2;
+  return V;
+}
+// Squared distance from p0 + d to the triangle, without division or branch: the plane distance and the
+// in-plane one.  With e the squared in-plane distance to the nearest edge, the latter is e outside and
+// e - s^2 = 0 inside, where s, the smallest distance inside an edge line, is that same distance.  (A
+// point beyond a needle's tip that the rounding puts inside both lines has s far below its distance to
+// the edges, so the difference stays its distance whatever the triangle's shape.)  Every rounding is
+// relative to |p0 - a| + |d| + the edges.
+__device__ __forceinline__ float view_d2(const LeafView& V, float3 d) {
+  auto at = [&](float3 g, float c) { return fmaf(g.x, d.x, fmaf(g.y, d.y, fmaf(g.z, d.z, c))); };
+  auto edge = [](float f, float g, float L) {
+    const float t = fmaxf(fmaxf(-g, g - L), 0.f);
+    return fmaf(t, t, __fmul_rn(f, f));
+  };
+  const float f0 = at(V.m0, V.f0), f1 = at(V.m1, V.f1), f2 = at(V.m2, V.f2), h = at(V.n, V.bn);
+  const float e = fminf(fminf(edge(f0, at(V.u0, V.g0), V.L0), edge(f1, at(V.u1, V.g1), V.L1)),
+                        edge(f2, at(V.u2, V.g2), V.L2));
+  const float s = fmaxf(fminf(fminf(f0, f1), f2), 0.f);
+  return fmaf(h, h, fmaxf(__fsub_rn(e, __fmul_rn(s, s)), 0.f));  // inside e is fl(s s): exactly 0
 }
 
 // Squared distance from p to the box [lo, hi].

@@ -242,15 +242,16 @@ __global__ void k_single_root(const float4* __restrict__ box32, BNode* nodes, in
 // record, both of the triangle at each sorted leaf.  The record's fields are computed in FP64 from
 // the triangle's vertices (mesh-local) and rounded once.
 __global__ void k_leaf_order(const int32_t* __restrict__ leaf_prim, const float4* __restrict__ v32,
+                             const float4* __restrict__ c32,
                              const TriRec64* __restrict__ rec, int n, double cx, double cy, double cz,
-                             float4* __restrict__ lv32, LeafTri* __restrict__ ltri) {
+                             float4* __restrict__ lv32, float4* __restrict__ ltri) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int prim = leaf_prim[i];
     lv32[3 * i] = v32[3 * prim];
     lv32[3 * i + 1] = v32[3 * prim + 1];
     lv32[3 * i + 2] = v32[3 * prim + 2];
+    const int id = c32[prim].w != 0.f ? prim : (prim | kWeakTri);
     const double* v = rec[prim].v;
-    const double ax = v[0] - cx, ay = v[1] - cy, az = v[2] - cz;
     const double e0[3] = {v[3] - v[0], v[4] - v[1], v[5] - v[2]};
     const double e1[3] = {v[6] - v[0], v[7] - v[1], v[8] - v[2]};
     const double e2[3] = {v[6] - v[3], v[7] - v[4], v[8] - v[5]};
@@ -260,9 +261,7 @@ __global__ void k_leaf_order(const int32_t* __restrict__ leaf_prim, const float4
     const double nx = e0[1] * e1[2] - e0[2] * e1[1], ny = e0[2] * e1[0] - e0[0] * e1[2], nz = e0[0] * e1[1] - e0[1] * e1[0];
     const double nn = nx * nx + ny * ny + nz * nz;
     LeafTri T;
-    T.a = make_float4((float)ax, (float)ay, (float)az, (float)(1.0 / l0));
-    T.e0 = make_float4((float)e0[0], (float)e0[1], (float)e0[2], (float)(1.0 / l1));
-    T.e1 = make_float4((float)e1[0], (float)e1[1], (float)e1[2], (float)(1.0 / l2));
+    T.a = make_float4((float)(v[0] - cx), (float)(v[1] - cy), (float)(v[2] - cz), __int_as_float(id));
     if (nn > 1e-20 * l0 * l1) {
       const double rn = 1.0 / sqrt(nn), un[3] = {nx * rn, ny * rn, nz * rn};
       // inward in-plane edge normals: n x (edge direction), edges a->b, b->c, c->a
@@ -276,19 +275,35 @@ __global__ void k_leaf_order(const int32_t* __restrict__ leaf_prim, const float4
         const double r = 1.0 / sqrt(mx * mx + my * my + mz * mz);
         m[k][0] = mx * r; m[k][1] = my * r; m[k][2] = mz * r;
       }
-      T.n = make_float4((float)un[0], (float)un[1], (float)un[2], __int_as_float(prim));
-      T.m0 = make_float4((float)m[0][0], (float)m[0][1], (float)m[0][2], 0.f);
+      T.n = make_float4((float)un[0], (float)un[1], (float)un[2], (float)sqrt(l0));
+      T.m0 = make_float4((float)m[0][0], (float)m[0][1], (float)m[0][2], (float)sqrt(l2));
       T.m1 = make_float4((float)m[1][0], (float)m[1][1], (float)m[1][2],
                          (float)(e0[0] * m[1][0] + e0[1] * m[1][1] + e0[2] * m[1][2]));
-      T.m2 = make_float4((float)m[2][0], (float)m[2][1], (float)m[2][2],
-                         (float)(e1[0] * m[2][0] + e1[1] * m[2][1] + e1[2] * m[2][2]));
-    } else {  // no area: the edges alone
-      T.n = make_float4(0.f, 0.f, 0.f, __int_as_float(prim));
-      T.m0 = make_float4(0.f, 0.f, 0.f, 1.f);
-      T.m1 = make_float4(0.f, 0.f, 0.f, 1.f);
-      T.m2 = make_float4(0.f, 0.f, 0.f, 1.f);
+      T.m2 = make_float4((float)m[2][0], (float)m[2][1], (float)m[2][2], (float)sqrt(l1));
+    } else {  // no area: the longest edge (see LeafTri)
+      const int k = l0 >= l1 && l0 >= l2 ? 0 : (l1 >= l2 ? 2 : 1);  // edge a->b, c->a or b->c
+      const double* d = k == 0 ? e0 : (k == 1 ? e2 : e1);
+      const double len = sqrt(k == 0 ? l0 : (k == 1 ? l2 : l1));
+      double u[3] = {1.0, 0.0, 0.0};
+      if (len > 0.0)
+        for (int q = 0; q < 3; ++q) u[q] = d[q] / len;
+      const int s = k == 1 ? 3 : 0;  // from b along b->c, else from a
+      // n: the coordinate axis least along u, made normal to it
+      const int j = fabs(u[0]) <= fabs(u[1]) && fabs(u[0]) <= fabs(u[2]) ? 0 : (fabs(u[1]) <= fabs(u[2]) ? 1 : 2);
+      double un[3];
+      for (int q = 0; q < 3; ++q) un[q] = (q == j ? 1.0 : 0.0) - u[j] * u[q];
+      const double rn = 1.0 / sqrt(un[0] * un[0] + un[1] * un[1] + un[2] * un[2]);
+      for (int q = 0; q < 3; ++q) un[q] *= rn;
+      T.a = make_float4((float)(v[s] - cx), (float)(v[s + 1] - cy), (float)(v[s + 2] - cz), __int_as_float(id));
+      T.n = make_float4((float)un[0], (float)un[1], (float)un[2], (float)len);
+      T.m0 = make_float4((float)(un[1] * u[2] - un[2] * u[1]), (float)(un[2] * u[0] - un[0] * u[2]),
+                         (float)(un[0] * u[1] - un[1] * u[0]), 0.f);
+      T.m1 = make_float4(0.f, 0.f, 0.f, kFlat);
+      T.m2 = make_float4(0.f, 0.f, 0.f, -kFlat);
     }
-    ltri[i] = T;
+    const float4 f[5] = {T.a, T.n, T.m0, T.m1, T.m2};
+#pragma unroll
+    for (int k = 0; k < 5; ++k) ltri[(int64_t)k * n + i] = f[k];
   }
 }
 
@@ -608,10 +623,10 @@ int mesh_upload_and_build(sdfgpu_ctx* ctx, const double* X, int64_t nnp, const i
     SDF_KERNEL(ctx);
   }
   float4* lv32;
-  LeafTri* ltri;
+  float4* ltri;  // LeafTris: five planes
   SDF_TRY(scratch_t(ctx, "lv32", (size_t)n * 3, &lv32));
-  SDF_TRY(scratch_t(ctx, "ltri", (size_t)n, &ltri));
-  k_leaf_order<<<grid_for(n, 256), 256, 0, sb>>>(leaf_prim, v32, rec, n, M.center[0], M.center[1], M.center[2], lv32,
+  SDF_TRY(scratch_t(ctx, "ltri", (size_t)n * 5, &ltri));
+  k_leaf_order<<<grid_for(n, 256), 256, 0, sb>>>(leaf_prim, v32, c32, rec, n, M.center[0], M.center[1], M.center[2], lv32,
                                                  ltri);
   SDF_KERNEL(ctx);
   // the rays and the 3-nearest-vertex fallback need only the tree; the unbounded searches wait for

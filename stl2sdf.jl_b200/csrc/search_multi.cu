@@ -21,18 +21,18 @@ template <int kMode>
 __global__ void __launch_bounds__(kUnbThreads, 4)
     k_unbounded_multi(const UnbArgs* __restrict__ items, const int64_t* __restrict__ off, int count,
                       unsigned long long* next, const int64_t* __restrict__ list, const unsigned long long* list_n,
-                      int64_t* counters) {
+                      int64_t* counters, int* __restrict__ spills) {
   constexpr bool kRadius = kMode == kUnbRadius, kListed = kMode == kUnbListed;
-  __shared__ int s_stack[kUnbWarps][kWarpStack];
+  __shared__ WideShared s_wide[kUnbWarps];
   // kRadius: each lane's radius and the warp's certified / fallback counts live in shared memory,
   // so the traversal loop keeps the plain search's registers
   __shared__ float s_r[kRadius ? kUnbThreads : 1];
   __shared__ unsigned s_cf[kRadius ? kUnbWarps : 1][2];
-  __shared__ int s_keep_t[kKeep * kUnbThreads];
-  __shared__ float s_keep_d[kKeep * kUnbThreads];
+  __shared__ int s_keep[kKeep * kUnbThreads];
   __shared__ __align__(16) unsigned char s_args_raw[kUnbWarps][sizeof(UnbArgs)];  // the warp's item (raw: no constructor)
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const UnbArgs& args = *reinterpret_cast<const UnbArgs*>(s_args_raw[w]);
+  int* spill = spills + (int64_t)(blockIdx.x * kUnbWarps + w) * kWideSpill;
   uint32_t fp64 = 0, errs = 0, visits = 0;  // per-thread statistics (far below 2^32)
   if (kRadius && lane == 0) s_cf[w][0] = s_cf[w][1] = 0u;
   const int64_t total = kListed ? (int64_t)*list_n : off[count];
@@ -60,7 +60,6 @@ __global__ void __launch_bounds__(kUnbThreads, 4)
     }
     const UnbArgs& A = args;
     const GridP& g = A.g;
-    int* stack = s_stack[w];
     const int64_t brick = gw - off[lo];
 #include "unb_brick.inc"
   }
@@ -91,13 +90,15 @@ void plan_set_redo(DistPlan& Pl, int64_t* redo, unsigned long long* redo_n, int6
   std::memcpy(Pl.unb, &A, sizeof(A));
 }
 
-// Resident CTAs of the multi-mesh search (one wave, at most one warp per work item).  Call before a
-// stream capture.
+// Resident CTAs of the multi-mesh search (one wave, at most one warp per work item), and their spilled
+// queues' buffer.  Call before a stream capture.
 int unb_multi_grid(sdfgpu_ctx* ctx, int64_t total, int64_t* grid) {
   int per_sm = 0, sms = 148;
   SDF_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_unbounded_multi<kUnbPlain>, kUnbThreads, 0));
   SDF_CUDA(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
   *grid = grid_for(total, kUnbWarps, (int64_t)sms * std::max(per_sm, 1));
+  int* spill;
+  SDF_TRY(scratch_t(ctx, "unb_spill", (size_t)*grid * kUnbWarps * kWideSpill, &spill));
   return 0;
 }
 
@@ -112,15 +113,16 @@ int unb_multi(sdfgpu_ctx* ctx, const void* d_items, const int64_t* d_off, int co
   if (count < 1) return 0;
   SDF_CUDA(ctx, cudaMemsetAsync(heads, 0, 3 * sizeof(unsigned long long), st));
   const UnbArgs* it = static_cast<const UnbArgs*>(d_items);
+  int* spill = buf<int>(ctx, "unb_spill");
   if (radius) {
     k_unbounded_multi<kUnbRadius><<<(unsigned)grid, kUnbThreads, 0, st>>>(it, d_off, count, heads, nullptr, nullptr,
-                                                                           ctx->d_counters);
+                                                                           ctx->d_counters, spill);
     SDF_KERNEL(ctx);
     k_unbounded_multi<kUnbListed><<<(unsigned)grid, kUnbThreads, 0, st>>>(it, d_off, count, heads + 1, redo, heads + 2,
-                                                                           ctx->d_counters);
+                                                                           ctx->d_counters, spill);
   } else {
     k_unbounded_multi<kUnbPlain><<<(unsigned)grid, kUnbThreads, 0, st>>>(it, d_off, count, heads, nullptr, nullptr,
-                                                                          ctx->d_counters);
+                                                                          ctx->d_counters, spill);
   }
   SDF_KERNEL(ctx);
   return 0;
