@@ -178,6 +178,17 @@ inline int scratch_t(sdfgpu_ctx* ctx, const char* name, size_t count, T** out) {
   return rc;
 }
 
+// The same outside the batch item's own names: buffers that only kernels on the context's own stream use,
+// one launch after the other, so the items of a worker share them.
+template <class T>
+inline int scratch_ctx(sdfgpu_ctx* ctx, const char* name, size_t count, T** out) {
+  std::string ns;
+  ns.swap(ctx->ns);
+  const int rc = scratch_t(ctx, name, count, out);
+  ns.swap(ctx->ns);
+  return rc;
+}
+
 template <class T>
 inline T* buf(sdfgpu_ctx* ctx, const char* name) {
   auto it = ctx->ns.empty() ? ctx->bufs.find(name) : ctx->bufs.find(ctx->ns + name);
@@ -243,7 +254,7 @@ int run_nearest_points(sdfgpu_ctx* ctx, const GridP& g, double* d_dist);
 // folds of many prepared meshes together.
 struct DistPlan {
   alignas(16) unsigned char fold[448];      // the fold kernel's arguments
-  alignas(16) unsigned char knn_args[448];  // the fallback kernel's arguments (when knn)
+  alignas(16) unsigned char knn_args[640];  // the fallback kernel's arguments (when knn)
   alignas(16) unsigned char unb[512];       // unbounded / learned: the search's arguments (UnbArgs)
   bool unbounded = false;                   // the plan is an unbounded search (unb), not a fold
   bool unb_radius = false;                  // ... started from the learned radius

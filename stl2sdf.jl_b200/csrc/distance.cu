@@ -399,116 +399,144 @@ __global__ void k_band(const float4* __restrict__ v32, const TriRec64* __restric
   }
 }
 
-constexpr int kStack = 64;
 constexpr int kKnnCap = 256;
 
 struct KnnArgs {
-  GridP g;
+  UnbArgs u;            // the tree, the leaves, the brick lattice and the results' arrays
   const uint8_t* status;
   const uint8_t* band;  // NULL: every node with an empty candidate set
-  const BNode* nodes;
-  const int32_t* leaf_prim;
-  const int32_t* tri_idx;  // not used (IEN64 is read instead)
   const int64_t* IEN;
   const double* X;
   const int32_t* ine_off;
   const int32_t* ine;
-  const TriRec64* rec;
-  float pad;
-  int64_t max_visits;
-  double* dist;
-  double* xp;
-  int64_t* counters;
 };
 
-// knn(vtx_kdtree, p, 3) + union of INE + ordered fold (dfOnTriangularMesh.jl:82-177).
-__global__ void k_knn_fallback(KnnArgs A) {
-  const GridP& g = A.g;
-  int64_t done = 0;
-  for (int64_t lin = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; lin < g.ngp; lin += (int64_t)gridDim.x * blockDim.x) {
-    if (A.status[lin]) continue;
-    if (A.band && !A.band[lin]) continue;
-    int64_t i, j, k;
-    node_ijk(g, lin, i, j, k);
-    const d3 p = gnode(g, i, j, k);
-    const float3 p32 = local32(g, p);
-    double bs[3] = {INFINITY, INFINITY, INFINITY};
-    int64_t bv[3] = {-1, -1, -1};
-    int stack[kStack];
-    int sp = 0;
-    stack[sp++] = 0;
-    bool overflow = false;
-    int64_t visits = 0;
-    while (sp > 0) {
-      if (++visits > A.max_visits) { overflow = true; break; }
-      const BNode nd = A.nodes[stack[--sp]];
-      const float r = isinf(bs[2]) ? INFINITY : (float)sqrt(bs[2]) + A.pad;
-      const int ch[2] = {nd.d.x, nd.d.y};
-      for (int side = 0; side < 2; ++side) {
-        float3 lo, hi;
-        child_box(nd, side, lo, hi);
-        if (lo.x > hi.x) continue;
-        if (!isinf(r) && box_d2(p32, lo, hi) > r * r) continue;
-        if (ch[side] & kLeafBit) {
-          const int prim = A.leaf_prim[ch[side] & 0x7fffffff];
-          for (int q = 0; q < 3; ++q) {
-            const int64_t vi = A.IEN[3 * (int64_t)prim + q] - 1;
-            if (vi == bv[0] || vi == bv[1] || vi == bv[2]) continue;
-            const double dx = ds(A.X[3 * vi], p.x), dy = ds(A.X[3 * vi + 1], p.y), dz = ds(A.X[3 * vi + 2], p.z);
-            double s = dm(dx, dx);
-            s = da(s, dm(dy, dy));
-            s = da(s, dm(dz, dz));
-            // insert (s, vi) into the sorted top 3 (ties to the lower vertex index)
-            int pos = 3;
-            while (pos > 0 && (s < bs[pos - 1] || (s == bs[pos - 1] && vi < bv[pos - 1]))) --pos;
-            if (pos < 3) {
-              for (int z = 2; z > pos; --z) { bs[z] = bs[z - 1]; bv[z] = bv[z - 1]; }
-              bs[pos] = s;
-              bv[pos] = vi;
-            }
-          }
+// The three nearest vertices found so far, by FP64 squared distance, ties to the lower vertex index.
+struct Knn3 {
+  double s[3];
+  int64_t v[3];
+};
+// Inserts the vertices of the kept triangles and empties the slots.
+template <int S>
+__device__ __noinline__ void knn_insert(const KnnArgs& A, LaneBest& L, const d3& p, Knn3& K) {
+#pragma unroll 1
+  for (int q = 0; q < L.n; ++q) {
+    const int64_t prim = L.t[q * S];
+#pragma unroll 1
+    for (int k = 0; k < 3; ++k) {
+      const int64_t vi = A.IEN[3 * prim + k] - 1;
+      if (vi == K.v[0] || vi == K.v[1] || vi == K.v[2]) continue;
+      const double dx = ds(A.X[3 * vi], p.x), dy = ds(A.X[3 * vi + 1], p.y), dz = ds(A.X[3 * vi + 2], p.z);
+      double s = dm(dx, dx);
+      s = da(s, dm(dy, dy));
+      s = da(s, dm(dz, dz));
+      auto before = [&](int k2) { return s < K.s[k2] || (s == K.s[k2] && vi < K.v[k2]); };
+      if (!before(2)) continue;
+      K.s[2] = s;
+      K.v[2] = vi;
+#pragma unroll
+      for (int k2 = 2; k2 > 0; --k2)
+        if (s < K.s[k2 - 1] || (s == K.s[k2 - 1] && vi < K.v[k2 - 1])) {
+          K.s[k2] = K.s[k2 - 1];
+          K.v[k2] = K.v[k2 - 1];
+          K.s[k2 - 1] = s;
+          K.v[k2 - 1] = vi;
         } else {
-          if (sp >= kStack) { overflow = true; break; }
-          stack[sp++] = ch[side];
+          break;
         }
-      }
-      if (overflow) break;
     }
-    if (overflow) { count_add(A.counters, C_ERR_STACK, 1); continue; }
-    int32_t cand[kKnnCap];
-    int nc = 0;
-    for (int q = 0; q < 3 && !overflow; ++q) {
-      if (bv[q] < 0) continue;
-      for (int32_t e = A.ine_off[bv[q]]; e < A.ine_off[bv[q] + 1]; ++e) {
-        if (nc >= kKnnCap) { overflow = true; break; }
-        cand[nc++] = A.ine[e];
-      }
-    }
-    if (overflow) { count_add(A.counters, C_ERR_CAPACITY, 1); continue; }
-    for (int a = 1; a < nc; ++a) {  // insertion sort, then unique
-      const int32_t v = cand[a];
-      int b = a - 1;
-      while (b >= 0 && cand[b] > v) { cand[b + 1] = cand[b]; --b; }
-      cand[b + 1] = v;
-    }
-    double m = kBig;
-    d3 proj = {0.0, 0.0, 0.0};
-    for (int a = 0; a < nc; ++a) {
-      if (a > 0 && cand[a] == cand[a - 1]) continue;
-      tri_step64(A.rec[cand[a]], p, m, proj, true);
-    }
-    double d = m;
-    if (fabs(d) > fabs(g.h)) d = g.h;
-    A.dist[lin] = d;
-    if (A.xp) {
-      A.xp[3 * lin] = proj.x;
-      A.xp[3 * lin + 1] = proj.y;
-      A.xp[3 * lin + 2] = proj.z;
-    }
-    ++done;
   }
-  for (int off = 16; off > 0; off >>= 1) done += __shfl_down_sync(0xffffffffu, done, off);
-  if ((threadIdx.x & 31) == 0 && done) count_add(A.counters, C_KNN, done);
+  L.n = 0;
+  L.m = fminf(L.m, __double2float_ru(sqrt(K.s[2])));  // the third distance so far, exactly
+}
+
+// The union of the three vertices' triangles folded in ascending index (dfOnTriangularMesh.jl:86-177).
+// Returns false when it holds more than kKnnCap.
+__device__ __noinline__ bool knn_fold(const KnnArgs& A, const Knn3& K, const d3& p, double& m, d3& proj) {
+  int32_t cand[kKnnCap];
+  int nc = 0;
+  for (int q = 0; q < 3; ++q) {
+    if (K.v[q] < 0) continue;
+    for (int32_t e = A.ine_off[K.v[q]]; e < A.ine_off[K.v[q] + 1]; ++e) {
+      if (nc >= kKnnCap) return false;
+      // insertion into the sorted list; a triangle of two of the vertices comes twice
+      const int32_t v = A.ine[e];
+      int b = nc;
+      while (b > 0 && cand[b - 1] > v) --b;
+      if (b > 0 && cand[b - 1] == v) continue;
+      for (int k = nc; k > b; --k) cand[k] = cand[k - 1];
+      cand[b] = v;
+      ++nc;
+    }
+  }
+  for (int a = 0; a < nc; ++a) tri_step64(A.u.rec[cand[a]], p, m, proj, true);
+  return true;
+}
+
+// knn(vtx_kdtree, p, 3) + union of INE + ordered fold (dfOnTriangularMesh.jl:82-177) of the nodes
+// without candidates, one warp per brick of 4 x 2 x 4 nodes: the brick search of the unbounded distance
+// with m the bound of the third nearest vertex, FP64 distances of the vertices it keeps, then the fold
+// per node.  The walk it replaces (a thread per node over the LBVH, children in stored order, a bound only
+// after three vertices) took 80.4 ms for 460k nodes over a 131k-triangle torus; this one 3.5 ms.
+// Bound: as k_unbounded; the FP64 distances of about 33 triangles' vertices per node and the folds' FP64
+// steps (about a dozen per node) are two fifths of it.
+__global__ void __launch_bounds__(kUnbThreads, 4) k_knn_bricks(const __grid_constant__ KnnArgs A) {
+  __shared__ WideShared s_wide[kUnbWarps];
+  __shared__ int s_keep[kKeep * kUnbThreads];
+  const UnbArgs& U = A.u;
+  const GridP& g = U.g;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int* spill = U.spill + (int64_t)(blockIdx.x * kUnbWarps + w) * kKnnSpill;
+  int lx, ly, lz, rep;
+  brick_lane(U.b, lane, lx, ly, lz, rep);
+  uint32_t done = 0, errs = 0, caps = 0, visits = 0;
+  for (int64_t brick = blockIdx.x * (int64_t)kUnbWarps + w; brick < U.nbricks;
+       brick += (int64_t)gridDim.x * kUnbWarps) {
+    const int64_t bx = brick % U.nb[0], by = (brick / U.nb[0]) % U.nb[1], bz = brick / (U.nb[0] * U.nb[1]);
+    const int64_t i = bx * U.b[0] + lx, j = by * U.b[1] + ly, k = bz * U.b[2] + lz;
+    const int64_t lin = i + g.n[0] * (j + g.n[1] * k);
+    bool mine = i <= g.N[0] && j <= g.N[1] && k <= g.N[2];
+    mine = mine && A.status[lin] == 0 && (!A.band || A.band[lin] != 0);
+    if (!__any_sync(0xffffffffu, mine)) continue;
+    const d3 p = gnode(g, min(i, g.N[0]), min(j, g.N[1]), min(k, g.N[2]));
+    const float3 p32 = local32(g, p);
+    LaneBest L;
+    L.m = INFINITY;
+    L.n = 0;
+    L.t = s_keep + threadIdx.x;
+    Knn3 K = {{INFINITY, INFINITY, INFINITY}, {-1, -1, -1}};
+    const bool ok = wide_search<kUnbThreads, true>(U, s_wide[w], spill, lane, p, p32, mine, L, visits,
+                                                   [&] { knn_insert<kUnbThreads>(A, L, p, K); });
+    if (!ok && lane == 0) ++errs;
+    if (mine && ok) {
+      knn_insert<kUnbThreads>(A, L, p, K);
+      double m = kBig;
+      d3 proj = {0.0, 0.0, 0.0};
+      if (knn_fold(A, K, p, m, proj)) {
+        double d = m;
+        if (fabs(d) > fabs(g.h)) d = g.h;
+        U.dist[lin] = d;
+        if (U.xp) {
+          U.xp[3 * lin] = proj.x;
+          U.xp[3 * lin + 1] = proj.y;
+          U.xp[3 * lin + 2] = proj.z;
+        }
+        ++done;
+      } else {
+        ++caps;
+      }
+    }
+    __syncwarp();
+  }
+  for (int off = 16; off > 0; off >>= 1) {
+    done += __shfl_down_sync(0xffffffffu, done, off);
+    caps += __shfl_down_sync(0xffffffffu, caps, off);
+  }
+  if (lane == 0) {
+    if (done) count_add(U.counters, C_KNN, done);
+    if (caps) count_add(U.counters, C_ERR_CAPACITY, caps);
+    if (errs) count_add(U.counters, C_ERR_STACK, errs);
+  }
 }
 
 // True nearest triangle of every node (no clamp), one warp per brick of 32 nodes (wide_search,
@@ -568,11 +596,8 @@ int ceil_log2(uint64_t v) {
 
 namespace {
 
-// The unbounded search's arguments for grid g on the current mesh (FP32 error model as in
-// run_distances), with the learned radius of every brick when use_learned and the network's bound
-// is on; the context stream waits for the LBVH and its oriented boxes.
-int unb_setup(sdfgpu_ctx* ctx, const GridP& g, int use_learned, double* d_dist, double* d_xp, UnbArgs& A) {
-  SDF_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->ev_obb, 0));  // the search walks the LBVH and its oriented boxes
+// The brick search's arguments for grid g in bricks b on the current mesh.
+void unb_tree(sdfgpu_ctx* ctx, const GridP& g, const int32_t b[3], double* d_dist, double* d_xp, UnbArgs& A) {
   A = UnbArgs{};
   A.g = g;
   A.nodes = buf<BNode>(ctx, "nodes");
@@ -586,14 +611,21 @@ int unb_setup(sdfgpu_ctx* ctx, const GridP& g, int use_learned, double* d_dist, 
   unb_mesh(ctx, A);
   unb_errors(ctx->mesh, g.E, A);
   A.nbricks = 1;
+  int bit = 0;
   for (int a = 0; a < 3; ++a) {
-    A.b[a] = ctx->brick[a];
+    A.b[a] = b[a];
     A.nb[a] = cdiv(g.n[a], A.b[a]);
     A.nbricks *= A.nb[a];
-  }
-  int bit = 0;
-  for (int a = 0; a < 3; ++a)  // lane bits: x first; the extents are powers of two (their product is 32)
+    // lane bits: x first; the extents are powers of two (their product is 32)
     for (int m = 1; m < A.b[a]; m <<= 1) A.lat[bit++][a] = (float)(g.h * m);
+  }
+}
+
+// The unbounded search's arguments for grid g on the current mesh, with the learned radius of every brick when use_learned and the network's bound
+// is on; the context stream waits for the LBVH and its oriented boxes.
+int unb_setup(sdfgpu_ctx* ctx, const GridP& g, int use_learned, double* d_dist, double* d_xp, UnbArgs& A) {
+  SDF_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->ev_obb, 0));  // the search walks the LBVH and its oriented boxes
+  unb_tree(ctx, g, ctx->brick, d_dist, d_xp, A);
   if (use_learned) {
     // the network's radius at each brick centre c, rc = (dhat (1 + alpha) + beta * coarse spacing
     // / s) s (a margin for the network's error and for the interpolation between its training
@@ -628,7 +660,7 @@ int run_distances(sdfgpu_ctx* ctx, const GridP& g, int mode, int use_learned, do
     SDF_CUDA(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
     const unsigned grid = grid_for(A.nbricks, kUnbWarps, (int64_t)sms * std::max(per_sm, 1));
     A.next = heads;
-    SDF_TRY(scratch_t(ctx, "unb_spill", (size_t)grid * kUnbWarps * kWideSpill, &A.spill));
+    SDF_TRY(scratch_ctx(ctx, "unb_spill", (size_t)grid * kUnbWarps * kWideSpill, &A.spill));
     if (A.radius) {
       SDF_TRY(scratch_t(ctx, "brick_redo", (size_t)A.nbricks, &A.redo));
       A.redo_n = heads + 2;
@@ -688,7 +720,6 @@ int dist_prepare(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, doub
   const float E = (float)g.E;
   const float eD_abs = 4.0e-6f * E;
   const float eD_rel = 4.0e-6f;
-  const float pad = 2.0e-6f * E;
   const double sr = 2.5 * g.h;
   const double R = mode == SDFGPU_MODE_REF_RULE ? sr * (1.0 + 1e-9) + 1e-6 * g.E : g.h * (1.0 + 1e-9) + 1e-6 * g.E;
   int32_t *tri_cnt, *tri_off, *tile_cnt, *tile_off, *vals, *vals2;
@@ -788,22 +819,16 @@ int dist_prepare(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, doub
       uint8_t* band = nullptr;
       if (!d_xp) SDF_TRY(scratch_t(ctx, "band", (size_t)g.ngp, &band));
       KnnArgs K;
-      K.g = g;
+      const int32_t b[3] = {4, 2, 4};
+      unb_tree(ctx, g, b, d_dist, d_xp, K.u);
+      const int64_t ctas = grid_for(K.u.nbricks, kUnbWarps, 148 * 4);
+      SDF_TRY(scratch_t(ctx, "knn_spill", (size_t)ctas * kUnbWarps * kKnnSpill, &K.u.spill));
       K.status = status;
       K.band = band;
-      K.nodes = buf<BNode>(ctx, "nodes");
-      K.leaf_prim = buf<int32_t>(ctx, "leaf_prim");
-      K.tri_idx = nullptr;
       K.IEN = buf<int64_t>(ctx, "IEN64");
       K.X = buf<double>(ctx, "X64");
       K.ine_off = buf<int32_t>(ctx, "ine_off");
       K.ine = buf<int32_t>(ctx, "ine");
-      K.rec = rec;
-      K.pad = pad;
-      K.max_visits = 2 * nel + 64;
-      K.dist = d_dist;
-      K.xp = d_xp;
-      K.counters = ctx->d_counters;
       std::memcpy(Pl.knn_args, &K, sizeof(K));
       Pl.knn = true;
       Pl.band = band;
@@ -847,10 +872,10 @@ int dist_knn(sdfgpu_ctx* ctx, const DistPlan& Pl, cudaStream_t st, bool wait_bvh
                                                    Pl.band);
     SDF_KERNEL(ctx);
   }
-  if (wait_bvh) SDF_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_bvh, 0));  // the fallback walks the LBVH
+  if (wait_bvh) SDF_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_obb, 0));  // the fallback walks the LBVH
   KnnArgs K;
   std::memcpy(&K, Pl.knn_args, sizeof(K));
-  k_knn_fallback<<<grid_for(g.ngp, 128, 148 * 16), 128, 0, st>>>(K);
+  k_knn_bricks<<<grid_for(K.u.nbricks, kUnbWarps, 148 * 4), kUnbThreads, 0, st>>>(K);
   SDF_KERNEL(ctx);
   return 0;
 }
@@ -892,7 +917,7 @@ void plan_set_counters(DistPlan& Pl, int64_t* counters) {
   if (Pl.knn) {
     KnnArgs K;
     std::memcpy(&K, Pl.knn_args, sizeof(K));
-    K.counters = counters;
+    K.u.counters = counters;
     std::memcpy(Pl.knn_args, &K, sizeof(K));
   }
 }

@@ -34,7 +34,8 @@ __global__ void __launch_bounds__(kUnbThreads, 4) k_nearest_points(const __grid_
     L.t = s_keep + threadIdx.x;
     double m64 = kBig;
     d3 proj = {0.0, 0.0, 0.0};
-    bool ok = wide_search<kUnbThreads>(A, s_wide[w], spill, lane, p, p32, mine, L, visits);
+    bool ok = wide_search<kUnbThreads, false>(A, s_wide[w], spill, lane, p, p32, mine, L, visits,
+                                                [&] { lane_prune<kUnbThreads>(A, L, p); });
     const bool over = mine && L.n > kKeep;
     if (ok && __any_sync(0xffffffffu, over))
       ok = exact_search(A, s_wide[w].queue, lane, 0, p, p32, over, band_of(A, L.m), m64, proj, fp64, visits);
@@ -78,7 +79,7 @@ UnbArgs point_args(sdfgpu_ctx* ctx, const GridP& g, double* d_dist) {
 int run_nearest_points(sdfgpu_ctx* ctx, const GridP& g, double* d_dist) {
   UnbArgs A = point_args(ctx, g, d_dist);
   const unsigned grid = grid_for(g.ngp, kUnbWarps, 148 * 4);
-  SDF_TRY(scratch_t(ctx, "unb_spill", (size_t)grid * kUnbWarps * kWideSpill, &A.spill));
+  SDF_TRY(scratch_ctx(ctx, "unb_spill", (size_t)grid * kUnbWarps * kWideSpill, &A.spill));
   k_nearest_points<<<grid, kUnbThreads, 0, ctx->stream>>>(A);
   SDF_KERNEL(ctx);
   return 0;

@@ -349,7 +349,9 @@ __device__ __forceinline__ void lane_resolve(const UnbArgs& A, LaneBest& L, cons
 // address.  Here the per-(child, node) work reads one word.
 constexpr int kWideNodes = 8;     // LBVH nodes opened per step (four grandchildren each: one per lane)
 constexpr int kWideQueue = 256;   // nodes waiting per warp in shared memory (a ring), 160 of them in use ...
-constexpr int kWideSpill = 2048;  // ... and behind them in device memory (a ring per resident warp)
+constexpr int kWideSpill = 2048;  // ... and behind them in device memory (a ring per resident warp; the
+                                  // nearest-vertex search has one of kKnnSpill)
+constexpr int kKnnSpill = 512;
 constexpr int kWideLeafs = 4;     // subtrees of up to this many triangles are queued whole
 constexpr int kWideLeafQ = 32 * kWideLeafs + 32;  // a step adds at most 32 kWideLeafs to at most 31
 static_assert(kWideLeafs < 8, "three bits of triangle counts");
@@ -357,12 +359,18 @@ static_assert(kWideLeafs < 8, "three bits of triangle counts");
 struct __align__(16) WideShared {
   float ub[32];           // per node: bound on the FP32 distances that matter, -3e38 for unused lanes
   float4 node[32];        // the nodes relative to node 0
-  float4 rep[kWideNodes]; // sample vertices of a step relative to the centre, .w = -|x|^2 (1 + 1e-6)
+  float4 rep[3 * kWideNodes]; // sample vertices of a step relative to the centre, .w = -|x|^2 (1 + 1e-6)
   int queue[kWideQueue];
   int leaf[kWideLeafQ];
   int2 cand[64];          // triangles left to evaluate: (sorted leaf, bit per node)
   int prim[32];           // triangle indices of the 32 being evaluated
 };
+
+// Whether three leaf-ordered vertices are distinct (global ids in .w).
+__device__ __forceinline__ bool differ3(const float4& a, const float4& b, const float4& c) {
+  const int i = __float_as_int(a.w), j = __float_as_int(b.w), k = __float_as_int(c.w);
+  return i != j && j != k && i != k;
+}
 
 // The linear function base + g . (p - p0) over the brick's lattice by the bits of the node index: lo
 // (bits 0-1) + hi (bits 2-3) + top (bit 4).  The loops over bit 4 stay rolled: the kernel's code is
@@ -450,9 +458,16 @@ __device__ __forceinline__ void child_plane(const P& A, int nid, int side, bool 
 // newest node of the shared ring is opened alone instead and its children stay there: depth-first
 // steps grow it by at most 3 per two levels of the tree (at most 62 levels: unique keys of 30 Morton bits
 // and a 32-bit index), which the 96 reserved entries hold.
-template <int S, class P>
+//
+// kKnn: the search for each lane's three nearest vertices (k_knn_bricks, distance.cu).  m then bounds
+// the distance of the third: a triangle's farthest vertex, where its vertices differ; the queued
+// leaves go to the evaluation as they are, and a triangle is kept when its nearest vertex lies
+// within band(m).  flush(): makes room in the slots (kKnn: called by all lanes, and empties them).
+template <int S, bool kKnn, class P, class Flush>
 __device__ __forceinline__ bool wide_search(const P& A, WideShared& W, int* spill, int lane, const d3& p,
-                                            const float3& p32, bool active, LaneBest& L, uint32_t& visits_out) {
+                                            const float3& p32, bool active, LaneBest& L, uint32_t& visits_out,
+                                            Flush flush) {
+  constexpr unsigned kSpill = kKnn ? kKnnSpill : kWideSpill;
   const float3 p0 = make_float3(__shfl_sync(0xffffffffu, p32.x, 0), __shfl_sync(0xffffffffu, p32.y, 0),
                                 __shfl_sync(0xffffffffu, p32.z, 0));
   // the brick's centre: half of every lattice step from node 0
@@ -474,13 +489,53 @@ __device__ __forceinline__ bool wide_search(const P& A, WideShared& W, int* spil
     int waiting = (int)(tail - head);
     if (waiting == 0 && stail != shead) {  // refill the shared ring
       waiting = (int)min(stail - shead, (unsigned)(kWideQueue - 96));
-      for (int i = lane; i < waiting; i += 32) W.queue[i] = spill[(shead + i) % kWideSpill];
+      for (int i = lane; i < waiting; i += 32) W.queue[i] = spill[(shead + i) % kSpill];
       shead += waiting;
       head = 0;
       tail = waiting;
       __syncwarp();
     }
-    if (nc >= 32 || (waiting == 0 && nl == 0 && nc > 0)) {
+    if constexpr (kKnn) {
+      if (nl >= 32 || (waiting == 0 && nl > 0)) {
+        // ---- eval of three vertices: lane = triangle, one node at a time
+        const int cnt = min(nl, 32);
+        nl -= cnt;
+        const int li = lane < cnt ? W.leaf[nl + lane] : 0;
+        const float4 a4 = A.lv32[3 * (int64_t)li], b4 = A.lv32[3 * (int64_t)li + 1], c4 = A.lv32[3 * (int64_t)li + 2];
+        const float3 a = f3(a4) - p0, b = f3(b4) - p0, e = f3(c4) - p0;
+        const bool three = lane < cnt && differ3(a4, b4, c4);
+        W.prim[lane] = __float_as_int(A.ltri.at(0, li).w) & ~kWeakTri;
+        unsigned mine = 0u;
+        float mnew = L.m;
+        __syncwarp();
+        for (unsigned todo = __ballot_sync(0xffffffffu, active); todo; todo &= todo - 1u) {
+          const int q = __ffs(todo) - 1;
+          const float3 P3 = f3(W.node[q]);
+          const float3 da = P3 - a, db = P3 - b, dc = P3 - e;
+          const float xa = dot3f(da, da), xb = dot3f(db, db), xc = dot3f(dc, dc);
+          const unsigned key = three ? __float_as_uint(fmaxf(xa, fmaxf(xb, xc))) : 0x7f800000u;
+          const float best = sqrt_approx(__uint_as_float(__reduce_min_sync(0xffffffffu, key)));
+          const float m = fminf(__shfl_sync(0xffffffffu, L.m, q), best);
+          const float bd = band_of(A, m);
+          const unsigned in = __ballot_sync(0xffffffffu, lane < cnt && !(fminf(xa, fminf(xb, xc)) > bd * bd));
+          if (lane == q) {
+            mine = in;
+            mnew = m;
+          }
+        }
+        if (!active) mine = 0u;
+        L.m = mnew;
+        while (true) {
+          for (; mine && L.n < kKeep; mine &= mine - 1u) L.t[L.n++ * S] = W.prim[__ffs(mine) - 1];
+          if (!__any_sync(0xffffffffu, mine != 0u)) break;
+          flush();  // all lanes together: one lane at a time took most of the kernel
+        }
+        if (active) W.ub[lane] = wide_bound(A, L.m);
+        __syncwarp();
+        continue;
+      }
+    }
+    if (!kKnn && (nc >= 32 || (waiting == 0 && nl == 0 && nc > 0))) {
       // ---- eval: lane = triangle, one node at a time
       const int cnt = min(nc, 32);
       nc -= cnt;
@@ -509,7 +564,7 @@ __device__ __forceinline__ bool wide_search(const P& A, WideShared& W, int* spil
       if (active) {
         if (L.m > band_of(A, mnew)) L.n = 0;  // everything kept so far is outside the new band
         L.m = mnew;
-        if (L.n + __popc(mine) > kKeep && L.n <= kKeep) lane_prune<S>(A, L, p);  // make room
+        if (L.n + __popc(mine) > kKeep && L.n <= kKeep) flush();  // make room
         for (; mine; mine &= mine - 1u) {
           if (L.n < kKeep) L.t[L.n * S] = W.prim[__ffs(mine) - 1];
           ++L.n;
@@ -519,7 +574,7 @@ __device__ __forceinline__ bool wide_search(const P& A, WideShared& W, int* spil
       __syncwarp();
       continue;
     }
-    if (nl >= 32 || (waiting == 0 && nl > 0)) {
+    if (!kKnn && (nl >= 32 || (waiting == 0 && nl > 0))) {
       // ---- leaves: lane = triangle, its plane and edge lines against every node
       const int cnt = min(nl, 32);
       nl -= cnt;
@@ -567,7 +622,7 @@ __device__ __forceinline__ bool wide_search(const P& A, WideShared& W, int* spil
     if (waiting == 0) break;
     // ---- open
     int n = min(kWideNodes, waiting);
-    const bool fifo = stail - shead + 4 * kWideNodes <= (unsigned)kWideSpill;
+    const bool fifo = stail - shead + 4 * kWideNodes <= kSpill;
     if (!fifo) n = 1;
     visits += n;
     if (visits > A.max_visits || (!fifo && waiting + 3 > kWideQueue)) { ok = false; break; }
@@ -579,10 +634,13 @@ __device__ __forceinline__ bool wide_search(const P& A, WideShared& W, int* spil
     bool act = (lane >> 2) < n;
     int nid = act ? W.queue[(first + (lane >> 2)) % kWideQueue] : 0;
     int4 q = A.nodes[nid].d;
-    if ((lane & 3) == 0) {  // the node's sample vertex
-      const float4 v = A.lv32[3 * (int64_t)((q.z + q.w) >> 1)];
+    if (kKnn ? (lane & 3) != 3 : (lane & 3) == 0) {  // the node's sample vertex (kKnn: all three of its triangle)
+      const int64_t l = 3 * (int64_t)((q.z + q.w) >> 1);
+      const float4 v = A.lv32[l + (kKnn ? lane & 3 : 0)];
+      const bool use = act && (!kKnn || differ3(A.lv32[l], A.lv32[l + 1], A.lv32[l + 2]));
       const float3 r = make_float3(v.x - c.x, v.y - c.y, v.z - c.z);
-      W.rep[lane >> 2] = make_float4(r.x, r.y, r.z, act ? dot3f(r, r) * -(1.f + 1.0e-6f) : -3.0e38f);
+      W.rep[kKnn ? 3 * (lane >> 2) + (lane & 3) : lane >> 2] =
+          make_float4(r.x, r.y, r.z, use ? dot3f(r, r) * -(1.f + 1.0e-6f) : -3.0e38f);
     }
     int side = (lane >> 1) & 1;
     int gamma = q.x & 0x7fffffff;
@@ -608,8 +666,11 @@ __device__ __forceinline__ bool wide_search(const P& A, WideShared& W, int* spil
       float best = -3.0e38f;
 #pragma unroll
       for (int k = 0; k < kWideNodes; ++k) {
-        const float4 r = W.rep[k];
-        best = fmaxf(best, fmaf(2.f * d.x, r.x, fmaf(2.f * d.y, r.y, fmaf(2.f * d.z, r.z, r.w))));
+        auto at = [&](int j) {
+          const float4 r = W.rep[j];
+          return fmaf(2.f * d.x, r.x, fmaf(2.f * d.y, r.y, fmaf(2.f * d.z, r.z, r.w)));
+        };
+        best = fmaxf(best, kKnn ? fminf(at(3 * k), fminf(at(3 * k + 1), at(3 * k + 2))) : at(k));
       }
       const float d2 = fmaf(dot3f(d, d), 1.f + 1.0e-6f, -best);
       L.m = fminf(L.m, sqrt_approx(fmaxf(d2, 0.f)) * (1.f + 2.0e-6f));
@@ -624,7 +685,7 @@ __device__ __forceinline__ bool wide_search(const P& A, WideShared& W, int* spil
       if (open) W.queue[(tail + __popc(mi & below)) % kWideQueue] = child;
       tail += more;
     } else {
-      if (open) spill[(stail + __popc(mi & below)) % kWideSpill] = child;
+      if (open) spill[(stail + __popc(mi & below)) % kSpill] = child;
       stail += more;
     }
     const unsigned add = want && !open ? (unsigned)num : 0u;  // triangles to queue: 0..kWideLeafs

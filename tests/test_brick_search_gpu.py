@@ -107,3 +107,31 @@ def test_mesh_away_from_the_origin(gpu_ctx, shift, scale):
     X = V * scale + shift
     o, h, N = box_grid(X, 18)
     check(gpu_ctx, X, F, o, h, N)
+
+
+@pytest.mark.parametrize("kind", ["sphere", "fan", "soup", "one", "repeated"])
+@pytest.mark.parametrize("want_xp", [False, True])
+def test_three_nearest_vertices(gpu_ctx, kind, want_xp):
+    """The reference rule's fallback where every node or most of them take it: meshes coarse against the
+    cell, a vertex of 40 triangles, disjoint triangles, fewer than three distinct vertices."""
+    rng = np.random.default_rng(11)
+    if kind == "sphere":
+        X, F = synthetic.icosphere(2, jitter=0.02, seed=4)
+    elif kind == "fan":
+        t = 2 * np.pi * np.arange(40) / 40
+        X = np.concatenate([np.stack([np.cos(t), np.sin(t), 0.2 * np.cos(3 * t)], 1), [[0.1, 0, 0.5]]])
+        F = np.stack([1 + np.arange(40), 1 + (np.arange(40) + 1) % 40, np.full(40, 41)], 1)
+    elif kind == "soup":
+        X, F = rng.uniform(-1, 1, (3 * 37, 3)), 1 + np.arange(3 * 37).reshape(-1, 3)
+    elif kind == "one":
+        X, F = rng.uniform(-1, 1, (3, 3)), np.array([[1, 2, 3]])
+    else:
+        X, F = rng.uniform(-1, 1, (3, 3)), np.array([[1, 2, 2], [2, 1, 1]])
+    F = np.ascontiguousarray(F, np.int64)
+    o, h, N = box_grid(X, 21)
+    gpu_ctx.set_mesh(X, F)
+    d, xp = gpu_ctx.distances(o, h, N, 0, want_xp=want_xp)
+    ref, xpr, _ = oracle.distances(X, F, o, h, N, mode=0, want_xp=want_xp)
+    assert np.array_equal(d, ref)
+    if want_xp:
+        assert np.array_equal(xp, xpr)
