@@ -76,3 +76,34 @@ def test_stl_to_sdf_pipeline_with_artifacts(gpu_ctx, tmp_path):
     s = oracle.signs(X, IEN, grid.AABB_min, grid.cell_size, grid.N)["sign"]
     ref, _, _, _ = artifacts.remove_sdf_artifacts(d * s, grid.N, 0.0, 0.01)
     assert np.array_equal(sdf, ref)
+
+
+@pytest.mark.parametrize("n", [(31, 7, 7), (32, 8, 8), (33, 9, 9), (64, 16, 17), (65, 1, 40), (1, 33, 33), (97, 25, 3)])
+@pytest.mark.parametrize("kind", ["noise", "dense", "full", "snake", "checkers"])
+def test_components_across_tiles(gpu_ctx, n, kind):
+    """Labels, counts and flips where components cross the 32 x 8 x 8 tiles in every way."""
+    nx, ny, nz = n
+    rng = np.random.default_rng(nx + ny + nz)
+    k, j, i = np.indices((nz, ny, nx))
+    if kind == "noise":
+        m = rng.random((nz, ny, nx)) < 0.3  # near the percolation threshold: long thin components
+    elif kind == "dense":
+        m = rng.random((nz, ny, nx)) < 0.6
+    elif kind == "full":
+        m = np.ones((nz, ny, nx), bool)
+    elif kind == "snake":  # rows joined alternately at their ends, layers too: one path through every tile
+        m = (j % 2 == 0) | (i == np.where(j % 4 == 1, nx - 1, 0))
+        m &= (k % 2 == 0) | ((j == 0) & (i == 0))
+    else:
+        m = (i + j + k) % 2 == 0
+    sdf = np.where(m, 1.0, -1.0).reshape(-1)
+    N = np.array(n) - 1
+    roots, comps, largest = gpu_ctx.components(N, sdf, 0.0)
+    ref = artifacts.labels(sdf >= 0.0, np.array(n))
+    assert np.array_equal(roots.astype(np.int64), ref)
+    sizes = np.unique(ref[ref >= 0], return_counts=True)[1]
+    assert (comps, largest) == (sizes.size, sizes.max(initial=0))
+    out = sdf.copy()
+    want = artifacts.remove_sdf_artifacts(sdf, N, 0.0, 0.3)
+    assert gpu_ctx.remove_artifacts(N, out, 0.0, 0.3) == want[1:]
+    assert np.array_equal(out, want[0])
