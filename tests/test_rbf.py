@@ -100,3 +100,28 @@ def test_stl_to_sdf_with_smoothing_reference_test_config(tmp_path, refinement):
     ref, rdims, _, _ = rbf.rbf_smoothing(sdf, grid.AABB_min, grid.AABB_max, grid.N, grid.cell_size, True, refinement)
     assert np.array_equal(dims, rdims)
     assert np.max(np.abs(vals - ref)) <= 2e-3 * np.max(np.abs(ref))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N", [(31, 7, 3), (32, 8, 4), (33, 9, 5), (1, 1, 1), (70, 2, 1), (3, 40, 12)])
+@pytest.mark.parametrize("thr", [0.5, 0.05, 1e-3, 1e-5, 2e-7])
+def test_gpu_products_across_tiles_and_cutoffs(gpu_ctx, N, thr):
+    """The product's 32 x 8 x 4 tiles with every halo, and the fine sums with every number of taps: the
+    approximation to FP32 rounding, the weights by the solver's own stopping rule (a matrix that is not
+    positive definite at a wide cut-off may not converge within the iteration cap; then only the former)."""
+    o, amax, N, h = _grid(N, 0.07, (0.1, -0.4, 0.3))
+    rng = np.random.default_rng(int(N.sum()))
+    d = rng.normal(size=int(np.prod(N + 1)))
+    # every node within the cut-off, which is what the library sums (the reference's 124 nearest are fewer
+    # than those beyond a radius of about 3 cells)
+    ref = rbf.evaluate(rbf.fine_axes(o, amax, N, 2)[0], rbf.coarse_axes(o, amax, N), rbf.process_vector(d), h, thr,
+                       k=min(d.size, 400))
+    got, _, _, _ = gpu_ctx.rbf_smoothing(o, amax, N, h, d, interpolation=False, smooth=2, threshold=thr)
+    # sums of up to 300 terms: the reference accumulates them in FP32
+    assert np.max(np.abs(got - ref)) <= 4e-6 * np.max(np.abs(ref))
+    if thr >= 1e-3 and d.size <= 1500:
+        _, w, its, res = gpu_ctx.rbf_smoothing(o, amax, N, h, d, True, 1, thr, want_weights=True)
+        K = rbf.kernel_matrix(rbf.coarse_axes(o, amax, N), h, thr)
+        b32 = rbf.process_vector(d)
+        if its < d.size:
+            assert np.linalg.norm(K @ w - b32) <= 1.05 * np.sqrt(np.finfo(np.float32).eps) * np.linalg.norm(b32)
