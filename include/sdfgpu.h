@@ -90,12 +90,12 @@ typedef struct sdfgpu_opts {
 typedef struct sdfgpu_stats {
   int64_t ngp;                    /* grid nodes of the call */
   int64_t nel;                    /* triangles of the mesh */
-  int64_t tile_pairs;             /* (tile, triangle) candidate pairs */
+  int64_t tile_pairs;             /* (tile, triangle) candidate pairs (0 where the scatter took the call) */
   int64_t active_tiles;           /* tiles with at least one candidate */
-  int64_t candidate_nodes;        /* nodes whose candidate set was non-empty */
+  int64_t candidate_nodes;        /* nodes whose candidate set was non-empty (0 where the scatter took it) */
   int64_t fp64_evals;             /* FP64 point-triangle evaluations (near-tie band) */
   int64_t knn_fallback_nodes;     /* nodes resolved by the 3-nearest-vertex fallback */
-  int64_t band_nodes;             /* nodes flagged within cell_size by the band scatter */
+  int64_t band_nodes;             /* nodes within cell_size of a triangle, where the scatter took the call */
   int64_t row_hits;               /* axis-ray (row, triangle) hits */
   int64_t undecided_nodes;        /* nodes whose 6 axis rays disagreed */
   int64_t extra_rays;             /* rays cast beyond the 6 axis rays */

@@ -122,6 +122,11 @@ int autotune_tile(sdfgpu_ctx* ctx, const double origin[3], double h, const int64
   double best_t = 1e300;
   int best_i = -1;
   double* d_dist = nullptr;
+  ctx->tune_tiles = !bricks;
+  struct Untune {
+    sdfgpu_ctx* c;
+    ~Untune() { c->tune_tiles = false; }
+  } untune{ctx};
   for (int c = 0; c < count; ++c) {
     for (int a = 0; a < 3; ++a) shape[a] = table[c][a];
     GridP g;

@@ -183,11 +183,12 @@ int reset_counters(sdfgpu_ctx* ctx) {
 }
 
 int finish_counters(sdfgpu_ctx* ctx, const GridP& g) {
-  int64_t tile_pairs = ctx->h_counters[C_TILE_PAIRS];
+  const int64_t tile_pairs = ctx->h_counters[C_TILE_PAIRS], band = ctx->h_counters[C_BAND];  // counted on the host
   SDF_CUDA(ctx, cudaMemcpyAsync(ctx->h_counters, ctx->d_counters, sizeof(int64_t) * C_NUM, cudaMemcpyDeviceToHost,
                                 ctx->stream));
   SDF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   ctx->h_counters[C_TILE_PAIRS] = tile_pairs;
+  ctx->h_counters[C_BAND] += band;
   sdfgpu_stats& s = ctx->stats;
   const int64_t* c = ctx->h_counters;
   s.ngp = g.ngp;

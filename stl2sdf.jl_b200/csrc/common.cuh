@@ -93,6 +93,8 @@ struct MeshDev {
   double bmin[3] = {0, 0, 0}, bmax[3] = {0, 0, 0};
   double E = 0.0;        // max |vertex - center| (inf-norm)
   double rho_max = 0.0;  // max vertex distance from its triangle's centroid
+  double rho_weak = 0.0; // the same over the triangles unfit for FP32 decisions
+  int64_t n_weak = 0;    // their number
   bool ine_ready = false;
 };
 
@@ -109,6 +111,7 @@ struct sdfgpu_ctx {
   cudaEvent_t ev[6] = {};
   std::string err;
   int32_t tile[3] = {4, 4, 4};
+  bool tune_tiles = false;       // the autotuner times the tile fold (run_distances)
   int32_t brick[3] = {4, 2, 4};  // nodes of one warp in the unbounded search (product 32)
   bool has_mesh = false;
   sdfgpu::MeshDev mesh;
@@ -253,7 +256,7 @@ int run_nearest_points(sdfgpu_ctx* ctx, const GridP& g, double* d_dist);
 // dist_fold runs one mesh's fold, dist_knn its 3-nearest-vertex fallback, dist_fold_multi the
 // folds of many prepared meshes together.
 struct DistPlan {
-  alignas(16) unsigned char fold[448];      // the fold kernel's arguments
+  alignas(16) unsigned char fold[512];      // the fold kernel's arguments (near.cu: those of its stage)
   alignas(16) unsigned char knn_args[640];  // the fallback kernel's arguments (when knn)
   alignas(16) unsigned char unb[512];       // unbounded / learned: the search's arguments (UnbArgs)
   bool unbounded = false;                   // the plan is an unbounded search (unb), not a fold
@@ -273,6 +276,10 @@ struct DistPlan {
 int dist_prepare(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, double* d_xp, DistPlan& P,
                  int use_learned = 0);
 int dist_fold(sdfgpu_ctx* ctx, const DistPlan& P);
+// The same stage as a scatter from the triangles to the nodes near them (near.cu).
+bool near_applies(const sdfgpu_ctx* ctx, const GridP& g, int mode);
+int near_prepare(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, DistPlan& P);
+int near_run(sdfgpu_ctx* ctx, const DistPlan& P);
 int dist_knn(sdfgpu_ctx* ctx, const DistPlan& P, cudaStream_t st, bool wait_bvh);
 int dist_fold_multi_grid(sdfgpu_ctx* ctx, int threads, int64_t total, int64_t* grid);
 int dist_fold_multi(sdfgpu_ctx* ctx, const void* d_args, const int64_t* d_off, int count, int64_t total, int threads,

@@ -680,6 +680,13 @@ int run_distances(sdfgpu_ctx* ctx, const GridP& g, int mode, int use_learned, do
   }
 
   DistPlan P;
+  if (!d_xp && !ctx->tune_tiles && near_applies(ctx, g, mode)) {
+    SDF_TRY(near_prepare(ctx, g, mode, d_dist, P));
+    SDF_MARK(ctx, T_TILES);
+    SDF_TRY(near_run(ctx, P));
+    SDF_MARK(ctx, T_FOLD);
+    return 0;
+  }
   SDF_TRY(dist_prepare(ctx, g, mode, d_dist, d_xp, P));
   SDF_MARK(ctx, T_TILES);
   SDF_TRY(dist_fold(ctx, P));

@@ -85,27 +85,87 @@ __global__ void k_prep(const double* __restrict__ X, int64_t nnp, const int64_t*
   }
 }
 
+// The FP32 record of a triangle (LeafTri, geom32.cuh), computed in FP64 from its vertices v, mesh-local,
+// and rounded once; id: its index, with kWeakTri when it is not fit for FP32 decisions.
+__device__ __forceinline__ LeafTri leaf_record(const double* v, int id, double cx, double cy, double cz) {
+  const double e0[3] = {v[3] - v[0], v[4] - v[1], v[5] - v[2]};
+  const double e1[3] = {v[6] - v[0], v[7] - v[1], v[8] - v[2]};
+  const double e2[3] = {v[6] - v[3], v[7] - v[4], v[8] - v[5]};
+  const double l0 = e0[0] * e0[0] + e0[1] * e0[1] + e0[2] * e0[2];
+  const double l1 = e1[0] * e1[0] + e1[1] * e1[1] + e1[2] * e1[2];
+  const double l2 = e2[0] * e2[0] + e2[1] * e2[1] + e2[2] * e2[2];
+  const double nx = e0[1] * e1[2] - e0[2] * e1[1], ny = e0[2] * e1[0] - e0[0] * e1[2], nz = e0[0] * e1[1] - e0[1] * e1[0];
+  const double nn = nx * nx + ny * ny + nz * nz;
+  LeafTri T;
+  T.a = make_float4((float)(v[0] - cx), (float)(v[1] - cy), (float)(v[2] - cz), __int_as_float(id));
+  if (nn > 1e-20 * l0 * l1) {
+    const double rn = 1.0 / sqrt(nn), un[3] = {nx * rn, ny * rn, nz * rn};
+    // inward in-plane edge normals: n x (edge direction), edges a->b, b->c, c->a
+    const double* ed[3] = {e0, e2, e1};
+    const double sg[3] = {1.0, 1.0, -1.0};
+    double m[3][3];
+    for (int k = 0; k < 3; ++k) {
+      const double* d = ed[k];
+      const double mx = sg[k] * (un[1] * d[2] - un[2] * d[1]), my = sg[k] * (un[2] * d[0] - un[0] * d[2]),
+                   mz = sg[k] * (un[0] * d[1] - un[1] * d[0]);
+      const double r = 1.0 / sqrt(mx * mx + my * my + mz * mz);
+      m[k][0] = mx * r; m[k][1] = my * r; m[k][2] = mz * r;
+    }
+    T.n = make_float4((float)un[0], (float)un[1], (float)un[2], (float)sqrt(l0));
+    T.m0 = make_float4((float)m[0][0], (float)m[0][1], (float)m[0][2], (float)sqrt(l2));
+    T.m1 = make_float4((float)m[1][0], (float)m[1][1], (float)m[1][2],
+                       (float)(e0[0] * m[1][0] + e0[1] * m[1][1] + e0[2] * m[1][2]));
+    T.m2 = make_float4((float)m[2][0], (float)m[2][1], (float)m[2][2], (float)sqrt(l1));
+  } else {  // no area: the longest edge (see LeafTri)
+    const int k = l0 >= l1 && l0 >= l2 ? 0 : (l1 >= l2 ? 2 : 1);  // edge a->b, c->a or b->c
+    const double* d = k == 0 ? e0 : (k == 1 ? e2 : e1);
+    const double len = sqrt(k == 0 ? l0 : (k == 1 ? l2 : l1));
+    double u[3] = {1.0, 0.0, 0.0};
+    if (len > 0.0)
+      for (int q = 0; q < 3; ++q) u[q] = d[q] / len;
+    const int s = k == 1 ? 3 : 0;  // from b along b->c, else from a
+    // n: the coordinate axis least along u, made normal to it
+    const int j = fabs(u[0]) <= fabs(u[1]) && fabs(u[0]) <= fabs(u[2]) ? 0 : (fabs(u[1]) <= fabs(u[2]) ? 1 : 2);
+    double un[3];
+    for (int q = 0; q < 3; ++q) un[q] = (q == j ? 1.0 : 0.0) - u[j] * u[q];
+    const double rn = 1.0 / sqrt(un[0] * un[0] + un[1] * un[1] + un[2] * un[2]);
+    for (int q = 0; q < 3; ++q) un[q] *= rn;
+    T.a = make_float4((float)(v[s] - cx), (float)(v[s + 1] - cy), (float)(v[s + 2] - cz), __int_as_float(id));
+    T.n = make_float4((float)un[0], (float)un[1], (float)un[2], (float)len);
+    T.m0 = make_float4((float)(un[1] * u[2] - un[2] * u[1]), (float)(un[2] * u[0] - un[0] * u[2]),
+                       (float)(un[0] * u[1] - un[1] * u[0]), k == 1 ? 1.f : 0.f);
+    T.m1 = make_float4(0.f, 0.f, 0.f, kFlat);
+    T.m2 = make_float4(0.f, 0.f, 0.f, -kFlat);
+  }
+  return T;
+}
+
 // Mesh-local FP32 copies: vertices, centroid, outward-rounded box; and rho = max vertex
 // distance from the centroid (decides whether the centroid rule can miss a triangle within h).
 // v32[3*el+k].w carries the global (0-based) index of vertex k; c32[el].w is 1 when the triangle
 // is well conditioned for FP32 decisions (no edge shorter than 1e-5 E, sine of the smallest
-// angle above ~1e-3, distinct vertices) and 0 when every decision on it must be made in FP64.
+// angle above ~1e-3, distinct vertices) and 0 when every decision on it must be made in FP64; rho_ord
+// receives rho, the same over such unfit triangles only, and their number.  tri32: the triangles' FP32
+// records (LeafTris by triangle index).
 __global__ void k_local32(const TriRec64* __restrict__ rec, const double4* __restrict__ cent,
                           const int64_t* __restrict__ IEN, int64_t nel, double cx, double cy, double cz, double E,
                           float4* __restrict__ v32, float4* __restrict__ c32, float4* __restrict__ box32,
-                          unsigned long long* rho_ord) {
-  double rho = 0.0;
+                          float4* __restrict__ tri32, unsigned long long* rho_ord) {
+  double rho = 0.0, rho_weak = 0.0;
+  unsigned weak = 0u;
   for (int64_t el = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; el < nel; el += (int64_t)gridDim.x * blockDim.x) {
     const TriRec64& r = rec[el];
     const double4 c = cent[el];
     int32_t gid[3];
+    double rt = 0.0;
     for (int k = 0; k < 3; ++k) {
       gid[k] = (int32_t)(IEN[3 * el + k] - 1);
       const double x = r.v[3 * k], y = r.v[3 * k + 1], z = r.v[3 * k + 2];
       v32[3 * el + k] = make_float4((float)(x - cx), (float)(y - cy), (float)(z - cz), __int_as_float(gid[k]));
       const double dx = x - c.x, dy = y - c.y, dz = z - c.z;
-      rho = fmax(rho, sqrt(dx * dx + dy * dy + dz * dz));
+      rt = fmax(rt, sqrt(dx * dx + dy * dy + dz * dz));
     }
+    rho = fmax(rho, rt);
     double L[3], lmin = 1e300, lmax = 0.0;
     for (int j = 0; j < 3; ++j) {
       const int a = j, b = (j + 1) % 3;
@@ -125,9 +185,27 @@ __global__ void k_local32(const TriRec64* __restrict__ rec, const double4* __res
                                 __double2float_rd(r.bmin[2] - cz), 0.f);
     box32[2 * el + 1] = make_float4(__double2float_ru(r.bmax[0] - cx), __double2float_ru(r.bmax[1] - cy),
                                     __double2float_ru(r.bmax[2] - cz), 0.f);
+    if (!ok) {
+      ++weak;
+      rho_weak = fmax(rho_weak, rt);
+    }
+    const LeafTri T = leaf_record(r.v, ok ? (int)el : (int)el | kWeakTri, cx, cy, cz);
+    const float4 f[5] = {T.a, T.n, T.m0, T.m1, T.m2};
+#pragma unroll
+    for (int k = 0; k < 5; ++k) tri32[(int64_t)k * nel + el] = f[k];
   }
-  for (int off = 16; off > 0; off >>= 1) rho = fmax(rho, __shfl_down_sync(0xffffffffu, rho, off));
-  if ((threadIdx.x & 31) == 0) atomicMax(rho_ord, dbl_ord(rho * (1.0 + 1e-12)));
+  for (int off = 16; off > 0; off >>= 1) {
+    rho = fmax(rho, __shfl_down_sync(0xffffffffu, rho, off));
+    rho_weak = fmax(rho_weak, __shfl_down_sync(0xffffffffu, rho_weak, off));
+    weak += __shfl_down_sync(0xffffffffu, weak, off);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(rho_ord, dbl_ord(rho * (1.0 + 1e-12)));
+    if (weak) {
+      atomicMax(rho_ord + 1, dbl_ord(rho_weak * (1.0 + 1e-12)));
+      atomicAdd(rho_ord + 2, (unsigned long long)weak);
+    }
+  }
 }
 
 __device__ __forceinline__ unsigned expand_bits10(unsigned v) {
@@ -237,73 +315,17 @@ __global__ void k_single_root(const float4* __restrict__ box32, BNode* nodes, in
   leaf_prim[0] = 0;
 }
 
-// Leaf-ordered copies for the unbounded searches and the oriented-box fit, which read the
-// triangles of runs of consecutive leaves: the FP32 vertices (3 x float4, as v32) and the LeafTri
-// record, both of the triangle at each sorted leaf.  The record's fields are computed in FP64 from
-// the triangle's vertices (mesh-local) and rounded once.
+// Leaf-ordered copies for the unbounded searches and the oriented-box fit, which read the triangles of
+// runs of consecutive leaves: the FP32 vertices (3 x float4, as v32) and the LeafTri record.
 __global__ void k_leaf_order(const int32_t* __restrict__ leaf_prim, const float4* __restrict__ v32,
-                             const float4* __restrict__ c32,
-                             const TriRec64* __restrict__ rec, int n, double cx, double cy, double cz,
-                             float4* __restrict__ lv32, float4* __restrict__ ltri) {
+                             const float4* __restrict__ tri32, int n, float4* __restrict__ lv32,
+                             float4* __restrict__ ltri) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int prim = leaf_prim[i];
-    lv32[3 * i] = v32[3 * prim];
-    lv32[3 * i + 1] = v32[3 * prim + 1];
-    lv32[3 * i + 2] = v32[3 * prim + 2];
-    const int id = c32[prim].w != 0.f ? prim : (prim | kWeakTri);
-    const double* v = rec[prim].v;
-    const double e0[3] = {v[3] - v[0], v[4] - v[1], v[5] - v[2]};
-    const double e1[3] = {v[6] - v[0], v[7] - v[1], v[8] - v[2]};
-    const double e2[3] = {v[6] - v[3], v[7] - v[4], v[8] - v[5]};
-    const double l0 = e0[0] * e0[0] + e0[1] * e0[1] + e0[2] * e0[2];
-    const double l1 = e1[0] * e1[0] + e1[1] * e1[1] + e1[2] * e1[2];
-    const double l2 = e2[0] * e2[0] + e2[1] * e2[1] + e2[2] * e2[2];
-    const double nx = e0[1] * e1[2] - e0[2] * e1[1], ny = e0[2] * e1[0] - e0[0] * e1[2], nz = e0[0] * e1[1] - e0[1] * e1[0];
-    const double nn = nx * nx + ny * ny + nz * nz;
-    LeafTri T;
-    T.a = make_float4((float)(v[0] - cx), (float)(v[1] - cy), (float)(v[2] - cz), __int_as_float(id));
-    if (nn > 1e-20 * l0 * l1) {
-      const double rn = 1.0 / sqrt(nn), un[3] = {nx * rn, ny * rn, nz * rn};
-      // inward in-plane edge normals: n x (edge direction), edges a->b, b->c, c->a
-      const double* ed[3] = {e0, e2, e1};
-      const double sg[3] = {1.0, 1.0, -1.0};
-      double m[3][3];
-      for (int k = 0; k < 3; ++k) {
-        const double* d = ed[k];
-        const double mx = sg[k] * (un[1] * d[2] - un[2] * d[1]), my = sg[k] * (un[2] * d[0] - un[0] * d[2]),
-                     mz = sg[k] * (un[0] * d[1] - un[1] * d[0]);
-        const double r = 1.0 / sqrt(mx * mx + my * my + mz * mz);
-        m[k][0] = mx * r; m[k][1] = my * r; m[k][2] = mz * r;
-      }
-      T.n = make_float4((float)un[0], (float)un[1], (float)un[2], (float)sqrt(l0));
-      T.m0 = make_float4((float)m[0][0], (float)m[0][1], (float)m[0][2], (float)sqrt(l2));
-      T.m1 = make_float4((float)m[1][0], (float)m[1][1], (float)m[1][2],
-                         (float)(e0[0] * m[1][0] + e0[1] * m[1][1] + e0[2] * m[1][2]));
-      T.m2 = make_float4((float)m[2][0], (float)m[2][1], (float)m[2][2], (float)sqrt(l1));
-    } else {  // no area: the longest edge (see LeafTri)
-      const int k = l0 >= l1 && l0 >= l2 ? 0 : (l1 >= l2 ? 2 : 1);  // edge a->b, c->a or b->c
-      const double* d = k == 0 ? e0 : (k == 1 ? e2 : e1);
-      const double len = sqrt(k == 0 ? l0 : (k == 1 ? l2 : l1));
-      double u[3] = {1.0, 0.0, 0.0};
-      if (len > 0.0)
-        for (int q = 0; q < 3; ++q) u[q] = d[q] / len;
-      const int s = k == 1 ? 3 : 0;  // from b along b->c, else from a
-      // n: the coordinate axis least along u, made normal to it
-      const int j = fabs(u[0]) <= fabs(u[1]) && fabs(u[0]) <= fabs(u[2]) ? 0 : (fabs(u[1]) <= fabs(u[2]) ? 1 : 2);
-      double un[3];
-      for (int q = 0; q < 3; ++q) un[q] = (q == j ? 1.0 : 0.0) - u[j] * u[q];
-      const double rn = 1.0 / sqrt(un[0] * un[0] + un[1] * un[1] + un[2] * un[2]);
-      for (int q = 0; q < 3; ++q) un[q] *= rn;
-      T.a = make_float4((float)(v[s] - cx), (float)(v[s + 1] - cy), (float)(v[s + 2] - cz), __int_as_float(id));
-      T.n = make_float4((float)un[0], (float)un[1], (float)un[2], (float)len);
-      T.m0 = make_float4((float)(un[1] * u[2] - un[2] * u[1]), (float)(un[2] * u[0] - un[0] * u[2]),
-                         (float)(un[0] * u[1] - un[1] * u[0]), 0.f);
-      T.m1 = make_float4(0.f, 0.f, 0.f, kFlat);
-      T.m2 = make_float4(0.f, 0.f, 0.f, -kFlat);
-    }
-    const float4 f[5] = {T.a, T.n, T.m0, T.m1, T.m2};
+    const int64_t prim = leaf_prim[i];
 #pragma unroll
-    for (int k = 0; k < 5; ++k) ltri[(int64_t)k * n + i] = f[k];
+    for (int k = 0; k < 3; ++k) lv32[3 * (int64_t)i + k] = v32[3 * prim + k];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) ltri[(int64_t)k * n + i] = tri32[(int64_t)k * n + prim];
   }
 }
 
@@ -537,7 +559,7 @@ int mesh_upload_and_build(sdfgpu_ctx* ctx, const double* X, int64_t nnp, const i
   SDF_TRY(scratch_t(ctx, "v32", (size_t)nel * 3, &v32));
   SDF_TRY(scratch_t(ctx, "c32", (size_t)nel, &c32));
   SDF_TRY(scratch_t(ctx, "box32", (size_t)nel * 2, &box32));
-  SDF_TRY(scratch_t(ctx, "bbox", 8, &bb));
+  SDF_TRY(scratch_t(ctx, "bbox", 10, &bb));
 
   unsigned long long init[8];
   for (int a = 0; a < 3; ++a) { init[a] = ~0ULL; init[3 + a] = 0ULL; }
@@ -569,10 +591,12 @@ int mesh_upload_and_build(sdfgpu_ctx* ctx, const double* X, int64_t nnp, const i
   }
   M.E = E;
 
-  unsigned long long rho0 = 0ULL;  // below the encoding of every non-negative double
-  SDF_CUDA(ctx, cudaMemcpyAsync(bb + 7, &rho0, sizeof(rho0), cudaMemcpyHostToDevice, st));
+  // rho, rho of the unfit triangles, their number: 0 is below the encoding of every non-negative double
+  SDF_CUDA(ctx, cudaMemsetAsync(bb + 7, 0, 3 * sizeof(unsigned long long), st));
+  float4* tri32;
+  SDF_TRY(scratch_t(ctx, "tri32", (size_t)nel * 5, &tri32));
   k_local32<<<grid_for(nel, 128), 128, 0, st>>>(rec, cent, dIEN, nel, M.center[0], M.center[1], M.center[2], M.E, v32,
-                                                 c32, box32, bb + 7);
+                                                 c32, box32, tri32, bb + 7);
   SDF_KERNEL(ctx);
 
   // LBVH, on its own stream: only the unbounded search, the 3-nearest-vertex fallback and the
@@ -626,8 +650,7 @@ int mesh_upload_and_build(sdfgpu_ctx* ctx, const double* X, int64_t nnp, const i
   float4* ltri;  // LeafTris: five planes
   SDF_TRY(scratch_t(ctx, "lv32", (size_t)n * 3, &lv32));
   SDF_TRY(scratch_t(ctx, "ltri", (size_t)n * 5, &ltri));
-  k_leaf_order<<<grid_for(n, 256), 256, 0, sb>>>(leaf_prim, v32, c32, rec, n, M.center[0], M.center[1], M.center[2], lv32,
-                                                 ltri);
+  k_leaf_order<<<grid_for(n, 256), 256, 0, sb>>>(leaf_prim, v32, tri32, n, lv32, ltri);
   SDF_KERNEL(ctx);
   // the rays and the 3-nearest-vertex fallback need only the tree; the unbounded searches wait for
   // the oriented boxes as well
@@ -640,11 +663,13 @@ int mesh_upload_and_build(sdfgpu_ctx* ctx, const double* X, int64_t nnp, const i
   k_obb_large<<<grid_for(2 * n_inner, 8, 148 * 16), 256, 0, sb>>>(nodes, lv32, n_inner, M.E, obb);
   SDF_KERNEL(ctx);
   SDF_CUDA(ctx, cudaEventRecord(ctx->ev_obb, sb));
-  unsigned long long hrho = 0;
-  SDF_CUDA(ctx, cudaMemcpyAsync(&hrho, bb + 7, sizeof(hrho), cudaMemcpyDeviceToHost, st));
+  unsigned long long hrho[3];
+  SDF_CUDA(ctx, cudaMemcpyAsync(hrho, bb + 7, sizeof(hrho), cudaMemcpyDeviceToHost, st));
   SDF_CUDA(ctx, cudaEventRecord(ctx->ev[5], st));
   SDF_CUDA(ctx, cudaStreamSynchronize(st));
-  M.rho_max = ord_dbl(hrho);
+  M.rho_max = ord_dbl(hrho[0]);
+  M.n_weak = (int64_t)hrho[2];
+  M.rho_weak = M.n_weak ? ord_dbl(hrho[1]) : 0.0;
   float ms = 0.f;
   SDF_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev[4], ctx->ev[5]));
   ctx->stats.ms_mesh = ms;

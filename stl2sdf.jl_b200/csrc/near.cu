@@ -1,0 +1,533 @@
+// near.cu -- the truncated distances (evalDistancesOnTriMesh, src/SignedDistances/dfOnTriangularMesh.jl:19-209)
+// of meshes whose triangles are small against the cell, without closest points: a scatter from the
+// triangles to the nodes within one cell of them instead of candidate lists.
+//
+// Every result is clamped to h (:202-206), and every value the fold can assign for a triangle is at
+// least its true distance, so a node farther than h from all triangles gets h.  For the others let D be
+// the smallest true distance.  A candidate's step (:101-176) assigns, given the running minimum m,
+//   its plane distance when p projects inside;
+//   otherwise F, the smallest distance to a foot on its edges, when F < m;
+//   otherwise V, the smallest distance to its vertices, when V < m.
+// Unless V < F < m can happen, the value does not depend on m: it is face, F or V.  So with the
+// triangles whose distance can equal D (the "ties") the fold's result is the smallest of their values
+// whenever no value depends on m, or those that do cannot go below the others -- or when they share
+// one V and, in index order, some F is not below the F before it: after the earlier one m is at most its
+// F, so the later one's feet do not improve it and V is taken.  Nodes for which none of this holds, and
+// nodes next to a triangle unfit for FP32 decisions, replay the whole fold (k_hard_*).
+// SDFGPU_MODE_EXACT takes the true minimum, so its ties' smallest value is the result.
+//
+// A triangle within h of a node has its centroid within h + rho of it (rho the mesh's largest
+// vertex-to-centroid distance), so for rho < 1.5 h all ties are candidates of the reference rule.
+//
+// Work: the (triangle, node) pairs of the triangles' boxes grown by h -- about 27 a triangle where
+// triangles are small against h -- against the 64 nodes of every tile each triangle's 2.5 h ball reaches.
+// Whole field calls on a B200, tile fold -> scatter: 16.8M nodes, 1.4M triangles, reference rule 7.25 ->
+// 3.61 ms; 33M nodes, 5.8M triangles, true minimum 25.6 -> 16.3 ms; 590k nodes, 131k triangles 1.33 ->
+// 0.77 ms; level at 149k nodes and 5k triangles (0.52 ms, launches).
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+#include "common.cuh"
+#include "unbounded.cuh"
+
+namespace sdfgpu {
+namespace {
+
+constexpr int kSlots = 16;        // triangles kept per near node
+constexpr int kHardCap = 1024;    // candidates listed per hard node (more: the mesh is scanned)
+constexpr int64_t kHardPool = 16 << 20;  // candidates listed in all
+constexpr int kTileShift = 2;     // flags of 4 x 4 x 4 node tiles with hard nodes
+
+struct NearArgs {
+  GridP g;
+  LeafTris tri;         // FP32 records by triangle index
+  const TriRec64* rec;
+  const double4* cent;
+  int64_t nel;
+  bool ref;             // the reference rule, else the true minimum
+  double reach;         // box growth: h plus the margin
+  double ih;            // 1 / h
+  float lim2, eD;       // squared FP32 distance of a near node; error of the FP32 distances
+  float E;
+  double rho;           // the mesh's largest vertex-to-centroid distance (edges are at most 2 rho)
+  double r2, rball;     // the reference's squared candidate radius; a radius that surely contains its ball
+  uint32_t* m2;         // per node: smallest squared FP32 distance (float bits)
+  int32_t* map;         // per near node: its slot index
+  int32_t* near_n;      // number of near nodes
+  int32_t* node;        // near nodes
+  int32_t* cnt;         // triangles in the band of each
+  int32_t* slot;        // kSlots each
+  int32_t* hidx;        // per near node: its hard index, or -1
+  int32_t* hard_n;
+  int32_t* hard;        // near indices of hard nodes
+  uint8_t* tflag;       // tiles with hard nodes
+  int64_t tn[3];
+  float* hbound;        // per hard node: bound on the distances that matter to its fold
+  int32_t* hcnt;        // its candidates within it
+  int64_t* hoff;        // their place in the pool, -1: none
+  int32_t* pool;
+  unsigned long long* pool_n;
+  double* dist;
+  int64_t* counters;
+};
+
+// Nodes of axis a with coordinate in [x0, x1] (grown by 1e-6 cells), as in the tile lists.
+__device__ __forceinline__ bool near_range(const NearArgs& A, int a, double x0, double x1, int& lo, int& hi) {
+  const GridP& g = A.g;
+  const double shift = (double)gidx(g, a, 0);
+  const double f0 = fmax((x0 - g.o[a]) * A.ih - shift - 1e-6, -1.0);
+  const double f1 = fmin((x1 - g.o[a]) * A.ih - shift + 1e-6, (double)g.N[a] + 1.0);
+  if (!(f0 <= f1)) return false;
+  lo = max((int)ceil(f0), 0);
+  hi = (int)min((int64_t)floor(f1), g.N[a]);
+  return lo <= hi;
+}
+
+// kFill false: every node's smallest squared distance, over the nodes near each triangle.  kFill true:
+// each near node's triangles within the band of its minimum.  A thread per triangle: the boxes of one
+// mesh differ little in size, and the triangle's frame stays in registers.  Bound: instruction issue
+// (about 60 per pair), half of the pairs beyond h.
+template <bool kFill>
+__global__ void __launch_bounds__(128) k_near_scatter(const __grid_constant__ NearArgs A) {
+  const GridP& g = A.g;
+  const float hf = (float)g.h;
+  for (int64_t el = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; el < A.nel; el += (int64_t)gridDim.x * blockDim.x) {
+    const TriRec64& r = A.rec[el];
+    int lo[3], hi[3];
+    bool any = true;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const double v0 = r.v[a], v1 = r.v[3 + a], v2 = r.v[6 + a];
+      any = any && near_range(A, a, fmin(v0, fmin(v1, v2)) - A.reach, fmax(v0, fmax(v1, v2)) + A.reach, lo[a], hi[a]);
+    }
+    if (!any) continue;
+    const LeafTri T = A.tri.load((int)el);
+    // the record's vertex a: v1, or the end of the longest edge of a triangle without area
+    const int s = T.m2.w < 0.f && T.m0.w != 0.f ? 3 : 0;
+    const LeafView V = leaf_view(T, f3(T.a));  // from points a + d
+    // nodes relative to a: FP64 differences rounded once, then FP32 steps along x
+    const float x0 = (float)(g.o[0] + g.h * (double)lo[0] - r.v[s]);
+    for (int k = lo[2]; k <= hi[2]; ++k) {
+      const float z = (float)(g.o[2] + g.h * (double)gidx(g, 2, k) - r.v[s + 2]);
+      for (int j = lo[1]; j <= hi[1]; ++j) {
+        const float y = (float)(g.o[1] + g.h * (double)j - r.v[s + 1]);
+        const int64_t row = g.n[0] * (j + g.n[1] * (int64_t)k);
+        for (int i = lo[0]; i <= hi[0]; ++i) {
+          const float d2 = view_d2(V, make_float3(fmaf(hf, (float)(i - lo[0]), x0), y, z));
+          if (!(d2 <= A.lim2)) continue;
+          const int64_t lin = row + i;
+          const uint32_t m = __ldcg(A.m2 + lin);
+          if (!kFill) {
+            if (__float_as_uint(d2) < m) atomicMin(A.m2 + lin, __float_as_uint(d2));
+          } else {
+            const float b = sqrt_approx(__uint_as_float(m)) * (1.f + 1e-6f) + 2.f * A.eD;
+            if (d2 > b * b) continue;
+            const int32_t q = A.map[lin];
+            const int c = atomicAdd(A.cnt + q, 1);
+            if (c < kSlots) A.slot[(int64_t)q * kSlots + c] = __float_as_int(T.a.w);
+          }
+        }
+      }
+    }
+  }
+}
+
+// Lists the near nodes; all others get h.
+__global__ void k_near_nodes(const __grid_constant__ NearArgs A) {
+  const GridP& g = A.g;
+  const int lane = threadIdx.x & 31;
+  for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < g.ngp; base += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t lin = base + threadIdx.x;
+    const bool in = lin < g.ngp;
+    const bool near = in && A.m2[lin] != 0x7f7f7f7fu;
+    if (in && !near) A.dist[lin] = g.h;
+    const unsigned mask = __ballot_sync(0xffffffffu, near);
+    if (!mask) continue;
+    int first = 0;
+    if (lane == 0) first = atomicAdd(A.near_n, __popc(mask));
+    first = __shfl_sync(0xffffffffu, first, 0);
+    if (near) {
+      const int q = first + __popc(mask & ((1u << lane) - 1u));
+      A.map[lin] = q;
+      A.node[q] = (int32_t)lin;
+    }
+  }
+}
+
+__device__ __forceinline__ d3 near_point(const GridP& g, int64_t lin) {
+  const int64_t i = lin % g.n[0], j = (lin / g.n[0]) % g.n[1], k = lin / (g.n[0] * g.n[1]);
+  return gnode(g, i, j, k);
+}
+
+// What the reference's step can assign for a triangle: `face` its plane distance when p projects inside
+// (else NaN), F the smallest distance to a valid foot (INFINITY: none) and V to a vertex -- the
+// expressions of tri_step64 (dfOnTriangularMesh.jl:104-176).
+__device__ __noinline__ void step_values(const TriRec64* __restrict__ rec, int t, const d3& p, double& face, double& F,
+                                         double& V) {
+  const TriRec64& r = rec[t];
+  double lam[3];
+  bary_solve(r, p, lam);
+  const d3 v0 = rec_v(r, 0), v1 = rec_v(r, 1), v2 = rec_v(r, 2);
+  face = nan("");
+  F = V = INFINITY;
+  if (lam[0] >= 0.0 && lam[1] >= 0.0 && lam[2] >= 0.0) {
+    const d3 xp = v_add(v_add(v_scale(v0, lam[0]), v_scale(v1, lam[1])), v_scale(v2, lam[2]));
+    face = v_norm(v_sub(p, xp));
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const d3 vj = rec_v(r, j);
+    const d3 u = {r.u[3 * j], r.u[3 * j + 1], r.u[3 * j + 2]};
+    const double P = v_dot(v_sub(p, vj), u);
+    if (P >= 0.0 && P <= r.L[j]) F = fmin(F, v_norm(v_sub(p, v_add(vj, v_scale(u, P)))));
+    V = fmin(V, v_norm(v_sub(p, vj)));
+  }
+}
+
+// One thread per near node: the result from its ties, or a place in the hard list.
+__global__ void __launch_bounds__(128) k_near_resolve(const __grid_constant__ NearArgs A) {
+  const GridP& g = A.g;
+  const int n_near = *A.near_n;
+  const double tol = 1e-9 * (double)A.E, tol2 = tol * tol;
+  uint32_t fp64 = 0;
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n_near; q += gridDim.x * blockDim.x) {
+    const int64_t lin = A.node[q];
+    const d3 p = near_point(g, lin);
+    int32_t* slot = A.slot + (int64_t)q * kSlots;
+    const int n = A.cnt[q];
+    bool hard = n < 1 || n > kSlots;
+    for (int s = 0; s < n && !hard; ++s) hard = (slot[s] & kWeakTri) != 0;
+    double m = INFINITY;
+    if (!hard) {
+      // the ties, as in lane_filter (unbounded.cuh)
+      double best = 1e300, lim = 1e300;
+      int left = 0;
+#pragma unroll 1
+      for (int s = 0; s < n; ++s) {
+        const int t = slot[s];
+        int feat;
+        const double d2 = near64(A.rec, t, p, tol2, feat);
+        if (d2 > lim) continue;
+        if (d2 < best) {
+          const double dl = 2.0 * tol * (double)sqrtf((float)d2) * (1.0 + 1e-6) + tol2;
+          if (d2 + dl < best) left = 0;
+          best = d2;
+          lim = d2 + dl;
+        }
+        slot[left++] = (int)((unsigned)t | (unsigned)(feat < 0 ? 7 : feat) << kFeatShift);
+      }
+      // in ascending triangle index
+      double Vc = INFINITY, Fprev = INFINITY;
+      int dependent = 0, last = -1;
+      bool sure = false, one_v = true;
+#pragma unroll 1
+      for (int it = 0; it < left; ++it) {
+        unsigned pick = 0u;
+        int tri = 0x7fffffff;
+        for (int s = 0; s < left; ++s) {
+          const unsigned u = (unsigned)slot[s];
+          const int t = (int)(u & kTriMask);
+          if (t > last && t < tri) { tri = t; pick = u; }
+        }
+        last = tri;
+        const int feat = (int)(pick >> kFeatShift);
+        ++fp64;
+        if (feat <= F_EDGE2 || (feat != 7 && !A.ref)) {  // face or edge: whatever m
+          double d;
+          d3 x;
+          feature64(A.rec[tri], p, feat, d, x);
+          m = fmin(m, d);
+          continue;
+        }
+        double face, F, V;
+        step_values(A.rec, tri, p, face, F, V);
+        if (face == face) m = fmin(m, face);
+        else if (!A.ref || !(V < F) || isinf(F)) m = fmin(m, fmin(F, V));
+        else {  // V < F: depends on m
+          if (dependent++ == 0) Vc = V;
+          else {
+            one_v = one_v && V == Vc;
+            sure = sure || F >= Fprev;
+          }
+          if (V < Vc) Vc = V;
+          Fprev = F;
+        }
+      }
+      if (dependent && m > Vc) {  // the values that depend on m can go below the others
+        if (one_v && sure) m = Vc;
+        else hard = true;
+      }
+    }
+    A.hidx[q] = -1;
+    if (hard) {
+      const int hq = atomicAdd(A.hard_n, 1);
+      A.hard[hq] = q;
+      A.hidx[q] = hq;
+      A.hcnt[hq] = 0;
+      A.hbound[hq] = INFINITY;
+      const int64_t i = lin % g.n[0], j = (lin / g.n[0]) % g.n[1], k = lin / (g.n[0] * g.n[1]);
+      A.tflag[((k >> kTileShift) * A.tn[1] + (j >> kTileShift)) * A.tn[0] + (i >> kTileShift)] = 1;
+      continue;
+    }
+    A.dist[lin] = m > g.h ? g.h : m;  // clamp (dfOnTriangularMesh.jl:202-206)
+  }
+  for (int off = 16; off > 0; off >>= 1) fp64 += __shfl_down_sync(0xffffffffu, fp64, off);
+  if ((threadIdx.x & 31) == 0 && fp64) count_add(A.counters, C_FP64, fp64);
+}
+
+// Whether triangle t is a candidate of node p: its centroid in the reference's ball, or for the true
+// minimum its box within reach.
+__device__ __forceinline__ bool hard_candidate(const NearArgs& A, int64_t t, const d3& p) {
+  if (A.ref) {
+    const double4 c = A.cent[t];
+    const double ex = ds(c.x, p.x), ey = ds(c.y, p.y), ez = ds(c.z, p.z);
+    double s = dm(ex, ex);
+    s = da(s, dm(ey, ey));
+    s = da(s, dm(ez, ez));
+    return s <= A.r2;
+  }
+  const TriRec64& r = A.rec[t];
+  return p.x >= r.bmin[0] - A.reach && p.x <= r.bmax[0] + A.reach && p.y >= r.bmin[1] - A.reach &&
+         p.y <= r.bmax[1] + A.reach && p.z >= r.bmin[2] - A.reach && p.z <= r.bmax[2] + A.reach;
+}
+
+// The hard nodes' candidates that matter: every triangle visits the flagged tiles its candidate region
+// reaches.  A step assigns at most the distance to the farthest point of its triangle, so the fold ends
+// at or below U = min over the triangles fit for FP32 decisions of (their distance + 2 rho); a value that
+// can be the result comes from a triangle within U, and whether its feet improve the minimum depends on
+// values up to U + 2 rho.  kPhase 0: that bound per node; 1: the candidates within it counted; 2: listed.
+template <int kPhase>
+__global__ void __launch_bounds__(128) k_hard_collect(const __grid_constant__ NearArgs A) {
+  if (*A.hard_n == 0) return;
+  const GridP& g = A.g;
+  const double tol = 1e-9 * (double)A.E;
+  for (int64_t el = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; el < A.nel; el += (int64_t)gridDim.x * blockDim.x) {
+    int lo[3], hi[3];
+    bool any = true;
+    if (A.ref) {
+      const double4 c4 = A.cent[el];
+      const double c[3] = {c4.x, c4.y, c4.z};
+#pragma unroll
+      for (int a = 0; a < 3; ++a) any = any && near_range(A, a, c[a] - A.rball, c[a] + A.rball, lo[a], hi[a]);
+    } else {
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+        any = any && near_range(A, a, A.rec[el].bmin[a] - A.reach, A.rec[el].bmax[a] + A.reach, lo[a], hi[a]);
+    }
+    if (!any) continue;
+    for (int tz = lo[2] >> kTileShift; tz <= hi[2] >> kTileShift; ++tz)
+      for (int ty = lo[1] >> kTileShift; ty <= hi[1] >> kTileShift; ++ty)
+        for (int tx = lo[0] >> kTileShift; tx <= hi[0] >> kTileShift; ++tx) {
+          if (!A.tflag[((int64_t)tz * A.tn[1] + ty) * A.tn[0] + tx]) continue;
+          constexpr int kT = 1 << kTileShift;
+          for (int k = max(lo[2], tz * kT); k <= min(hi[2], tz * kT + kT - 1); ++k)
+            for (int j = max(lo[1], ty * kT); j <= min(hi[1], ty * kT + kT - 1); ++j)
+              for (int i = max(lo[0], tx * kT); i <= min(hi[0], tx * kT + kT - 1); ++i) {
+                const int64_t lin = i + g.n[0] * (j + g.n[1] * (int64_t)k);
+                if (A.m2[lin] == 0x7f7f7f7fu) continue;
+                const int hq = A.hidx[A.map[lin]];
+                if (hq < 0) continue;
+                const d3 p = gnode(g, i, j, k);
+                if (!hard_candidate(A, el, p)) continue;
+                const bool weak = (__float_as_int(A.tri.at(0, (int)el).w) & kWeakTri) != 0;
+                int feat;
+                const double d = weak ? 0.0 : sqrt(near64(A.rec, (int)el, p, tol * tol, feat));
+                if (kPhase == 0) {
+                  const float b = __double2float_ru(d + 4.0 * A.rho + 4.0 * tol);
+                  if (!weak) atomicMin(reinterpret_cast<int*>(A.hbound + hq), __float_as_int(b));  // non-negative
+                  continue;
+                }
+                if (d - tol > (double)A.hbound[hq]) continue;
+                if (kPhase == 1) {
+                  atomicAdd(A.hcnt + hq, 1);
+                } else if (A.hoff[hq] >= 0) {
+                  A.pool[A.hoff[hq] + atomicAdd(A.hcnt + hq, 1)] = (int32_t)el;
+                }
+              }
+        }
+  }
+}
+
+// Places for the lists (between counting and listing); the counts start again at 0.
+__global__ void k_hard_place(const __grid_constant__ NearArgs A) {
+  const int n_hard = *A.hard_n;
+  for (int hq = blockIdx.x * blockDim.x + threadIdx.x; hq < n_hard; hq += gridDim.x * blockDim.x) {
+    const int c = A.hcnt[hq];
+    int64_t off = -1;
+    if (c <= kHardCap) {
+      off = (int64_t)atomicAdd(A.pool_n, (unsigned long long)c);
+      if (off + c > kHardPool) off = -1;
+    }
+    A.hoff[hq] = off;
+    A.hcnt[hq] = 0;
+  }
+}
+
+// Replays the fold of a hard node, one warp each: the candidates in ascending index 32 at a time, a lane
+// per candidate bounding its distance from below (near64; 0 where that is not certain), and the
+// reference step on those that the running minimum does not exclude (every value a step can assign is at
+// least the true distance).  The few nodes whose list is too long scan the mesh instead.
+__global__ void __launch_bounds__(128) k_hard_replay(const __grid_constant__ NearArgs A) {
+  __shared__ int s_list[4][kHardCap];
+  const GridP& g = A.g;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int n_hard = *A.hard_n;
+  const double tol = 1e-9 * (double)A.E;
+  uint32_t fp64 = 0;
+  for (int hq = blockIdx.x * 4 + w; hq < n_hard; hq += gridDim.x * 4) {
+    const int64_t lin = A.node[A.hard[hq]];
+    const d3 p = near_point(g, lin);
+    double m = kBig;
+    d3 proj = {0.0, 0.0, 0.0};
+    auto batch = [&](int t) {  // this lane's candidate, or -1; ascending over the lanes
+      double lb = INFINITY;
+      if (t >= 0) {
+        int feat;
+        lb = (__float_as_int(A.tri.at(0, t).w) & kWeakTri) ? 0.0
+                                                           : sqrt(near64(A.rec, t, p, tol * tol, feat)) - tol;
+      }
+      for (unsigned todo = __ballot_sync(0xffffffffu, lb <= m); todo; todo &= todo - 1u) {
+        const int src = __ffs(todo) - 1;
+        if (!(__shfl_sync(0xffffffffu, lb, src) <= m)) continue;
+        tri_step64(A.rec[__shfl_sync(0xffffffffu, t, src)], p, m, proj, A.ref);
+        ++fp64;
+      }
+    };
+    if (A.hoff[hq] >= 0) {
+      const int n = A.hcnt[hq];
+      int *list = s_list[w], *sorted = A.pool + A.hoff[hq];
+      for (int s = lane; s < n; s += 32) list[s] = sorted[s];
+      __syncwarp();
+      for (int s = lane; s < n; s += 32) {  // rank sort (the indices are distinct)
+        const int t = list[s];
+        int rank = 0;
+        for (int o = 0; o < n; ++o) rank += list[o] < t;
+        sorted[rank] = t;
+      }
+      __syncwarp();
+      for (int base = 0; base < n; base += 32) batch(base + lane < n ? sorted[base + lane] : -1);
+    } else {
+      for (int64_t base = 0; base < A.nel; base += 32) {
+        const int64_t t = base + lane;
+        const bool in = t < A.nel && hard_candidate(A, t, p);
+        if (__any_sync(0xffffffffu, in)) batch(in ? (int)t : -1);
+      }
+    }
+    if (lane == 0) A.dist[lin] = m > g.h ? g.h : m;
+    __syncwarp();
+  }
+  if (lane == 0 && fp64) count_add(A.counters, C_FP64, fp64);
+}
+
+}  // namespace
+
+// Whether near_distances takes this call: triangles of at most 1.5 (reference rule) or 4 cells from their
+// centroid, the mesh near the coordinate origin (see unb_mesh), and few and small triangles unfit for
+// FP32 decisions, each of which sends the nodes nearest to it to the replay.
+bool near_applies(const sdfgpu_ctx* ctx, const GridP& g, int mode) {
+  const MeshDev& M = ctx->mesh;
+  double off = 0.0;
+  for (int a = 0; a < 3; ++a) off = std::max(off, std::fabs(M.center[a]));
+  const double rho = M.rho_max * (1.0 + 1e-9) + 1e-6 * g.E;
+  return off <= 64.0 * M.E && rho < (mode == SDFGPU_MODE_REF_RULE ? 1.5 : 4.0) * g.h && M.rho_weak <= 1.5 * g.h &&
+         M.n_weak <= M.nel / 64;
+}
+
+// The two parts of the stage: near_prepare finds every node's nearest distance in FP32 and the near nodes
+// (whose number the host waits for, to size their slots); near_run the results.
+static_assert(sizeof(NearArgs) <= sizeof(DistPlan::fold), "DistPlan::fold holds a NearArgs");
+
+int near_prepare(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, DistPlan& Pl) {
+  cudaStream_t st = ctx->stream;
+  const MeshDev& M = ctx->mesh;
+  NearArgs A{};
+  A.g = g;
+  A.tri = LeafTris{buf<float4>(ctx, "tri32"), M.nel};
+  A.rec = buf<TriRec64>(ctx, "rec");
+  A.cent = buf<double4>(ctx, "cent64");
+  A.nel = M.nel;
+  A.ref = mode == SDFGPU_MODE_REF_RULE;
+  // FP32 distances in the triangle's own frame: every rounding is relative to |p - a| + the edges, at most
+  // d + 4 rho + 2 rho; below 1e-6 of that in all (see view_d2)
+  A.eD = (float)(1.5e-6 * (g.h + 6.0 * M.rho_max));
+  const double lim = (g.h + 4.0 * (double)A.eD) * (1.0 + 1e-6);
+  A.lim2 = (float)(lim * lim);
+  A.reach = lim * (1.0 + 1e-9) + 1e-9 * g.E;
+  A.ih = 1.0 / g.h;
+  A.E = (float)g.E;
+  A.rho = M.rho_max;
+  const double sr = 2.5 * g.h;
+  A.r2 = sr * sr;
+  A.rball = sr * (1.0 + 1e-9) + 1e-6 * g.E;
+  A.dist = d_dist;
+  A.counters = ctx->d_counters;
+  int64_t tiles = 1;
+  for (int a = 0; a < 3; ++a) {
+    A.tn[a] = (g.n[a] >> kTileShift) + 1;
+    tiles *= A.tn[a];
+  }
+  int32_t* counts;  // near nodes, hard nodes
+  SDF_TRY(scratch_t(ctx, "near_m2", (size_t)g.ngp, &A.m2));
+  SDF_TRY(scratch_t(ctx, "near_map", (size_t)g.ngp, &A.map));
+  SDF_TRY(scratch_t(ctx, "near_node", (size_t)g.ngp, &A.node));
+  SDF_TRY(scratch_t(ctx, "near_counts", 2, &counts));
+  SDF_TRY(scratch_t(ctx, "near_tflag", (size_t)tiles, &A.tflag));
+  A.near_n = counts;
+  A.hard_n = counts + 1;
+  SDF_CUDA(ctx, cudaMemsetAsync(A.m2, 0x7f, sizeof(uint32_t) * g.ngp, st));  // 3.39e38
+  SDF_CUDA(ctx, cudaMemsetAsync(counts, 0, 2 * sizeof(int32_t), st));
+  SDF_CUDA(ctx, cudaMemsetAsync(A.tflag, 0, (size_t)tiles, st));
+  const unsigned gt = grid_for(M.nel, 128, 148 * 64);
+  k_near_scatter<false><<<gt, 128, 0, st>>>(A);
+  SDF_KERNEL(ctx);
+  k_near_nodes<<<grid_for(g.ngp, 256, 148 * 16), 256, 0, st>>>(A);
+  SDF_KERNEL(ctx);
+  int32_t n_near = 0;
+  SDF_CUDA(ctx, cudaMemcpyAsync(&n_near, A.near_n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+  SDF_CUDA(ctx, cudaStreamSynchronize(st));
+  SDF_TRY(scratch_t(ctx, "near_cnt", (size_t)n_near, &A.cnt));
+  SDF_TRY(scratch_t(ctx, "near_slot", (size_t)n_near * kSlots, &A.slot));
+  SDF_TRY(scratch_t(ctx, "near_hidx", (size_t)n_near, &A.hidx));
+  SDF_TRY(scratch_t(ctx, "near_hard", (size_t)n_near, &A.hard));
+  SDF_TRY(scratch_t(ctx, "near_hbound", (size_t)n_near, &A.hbound));
+  SDF_TRY(scratch_t(ctx, "near_hcnt", (size_t)n_near, &A.hcnt));
+  SDF_TRY(scratch_t(ctx, "near_hoff", (size_t)n_near, &A.hoff));
+  SDF_TRY(scratch_t(ctx, "near_pool", (size_t)kHardPool, &A.pool));
+  SDF_TRY(scratch_t(ctx, "near_pool_n", 1, &A.pool_n));
+  std::memcpy(Pl.fold, &A, sizeof(A));
+  Pl.g = g;
+  Pl.nonempty = n_near;
+  return 0;
+}
+
+int near_run(sdfgpu_ctx* ctx, const DistPlan& Pl) {
+  cudaStream_t st = ctx->stream;
+  NearArgs A;
+  std::memcpy(&A, Pl.fold, sizeof(A));
+  const int64_t n = Pl.nonempty;
+  ctx->h_counters[C_BAND] = n;
+  if (n == 0) return 0;
+  SDF_CUDA(ctx, cudaMemsetAsync(A.cnt, 0, sizeof(int32_t) * n, st));
+  const unsigned gt = grid_for(A.nel, 128, 148 * 64);
+  k_near_scatter<true><<<gt, 128, 0, st>>>(A);
+  SDF_KERNEL(ctx);
+  k_near_resolve<<<grid_for(n, 128, 148 * 32), 128, 0, st>>>(A);
+  SDF_KERNEL(ctx);
+  // these return at once when no node is hard
+  SDF_CUDA(ctx, cudaMemsetAsync(A.pool_n, 0, sizeof(unsigned long long), st));
+  k_hard_collect<0><<<gt, 128, 0, st>>>(A);
+  SDF_KERNEL(ctx);
+  k_hard_collect<1><<<gt, 128, 0, st>>>(A);
+  SDF_KERNEL(ctx);
+  k_hard_place<<<grid_for(n, 256, 148), 256, 0, st>>>(A);
+  SDF_KERNEL(ctx);
+  k_hard_collect<2><<<gt, 128, 0, st>>>(A);
+  SDF_KERNEL(ctx);
+  k_hard_replay<<<grid_for(n, 4, 148 * 8), 128, 0, st>>>(A);
+  SDF_KERNEL(ctx);
+  return 0;
+}
+
+}  // namespace sdfgpu
