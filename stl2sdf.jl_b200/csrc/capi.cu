@@ -256,6 +256,7 @@ int run_all(sdfgpu_ctx* ctx, const GridP& g, bool want_dist, bool want_sign, int
   auto join = [&]() {
     if (forked && cudaEventRecord(ctx->ev_join, ss) == cudaSuccess) cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0);
     forked = false;
+    cudaStreamWaitEvent(ctx->stream, ctx->ev_bvh, 0);
     cudaStreamWaitEvent(ctx->stream, ctx->ev_obb, 0);
   };
   auto stages = [&]() -> int {

@@ -96,6 +96,7 @@ struct MeshDev {
   double rho_weak = 0.0; // the same over the triangles unfit for FP32 decisions
   int64_t n_weak = 0;    // their number
   bool ine_ready = false;
+  int tree = 0;          // 1: the LBVH is built or enqueued, 2: its oriented boxes too
 };
 
 struct DevBuf {
@@ -111,6 +112,7 @@ struct sdfgpu_ctx {
   cudaEvent_t ev[6] = {};
   std::string err;
   int32_t tile[3] = {4, 4, 4};
+  int tree_used = 0;             // what the resident mesh's calls needed: 1 the LBVH, 2 its boxes too
   bool tune_tiles = false;       // the autotuner times the tile fold (run_distances)
   int32_t brick[3] = {4, 2, 4};  // nodes of one warp in the unbounded search (product 32)
   bool has_mesh = false;
@@ -247,6 +249,7 @@ int make_grid(sdfgpu_ctx* ctx, const double origin[3], double h, const int64_t N
 int mesh_upload_and_build(sdfgpu_ctx* ctx, const double* X, int64_t nnp, const int64_t* IEN, int64_t nel,
                           bool device_ptrs);
 int ensure_ine(sdfgpu_ctx* ctx);
+int ensure_tree(sdfgpu_ctx* ctx, bool boxes);
 int run_distances(sdfgpu_ctx* ctx, const GridP& g, int mode, int use_learned, double* d_dist, double* d_xp);
 // Exact unbounded distances of a sparse grid's nodes, one thread per node (learned.cu).
 int run_nearest_points(sdfgpu_ctx* ctx, const GridP& g, double* d_dist);

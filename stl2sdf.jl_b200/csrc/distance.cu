@@ -624,6 +624,7 @@ void unb_tree(sdfgpu_ctx* ctx, const GridP& g, const int32_t b[3], double* d_dis
 // The unbounded search's arguments for grid g on the current mesh, with the learned radius of every brick when use_learned and the network's bound
 // is on; the context stream waits for the LBVH and its oriented boxes.
 int unb_setup(sdfgpu_ctx* ctx, const GridP& g, int use_learned, double* d_dist, double* d_xp, UnbArgs& A) {
+  SDF_TRY(ensure_tree(ctx, true));
   SDF_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->ev_obb, 0));  // the search walks the LBVH and its oriented boxes
   unb_tree(ctx, g, ctx->brick, d_dist, d_xp, A);
   if (use_learned) {
@@ -823,6 +824,7 @@ int dist_prepare(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, doub
     const bool big_tris = M.rho_max * (1.0 + 1e-9) + 1e-6 * g.E >= 1.5 * g.h;
     if (big_tris || d_xp) {
       SDF_TRY(ensure_ine(ctx));
+      SDF_TRY(ensure_tree(ctx, true));
       uint8_t* band = nullptr;
       if (!d_xp) SDF_TRY(scratch_t(ctx, "band", (size_t)g.ngp, &band));
       KnnArgs K;

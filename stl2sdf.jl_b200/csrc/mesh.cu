@@ -529,6 +529,84 @@ __global__ void k_ine_fill(const int64_t* __restrict__ IEN, int64_t nel, const i
 
 }  // namespace
 
+// The LBVH of the resident mesh and, with `boxes`, its oriented child boxes, built on first use on a stream
+// of their own: only the unbounded searches, the 3-nearest-vertex fallback (both with the boxes) and the
+// adaptive rays of many nodes read them, and wait for ev_obb or ev_bvh; the clamped distances and the
+// axis rays do not.  (Building them for every mesh took a third of a reference-rule call on 1.4M
+// triangles.)  set_mesh enqueues at once what the last mesh's calls used (ctx->tree_used), so that a
+// program of unbounded calls overlaps the build as before.
+int ensure_tree(sdfgpu_ctx* ctx, bool boxes) {
+  MeshDev& M = ctx->mesh;
+  ctx->tree_used = std::max(ctx->tree_used, boxes ? 2 : 1);
+  const int64_t nel = M.nel;
+  const int n = (int)nel;
+  cudaStream_t sb = ctx->bvh_stream;
+  BNode* nodes = buf<BNode>(ctx, "nodes");
+  float4* lv32 = buf<float4>(ctx, "lv32");
+  if (M.tree < 1) {
+    float4 *v32 = buf<float4>(ctx, "v32"), *c32 = buf<float4>(ctx, "c32"), *box32 = buf<float4>(ctx, "box32"),
+           *tri32 = buf<float4>(ctx, "tri32");
+    SDF_CUDA(ctx, cudaStreamWaitEvent(sb, ctx->ev_mesh, 0));
+    unsigned long long* keys2;
+    int32_t *int_parent, *leaf_parent, *flags, *leaf_prim;
+    SDF_TRY(scratch_t(ctx, "keys2", (size_t)n, &keys2));
+    SDF_TRY(scratch_t(ctx, "nodes", (size_t)std::max(1, n - 1), &nodes));
+    SDF_TRY(scratch_t(ctx, "int_parent", (size_t)n, &int_parent));
+    SDF_TRY(scratch_t(ctx, "leaf_parent", (size_t)n, &leaf_parent));
+    SDF_TRY(scratch_t(ctx, "flags", (size_t)n, &flags));
+    SDF_TRY(scratch_t(ctx, "leaf_prim", (size_t)n, &leaf_prim));
+    if (n == 1) {
+      k_single_root<<<1, 1, 0, sb>>>(box32, nodes, leaf_prim);
+      SDF_KERNEL(ctx);
+    } else {
+      const float lox = (float)(M.bmin[0] - M.center[0]), loy = (float)(M.bmin[1] - M.center[1]),
+                  loz = (float)(M.bmin[2] - M.center[2]);
+      const double ext = std::max(M.bmax[0] - M.bmin[0], std::max(M.bmax[1] - M.bmin[1], M.bmax[2] - M.bmin[2]));
+      const float inv = ext > 0 ? (float)(1024.0 / ext) : 1.0f;
+      uint32_t *code, *code2;
+      int32_t *idx, *idx2;
+      SDF_TRY(scratch_t(ctx, "mcode", (size_t)n, &code));
+      SDF_TRY(scratch_t(ctx, "mcode2", (size_t)n, &code2));
+      SDF_TRY(scratch_t(ctx, "midx", (size_t)n, &idx));
+      SDF_TRY(scratch_t(ctx, "midx2", (size_t)n, &idx2));
+      k_morton<<<grid_for(nel, 256), 256, 0, sb>>>(c32, nel, lox, loy, loz, inv, code, idx);
+      SDF_KERNEL(ctx);
+      size_t tmp_bytes = 0;
+      SDF_CUDA(ctx, cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, code, code2, idx, idx2, n, 0, 30, sb));
+      void* tmp;
+      SDF_TRY(scratch(ctx, "cub_tmp_bvh", tmp_bytes, &tmp));
+      SDF_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, code, code2, idx, idx2, n, 0, 30, sb));
+      k_pack_keys<<<grid_for(n, 256), 256, 0, sb>>>(code2, idx2, n, keys2);
+      SDF_KERNEL(ctx);
+      SDF_CUDA(ctx, cudaMemsetAsync(int_parent, 0xff, sizeof(int32_t) * n, sb));
+      SDF_CUDA(ctx, cudaMemsetAsync(flags, 0, sizeof(int32_t) * n, sb));
+      k_karras<<<grid_for(n - 1, 256), 256, 0, sb>>>(keys2, n, nodes, int_parent, leaf_parent);
+      SDF_KERNEL(ctx);
+      k_refit<<<grid_for(n, 256), 256, 0, sb>>>(keys2, box32, n, nodes, int_parent, leaf_parent, flags, leaf_prim);
+      SDF_KERNEL(ctx);
+    }
+    float4* ltri;  // LeafTris: five planes
+    SDF_TRY(scratch_t(ctx, "lv32", (size_t)n * 3, &lv32));
+    SDF_TRY(scratch_t(ctx, "ltri", (size_t)n * 5, &ltri));
+    k_leaf_order<<<grid_for(n, 256), 256, 0, sb>>>(leaf_prim, v32, tri32, n, lv32, ltri);
+    SDF_KERNEL(ctx);
+    SDF_CUDA(ctx, cudaEventRecord(ctx->ev_bvh, sb));
+    M.tree = 1;
+  }
+  if (boxes && M.tree < 2) {
+    OBox* obb;
+    const int n_inner = std::max(1, n - 1);
+    SDF_TRY(scratch_t(ctx, "obb", (size_t)2 * n_inner, &obb));
+    k_obb_small<<<grid_for(2 * n_inner, 256), 256, 0, sb>>>(nodes, lv32, n_inner, M.E, obb);
+    SDF_KERNEL(ctx);
+    k_obb_large<<<grid_for(2 * n_inner, 8, 148 * 16), 256, 0, sb>>>(nodes, lv32, n_inner, M.E, obb);
+    SDF_KERNEL(ctx);
+    SDF_CUDA(ctx, cudaEventRecord(ctx->ev_obb, sb));
+    M.tree = 2;
+  }
+  return 0;
+}
+
 int mesh_upload_and_build(sdfgpu_ctx* ctx, const double* X, int64_t nnp, const int64_t* IEN, int64_t nel,
                           bool device_ptrs) {
   cudaStream_t st = ctx->stream;
@@ -538,7 +616,11 @@ int mesh_upload_and_build(sdfgpu_ctx* ctx, const double* X, int64_t nnp, const i
   ctx->has_mesh = false;
   ctx->mesh.ine_ready = false;
   ctx->launches = 0;
+  const int eager = ctx->tree_used;  // what the last mesh's calls needed, before set_mesh's own host wait
+  ctx->tree_used = 0;
+  ctx->mesh.tree = 0;
   // the previous mesh's LBVH build reads the buffers rewritten below
+  SDF_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_bvh, 0));
   SDF_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_obb, 0));
   SDF_CUDA(ctx, cudaEventRecord(ctx->ev[4], st));
 
@@ -599,70 +681,9 @@ int mesh_upload_and_build(sdfgpu_ctx* ctx, const double* X, int64_t nnp, const i
                                                  c32, box32, tri32, bb + 7);
   SDF_KERNEL(ctx);
 
-  // LBVH, on its own stream: only the unbounded search, the 3-nearest-vertex fallback and the
-  // adaptive rays read it, and they wait for ev_bvh (the unbounded search for ev_obb, which also
-  // covers the oriented boxes); the tile lists and the fold do not, so the build overlaps the
-  // distance stage of the next call.
   SDF_CUDA(ctx, cudaEventRecord(ctx->ev_mesh, st));
-  cudaStream_t sb = ctx->bvh_stream;
-  SDF_CUDA(ctx, cudaStreamWaitEvent(sb, ctx->ev_mesh, 0));
-  const int n = (int)nel;
-  unsigned long long* keys2;
-  BNode* nodes;
-  int32_t *int_parent, *leaf_parent, *flags, *leaf_prim;
-  SDF_TRY(scratch_t(ctx, "keys2", (size_t)n, &keys2));
-  SDF_TRY(scratch_t(ctx, "nodes", (size_t)std::max(1, n - 1), &nodes));
-  SDF_TRY(scratch_t(ctx, "int_parent", (size_t)n, &int_parent));
-  SDF_TRY(scratch_t(ctx, "leaf_parent", (size_t)n, &leaf_parent));
-  SDF_TRY(scratch_t(ctx, "flags", (size_t)n, &flags));
-  SDF_TRY(scratch_t(ctx, "leaf_prim", (size_t)n, &leaf_prim));
-  if (n == 1) {
-    k_single_root<<<1, 1, 0, sb>>>(box32, nodes, leaf_prim);
-    SDF_KERNEL(ctx);
-  } else {
-    const float lox = (float)(M.bmin[0] - M.center[0]), loy = (float)(M.bmin[1] - M.center[1]),
-                loz = (float)(M.bmin[2] - M.center[2]);
-    const double ext = std::max(M.bmax[0] - M.bmin[0], std::max(M.bmax[1] - M.bmin[1], M.bmax[2] - M.bmin[2]));
-    const float inv = ext > 0 ? (float)(1024.0 / ext) : 1.0f;
-    uint32_t *code, *code2;
-    int32_t *idx, *idx2;
-    SDF_TRY(scratch_t(ctx, "mcode", (size_t)n, &code));
-    SDF_TRY(scratch_t(ctx, "mcode2", (size_t)n, &code2));
-    SDF_TRY(scratch_t(ctx, "midx", (size_t)n, &idx));
-    SDF_TRY(scratch_t(ctx, "midx2", (size_t)n, &idx2));
-    k_morton<<<grid_for(nel, 256), 256, 0, sb>>>(c32, nel, lox, loy, loz, inv, code, idx);
-    SDF_KERNEL(ctx);
-    size_t tmp_bytes = 0;
-    SDF_CUDA(ctx, cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, code, code2, idx, idx2, n, 0, 30, sb));
-    void* tmp;
-    SDF_TRY(scratch(ctx, "cub_tmp_bvh", tmp_bytes, &tmp));
-    SDF_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, code, code2, idx, idx2, n, 0, 30, sb));
-    k_pack_keys<<<grid_for(n, 256), 256, 0, sb>>>(code2, idx2, n, keys2);
-    SDF_KERNEL(ctx);
-    SDF_CUDA(ctx, cudaMemsetAsync(int_parent, 0xff, sizeof(int32_t) * n, sb));
-    SDF_CUDA(ctx, cudaMemsetAsync(flags, 0, sizeof(int32_t) * n, sb));
-    k_karras<<<grid_for(n - 1, 256), 256, 0, sb>>>(keys2, n, nodes, int_parent, leaf_parent);
-    SDF_KERNEL(ctx);
-    k_refit<<<grid_for(n, 256), 256, 0, sb>>>(keys2, box32, n, nodes, int_parent, leaf_parent, flags, leaf_prim);
-    SDF_KERNEL(ctx);
-  }
-  float4* lv32;
-  float4* ltri;  // LeafTris: five planes
-  SDF_TRY(scratch_t(ctx, "lv32", (size_t)n * 3, &lv32));
-  SDF_TRY(scratch_t(ctx, "ltri", (size_t)n * 5, &ltri));
-  k_leaf_order<<<grid_for(n, 256), 256, 0, sb>>>(leaf_prim, v32, tri32, n, lv32, ltri);
-  SDF_KERNEL(ctx);
-  // the rays and the 3-nearest-vertex fallback need only the tree; the unbounded searches wait for
-  // the oriented boxes as well
-  SDF_CUDA(ctx, cudaEventRecord(ctx->ev_bvh, sb));
-  OBox* obb;
-  const int n_inner = std::max(1, n - 1);
-  SDF_TRY(scratch_t(ctx, "obb", (size_t)2 * n_inner, &obb));
-  k_obb_small<<<grid_for(2 * n_inner, 256), 256, 0, sb>>>(nodes, lv32, n_inner, M.E, obb);
-  SDF_KERNEL(ctx);
-  k_obb_large<<<grid_for(2 * n_inner, 8, 148 * 16), 256, 0, sb>>>(nodes, lv32, n_inner, M.E, obb);
-  SDF_KERNEL(ctx);
-  SDF_CUDA(ctx, cudaEventRecord(ctx->ev_obb, sb));
+  if (eager) SDF_TRY(ensure_tree(ctx, eager > 1));
+  ctx->tree_used = 0;
   unsigned long long hrho[3];
   SDF_CUDA(ctx, cudaMemcpyAsync(hrho, bb + 7, sizeof(hrho), cudaMemcpyDeviceToHost, st));
   SDF_CUDA(ctx, cudaEventRecord(ctx->ev[5], st));

@@ -34,6 +34,7 @@ namespace {
 constexpr double kEps = 1e-8;  // check_ray_inside_bvh default (:118), passed to MT (:132)
 constexpr int kRowCap = 64;    // hits per row a node sorts in registers/local memory
 constexpr int kRayCap = 256;   // hits per generic ray
+constexpr int64_t kAllPairsNodes = 64;  // undecided nodes whose rays may test every triangle
 constexpr int kStack = 64;
 
 // A row hit: the Möller–Trumbore constants of one triangle for one grid row, from which each node
@@ -604,6 +605,74 @@ __global__ void __launch_bounds__(128) k_rays(RayArgs A, int round) {
   if ((threadIdx.x & 31) == 0 && band) count_add(A.counters, C_SIGN_BAND, band);
 }
 
+// The rays of a few undecided nodes against every triangle, without the LBVH (which then need not be
+// built): one thread per triangle, all requested rays.  Most pairs end at a distance test of the
+// triangle's centroid from the ray's line; the rest take the tests of ray_parity, so the hits are the same.
+// Bound: that test, about 15 FP32 instructions a pair.
+__global__ void __launch_bounds__(128) k_rays_all(RayArgs A, const float4* __restrict__ c32, int64_t nel, float reach,
+                                                  int32_t* __restrict__ hit_n, double* __restrict__ hit_t) {
+  const GridP& g = A.g;
+  const int count = (int)A.rq_cnt[0];
+  int64_t band = 0;
+  for (int64_t el = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; el < nel; el += (int64_t)gridDim.x * blockDim.x) {
+    const float4 c = c32[el];
+    for (int t = 0; t < count; ++t) {
+      const int64_t lin = A.list[A.req_node[t]];
+      const int64_t i = lin % g.n[0], j = (lin / g.n[0]) % g.n[1], k = lin / (g.n[0] * g.n[1]);
+      const d3 p = gnode(g, i, j, k);
+      const double* dir = c_dirs + 3 * (A.req_ray[t] - 1);
+      const float dx = (float)dir[0], dy = (float)dir[1], dz = (float)dir[2];
+      const float wx = c.x - (float)(p.x - g.center[0]), wy = c.y - (float)(p.y - g.center[1]),
+                  wz = c.z - (float)(p.z - g.center[2]);
+      // distance of the centroid from the line: |w - (w . d) d|, d a unit vector
+      const float s = fmaf(wx, dx, fmaf(wy, dy, wz * dz));
+      const float qx = fmaf(-s, dx, wx), qy = fmaf(-s, dy, wy), qz = fmaf(-s, dz, wz);
+      if (fmaf(qx, qx, fmaf(qy, qy, qz * qz)) > reach * reach || s < -reach) continue;
+      const TriRec64& r = A.rec[el];
+      const d3 d = {dir[0], dir[1], dir[2]};
+      const int dec = mt32(p, d, rec_v(r, 0), rec_v(r, 1), rec_v(r, 2));
+      if (dec == 0) continue;
+      if (dec == 2) ++band;
+      double tt;
+      if (mt64(p, d, rec_v(r, 0), rec_v(r, 1), rec_v(r, 2), kEps, tt)) {
+        const int q = atomicAdd(hit_n + t, 1);
+        if (q < kRayCap) hit_t[(int64_t)t * kRayCap + q] = tt;
+      }
+    }
+  }
+  for (int off = 16; off > 0; off >>= 1) band += __shfl_down_sync(0xffffffffu, band, off);
+  if ((threadIdx.x & 31) == 0 && band) count_add(A.counters, C_SIGN_BAND, band);
+}
+
+// Parities of those rays from their hits: sorted, distinct within eps (:114-154).
+__global__ void k_rays_parity(RayArgs A, const int32_t* __restrict__ hit_n, double* __restrict__ hit_t) {
+  const int count = (int)A.rq_cnt[0];
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
+    const int n = hit_n[t];
+    int parity = 0;
+    if (n > kRayCap) {
+      count_add(A.counters, C_ERR_CAPACITY, 1);
+    } else if (n > 0) {
+      double* ts = hit_t + (int64_t)t * kRayCap;
+      for (int a = 1; a < n; ++a) {
+        const double v = ts[a];
+        int b = a;
+        while (b > 0 && ts[b - 1] > v) { ts[b] = ts[b - 1]; --b; }
+        ts[b] = v;
+      }
+      int unique = 1;
+      for (int a = 1; a < n; ++a)
+        if (fabs(ds(ts[a], ts[a - 1])) > kEps) ++unique;
+      parity = unique & 1;
+    }
+    const int64_t q = A.req_node[t];
+    const uint64_t bit = 1ULL << (A.req_ray[t] - 1);
+    if (parity) atomicOr((unsigned long long*)&A.parbits[q], (unsigned long long)bit);
+    atomicOr((unsigned long long*)&A.have[q], (unsigned long long)bit);
+    count_add(A.counters, C_EXTRA_RAYS, 1);
+  }
+}
+
 // generalized_winding_number (:295-328).  The triangles are cut into fixed chunks; one CTA sums
 // one chunk for one node (fixed-order block reduction) and k_winding_final adds the chunk sums
 // in chunk order, so the result does not depend on scheduling and one node still fills the GPU.
@@ -783,7 +852,13 @@ int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int 
     SDF_TRY(scratch_t(ctx, "rq_cnt", (size_t)kRounds + 1, &rq_cnt));
     SDF_CUDA(ctx, cudaMemsetAsync(done, 0, (size_t)nund, st));
     SDF_CUDA(ctx, cudaMemsetAsync(rq_cnt, 0, sizeof(int64_t) * (kRounds + 1), st));
-    SDF_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_bvh, 0));  // the adaptive rays walk the LBVH
+    // Few (ray, triangle) pairs: all of them, at about 0.5 ps each (24 rays x 1.4M triangles in 20 us)
+    // instead of walks of the LBVH whose latency (0.28 ms there) and build (0.6 ms) they would pay for.
+    const bool all_pairs = nund <= kAllPairsNodes && (double)nund * 30.0 * (double)nel <= 4.0e8;
+    if (!all_pairs) {
+      SDF_TRY(ensure_tree(ctx, false));
+      SDF_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_bvh, 0));  // the adaptive rays walk the LBVH
+    }
     RayArgs R;
     R.g = g;
     R.nodes = buf<BNode>(ctx, "nodes");
@@ -813,7 +888,19 @@ int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int 
     for (int r = 0; r < rounds; ++r) {
       k_round<<<grid_for(nund, 128), 128, 0, st>>>(R, nund, r, 0);
       SDF_KERNEL(ctx);
-      k_rays<<<grid_for(nund * 8, 128, 148 * 32), 128, 0, st>>>(R, r);
+      if (all_pairs) {
+        int32_t* hit_n;
+        double* hit_t;
+        SDF_TRY(scratch_t(ctx, "ray_hit_n", (size_t)nund * 36, &hit_n));
+        SDF_TRY(scratch_t(ctx, "ray_hit_t", (size_t)nund * 36 * kRayCap, &hit_t));
+        SDF_CUDA(ctx, cudaMemsetAsync(hit_n, 0, sizeof(int32_t) * nund * 36, st));
+        const float reach = (float)(M.rho_max * (1.0 + 1e-5) + 4e-6 * g.E);
+        k_rays_all<<<grid_for(nel, 128, 148 * 64), 128, 0, st>>>(R, buf<float4>(ctx, "c32"), nel, reach, hit_n, hit_t);
+        SDF_KERNEL(ctx);
+        k_rays_parity<<<grid_for(nund * 36, 64), 64, 0, st>>>(R, hit_n, hit_t);
+      } else {
+        k_rays<<<grid_for(nund * 8, 128, 148 * 32), 128, 0, st>>>(R, r);
+      }
       SDF_KERNEL(ctx);
     }
     k_round<<<grid_for(nund, 128), 128, 0, st>>>(R, nund, kRounds, 1);

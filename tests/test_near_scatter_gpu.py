@@ -102,3 +102,17 @@ def test_slab_and_signed(gpu_ctx, mode):
     for k0, k1 in ((0, 0), (3, 8), (13, 13)):
         part = gpu_ctx.sdf_slab(o, h, N, k0, k1, mode)
         assert np.array_equal(part, full[n * k0:n * (k1 + 1)])
+
+
+@pytest.mark.parametrize("n", [3, 5, 7, 9, 16])
+@pytest.mark.parametrize("drop", [1, 40, 200])
+def test_adaptive_rays_of_few_and_many_nodes(gpu_ctx, n, drop):
+    """An open surface on growing grids: the undecided nodes' rays go against all triangles while they are
+    few and through the LBVH beyond; signs and confidences equal the oracle's either way."""
+    V, F = synthetic.icosphere(3, jitter=0.05, seed=7)
+    F = np.ascontiguousarray(np.delete(F, np.random.default_rng(n).choice(len(F), drop, replace=False), axis=0))
+    o, h, N = np.full(3, -1.21), 2.37 / n, np.array([n, n, n])
+    gpu_ctx.set_mesh(V, F)
+    s, c = gpu_ctx.signs(o, h, N)
+    ref = oracle.signs(V, F, o, h, N)
+    assert np.array_equal(s, ref["sign"]) and np.array_equal(c, ref["conf"])
