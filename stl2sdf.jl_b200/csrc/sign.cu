@@ -11,16 +11,18 @@
 //     the node's x.  And the -x ray of the same node sees a = -a, f = -f, the same u and v, and
 //     t = -t exactly.  So one list of (row, triangle) hits per axis serves both directions of
 //     every node of the row.  The lists are built by a triangle scatter over the rows its
-//     projected box covers (FP64 decisions, exactly the reference's); each node then evaluates
-//     only t for the hits of its three rows with the reference's formula, sorts, de-duplicates
-//     within eps and takes parities.  A warp walks 32 consecutive nodes of one row, so the row's
-//     hits are broadcast loads.
+//     projected box covers (FP64 decisions, exactly the reference's).  t is linear in the node's
+//     coordinate with slope -1, so a hit's coordinate and a bound of the rounding of t split the row's
+//     nodes into those certainly below the hit, those certainly above it, and a node or none within the
+//     bound; and the gaps between the row's hits say which of them merge within eps.  So a row's parities
+//     are bit masks over its nodes, made of one prefix per distinct hit.  Where a node lies within the
+//     bound of a hit, or a gap is near eps, the node evaluates t for all hits of the row with the
+//     reference's formula, sorts, de-duplicates within eps and takes parities.
 //   * Nodes whose 6 votes disagree continue with the reference's batches on the LBVH: FP32 slab
 //     tests with an explicit margin prune, FP64 Möller–Trumbore decides.
 //   * Nodes left with confidence < threshold sum the winding number over all triangles, one CTA
 //     per node with a fixed-order block reduction.
-#include <cub/cub.cuh>
-
+#include <algorithm>
 #include <cstring>
 
 #include "common.cuh"
@@ -39,12 +41,11 @@ constexpr int kStack = 64;
 
 // A row hit: the Möller–Trumbore constants of one triangle for one grid row, from which each node
 // of the row gets t with the reference's operation order (see the per-axis formulas below).
-struct __align__(16) RowHit {
+struct RowHit {
   double v1a;  // v1 coordinate along the row axis
   double K1, K2, P;
   double ea, eb, fa, fb;
   double f;
-  double key;  // approximate hit coordinate along the axis (row ordering only)
 };
 
 template <int AX>
@@ -99,7 +100,6 @@ __device__ __forceinline__ bool row_test(const TriRec64& r, double ob, double oc
       R.v1a = v1.z; R.K1 = dm(s.y, e1.z); R.K2 = dm(s.x, e1.z); R.P = dm(e2.z, q.z);
       R.ea = e1.y; R.eb = e1.x; R.fa = e2.x; R.fb = e2.y;
     }
-    R.key = R.v1a + row_t<AX>(R, R.v1a);
     *out = R;
   }
   return true;
@@ -170,7 +170,7 @@ __device__ __forceinline__ bool axis_range2(const GridP& g, int a, double x0, do
 template <int AX>
 __device__ __forceinline__ void tri_rows(const GridP& g, const TriRec64& r, bool fill, int64_t row_base,
                                          int32_t* row_cnt, const int32_t* row_off, int32_t* row_cur, RowHit* hits,
-                                         unsigned long long* rkey, int32_t* ridx, int64_t& nhit, int64_t& nband) {
+                                         double2* where, int64_t& nhit, int64_t& nband) {
   const int b = AX == 0 ? 1 : 0, c = AX == 2 ? 1 : 2;
   int64_t b0, b1, c0, c1;
   if (!axis_range2(g, b, r.bmin[b], r.bmax[b], b0, b1)) return;
@@ -190,11 +190,14 @@ __device__ __forceinline__ void tri_rows(const GridP& g, const TriRec64& r, bool
         if (row_test<AX>(r, ob, oc, &R)) {  // the hit's FP64 constants (and the band's decision)
           const int32_t pos = row_off[row] + atomicAdd(&row_cur[row], 1);
           hits[pos] = R;
-          // sort key: row in the high word, the hit coordinate (ordered float bits) in the low word
-          uint32_t u = __float_as_uint((float)R.key);
-          u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-          rkey[pos] = ((unsigned long long)row << 32) | u;
-          ridx[pos] = pos;
+          // the hit's coordinate, and a bound on |t - (coordinate - xa)| over the row's nodes: t is formed
+          // from terms of these absolute sums by at most a dozen roundings, f's own error among them
+          const double x0 = g.o[AX] + g.h * (double)gidx(g, AX, 0), x1 = g.o[AX] + g.h * (double)gidx(g, AX, g.N[AX]);
+          const double S = fmax(fabs(x0 - R.v1a), fabs(x1 - R.v1a));
+          const double sum = fabs(R.P) + fabs(R.fa) * (fabs(R.K1) + S * fabs(R.ea)) +
+                             fabs(R.fb) * (fabs(R.K2) + S * fabs(R.eb));
+          const double x = R.v1a + row_t<AX>(R, R.v1a), e = 7.2e-15 * (fabs(R.f) * sum + S + fabs(R.v1a));
+          where[pos] = make_double2(x, e);
         }
       }
     }
@@ -203,13 +206,13 @@ __device__ __forceinline__ void tri_rows(const GridP& g, const TriRec64& r, bool
 
 __global__ void k_rows(const TriRec64* __restrict__ rec, int64_t nel, GridP g, int64_t base_y, int64_t base_z,
                        bool fill, int32_t* row_cnt, const int32_t* row_off, int32_t* row_cur, RowHit* hits,
-                       unsigned long long* rkey, int32_t* ridx, int64_t* counters) {
+                       double2* where, int64_t* counters) {
   int64_t nhit = 0, nband = 0;
   for (int64_t el = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; el < nel; el += (int64_t)gridDim.x * blockDim.x) {
     const TriRec64 r = rec[el];
-    tri_rows<0>(g, r, fill, 0, row_cnt, row_off, row_cur, hits, rkey, ridx, nhit, nband);
-    tri_rows<1>(g, r, fill, base_y, row_cnt, row_off, row_cur, hits, rkey, ridx, nhit, nband);
-    tri_rows<2>(g, r, fill, base_z, row_cnt, row_off, row_cur, hits, rkey, ridx, nhit, nband);
+    tri_rows<0>(g, r, fill, 0, row_cnt, row_off, row_cur, hits, where, nhit, nband);
+    tri_rows<1>(g, r, fill, base_y, row_cnt, row_off, row_cur, hits, where, nhit, nband);
+    tri_rows<2>(g, r, fill, base_z, row_cnt, row_off, row_cur, hits, where, nhit, nband);
   }
   if (!fill) {
     for (int off = 16; off > 0; off >>= 1) {
@@ -221,11 +224,36 @@ __global__ void k_rows(const TriRec64* __restrict__ rec, int64_t nel, GridP g, i
   }
 }
 
-// Gathers the row hits into (row, hit coordinate) order after the radix sort of their keys.
-__global__ void k_gather_rows(int64_t n, const int32_t* __restrict__ order, const RowHit* __restrict__ src,
-                              RowHit* __restrict__ dst) {
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x)
-    dst[q] = src[order[q]];
+// Per row: the first hit, and their number with two flags.  Hits certainly within eps / 4 of one another
+// are one hit to every node outside their bounds: all but the first get a negative bound (its magnitude
+// stays), and kRowOdd says whether the number of distinct hits is odd.  kRowClose: two hits of the row
+// are neither that close nor certainly more than eps apart, or there are too many of them to compare
+// (then over[0] counts the row too).
+constexpr int kRowClose = 1 << 30, kRowOdd = 1 << 29, kRowCount = kRowOdd - 1;
+__global__ void k_row_info(int64_t nrows, const int32_t* __restrict__ row_off, const int32_t* __restrict__ row_cnt,
+                           double2* __restrict__ where, int2* __restrict__ info, int32_t* __restrict__ over) {
+  for (int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; row < nrows; row += (int64_t)gridDim.x * blockDim.x) {
+    const int off = row_off[row], n = row_cnt[row];
+    bool close = n > kRowCap;
+    if (close) atomicAdd(over, 1);
+    int distinct = n;
+    for (int a = 1; a < n && !close; ++a) {
+      const double2 p = where[off + a];
+      bool same = false;
+      for (int b = 0; b < a && !close; ++b) {
+        const double2 q = where[off + b];
+        const double gap = fabs(p.x - q.x), e = 2.0 * (p.y + fabs(q.y));
+        const bool near = gap + e < 0.25 * kEps;
+        same = same || near;
+        close = !near && !(gap > kEps + e);
+      }
+      if (same) {
+        where[off + a].y = -p.y;
+        --distinct;
+      }
+    }
+    info[row] = make_int2(off, n | (close ? kRowClose : 0) | ((distinct & 1) ? kRowOdd : 0));
+  }
 }
 
 // Number of distinct hits (gaps > eps) among sorted t values passing the direction's t > eps.
@@ -252,34 +280,76 @@ __device__ __forceinline__ int clusters_neg(const double* ts, int n) {
   return c;
 }
 
-// Parities of the +AX / -AX rays of every node.  Thread order runs along the AX rows.
-// par bit0: +AX inside, bit1: -AX inside, bit7: row overflow (node takes the generic path).
+// Parities of the +AX / -AX rays at coordinate xa of a row, from t of all its hits (bit 0: +AX, bit 1: -AX).
 template <int AX>
-__global__ void __launch_bounds__(256) k_axis_parity(GridP g, int64_t row_base, const int32_t* __restrict__ row_off,
-                                                     const int32_t* __restrict__ row_cnt,
-                                                     const RowHit* __restrict__ hits, uint8_t* __restrict__ par) {
-  const int b = AX == 0 ? 1 : 0, c = AX == 2 ? 1 : 2;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < g.ngp; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t ia = t % g.n[AX];
-    const int64_t rest = t / g.n[AX];
-    const int64_t jb = rest % g.n[b], jc = rest / g.n[b];
-    int64_t idx[3];
-    idx[AX] = ia; idx[b] = jb; idx[c] = jc;
-    const int64_t lin = idx[0] + g.n[0] * (idx[1] + g.n[1] * idx[2]);
-    const int64_t row = row_base + jc * g.n[b] + jb;
-    const int32_t off = row_off[row], n = row_cnt[row];
-    if (n > kRowCap) { par[lin] = 0x80; continue; }
-    const double xa = da(g.o[AX], dm(g.h, (double)gidx(g, AX, ia)));
-    double ts[kRowCap];
-    for (int q = 0; q < n; ++q) {
-      const double tv = row_t<AX>(hits[off + q], xa);
-      int p = q - 1;
-      while (p >= 0 && ts[p] > tv) { ts[p + 1] = ts[p]; --p; }
-      ts[p + 1] = tv;
-    }
-    const int cp = clusters_pos(ts, n), cn = clusters_neg(ts, n);
-    par[lin] = (uint8_t)((cp & 1) | ((cn & 1) << 1));
+__device__ __noinline__ uint8_t row_parity(const RowHit* __restrict__ hits, int n, double xa) {
+  double ts[kRowCap];
+  for (int q = 0; q < n; ++q) {
+    const double tv = row_t<AX>(hits[q], xa);
+    int p = q - 1;
+    while (p >= 0 && ts[p] > tv) { ts[p + 1] = ts[p]; --p; }
+    ts[p + 1] = tv;
   }
+  return (uint8_t)((clusters_pos(ts, n) & 1) | ((clusters_neg(ts, n) & 1) << 1));
+}
+
+struct MaskArgs {
+  GridP g;
+  int64_t nrows[3], base[3];  // rows along x, y, z, and the first of each among all rows
+  int64_t mbase[4];           // first mask word of each axis, and their number
+  const int2* info;
+  const RowHit* hits;
+  const double2* where;
+  uint2* mask;  // per axis [word of 32 nodes][row]: bits of the +AX and of the -AX ray
+};
+
+// One thread per row and 32 of its nodes.  Bound: the reads of the rows' hits, which the words of a row
+// share in L2.
+template <int AX>
+__device__ __forceinline__ void row_mask(const MaskArgs& A, int64_t q) {
+  const GridP& g = A.g;
+  const int64_t word = q / A.nrows[AX], row = q - word * A.nrows[AX];
+  const int2 in = A.info[A.base[AX] + row];
+  const int n = in.y & kRowCount;
+  uint2 m = make_uint2(0u, 0u);
+  if (n > 0 && n <= kRowCap) {
+    const int first = (int)(word * 32), last = (int)min((int64_t)31, g.n[AX] - 1 - first);  // this word's nodes
+    unsigned exact = (in.y & kRowClose) ? 0xffffffffu : 0u;
+    if (!exact) {
+      const double o = g.o[AX] + g.h * (double)gidx(g, AX, 0), inv = 1.0 / g.h;
+      const double slack = fabs(g.o[AX]) * inv + (double)g.n[AX] + 1.0;
+      for (int a = 0; a < n; ++a) {
+        const double2 c = A.where[in.x + a];
+        // the hit in nodes from the row's first, and the half width of the window around it in which t's
+        // sign against eps is open (eps, t's bound, and the roundings of this line and of the nodes)
+        const double r = (c.x - o) * inv;
+        const double w = 1.01 * (kEps + fabs(c.y)) * inv + 1e-13 * (fabs(r) + fabs(c.x) * inv + slack);
+        if (!(fabs(r) + w < 1e9)) { exact = 0xffffffffu; break; }
+        const int lo = max(0, min(32, (int)ceil(r - w) - first)), hi = max(-1, min(31, (int)floor(r + w) - first));
+        const unsigned below = lo == 32 ? 0xffffffffu : (1u << lo) - 1u;  // nodes below the hit
+        if (!signbit(c.y)) m.x ^= below;
+        if (hi >= lo) exact |= (0xffffffffu >> (31 - hi)) & ~below;
+      }
+      m.y = (in.y & kRowOdd) ? ~m.x : m.x;
+    }
+    exact &= 0xffffffffu >> (31 - last);
+    while (exact) {
+      const int b = __ffs(exact) - 1;
+      exact &= exact - 1u;
+      const unsigned par = row_parity<AX>(A.hits + in.x, n, da(g.o[AX], dm(g.h, (double)gidx(g, AX, first + b))));
+      m.x = (m.x & ~(1u << b)) | ((par & 1u) << b);
+      m.y = (m.y & ~(1u << b)) | ((par >> 1) << b);
+    }
+  }
+  A.mask[A.mbase[AX] + q] = m;
+}
+
+__global__ void __launch_bounds__(128) k_row_masks(const __grid_constant__ MaskArgs A) {
+  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (q >= A.mbase[3]) return;
+  if (q < A.mbase[1]) row_mask<0>(A, q);
+  else if (q < A.mbase[2]) row_mask<1>(A, q - A.mbase[1]);
+  else row_mask<2>(A, q - A.mbase[2]);
 }
 
 // adaptive_point_in_mesh_raycast (:234-288).  cast(i) returns the parity of ray i (1-based) or
@@ -318,7 +388,7 @@ __device__ __forceinline__ int vote_logic(int min_rays, int max_rays, Cast cast,
   return 0;
 }
 
-__device__ __forceinline__ int axis_bit(uint8_t px, uint8_t py, uint8_t pz, int i) {
+__device__ __forceinline__ int axis_bit(unsigned px, unsigned py, unsigned pz, int i) {
   // rays 1..6: +X +Y +Z -X -Y -Z
   switch (i) {
     case 1: return px & 1;
@@ -332,7 +402,10 @@ __device__ __forceinline__ int axis_bit(uint8_t px, uint8_t py, uint8_t pz, int 
 
 struct VoteArgs {
   GridP g;
-  const uint8_t* par[3];
+  const uint2* mask[3];     // the axes' masks, [word][row]
+  const int32_t* row_cnt;   // rows along x, then y, then z
+  const int32_t* over;      // rows with more than kRowCap hits
+  uint32_t tiles[3];
   int min_rays, max_rays;
   double conf_thresh;
   int use_winding;
@@ -345,34 +418,94 @@ struct VoteArgs {
   int64_t* counters;
 };
 
-__global__ void k_vote(VoteArgs A) {
+// The vote of a node whose six rays differ (or that cannot be decided here): the result, or its place in
+// the lists of the nodes that go on.
+__device__ __noinline__ void vote_node(const VoteArgs& A, int64_t lin, unsigned px, unsigned py, unsigned pz, bool ovf) {
+  double s, cf;
+  int total;
+  if (vote_logic(A.min_rays, A.max_rays, [&](int r) { return (r <= 6 && !ovf) ? axis_bit(px, py, pz, r) : -1; }, s, cf,
+                 total)) {
+    const int64_t slot = atomicAdd((unsigned long long*)&A.counters[C_LIST_UNDECIDED], 1ULL);
+    A.und_list[slot] = (int32_t)lin;
+    uint64_t have = 0, par = 0;
+    if (!ovf) {
+      have = 0x3FULL;
+      for (int r = 1; r <= 6; ++r) par |= (uint64_t)axis_bit(px, py, pz, r) << (r - 1);
+    }
+    A.und_have[slot] = have;
+    A.und_par[slot] = par;
+    return;
+  }
+  if (A.use_winding && cf < A.conf_thresh) {
+    const int64_t slot = atomicAdd((unsigned long long*)&A.counters[C_LIST_WINDING], 1ULL);
+    A.wind_list[slot] = (int32_t)lin;
+    cf = 0.8;
+  }
+  A.sign[lin] = s;
+  if (A.conf) A.conf[lin] = cf;
+}
+
+// The vote of every node from the rows' masks: one warp per 32 x kVoteJ x kVoteK nodes, a lane per column, so
+// that a mask word is read once for kVoteJ or kVoteK nodes of a lane.  Measured on 16.8M nodes and 321k hits
+// (B200): 52 us, and 23 us for the masks and the rows' flags, against 0.78 ms for a pass per axis in row order (which evaluated every
+// t, and wrote its parities a sector per byte along y and z) and the vote, 0.10 ms for the radix sort of
+// the hits that it needed, and 0.22 ms for comparing each node with its rows' hits.  Bound: the 8 or 16 bytes
+// a node it writes.
+constexpr int kVoteJ = 4, kVoteK = 4;
+static_assert(32 % kVoteJ == 0 && 32 % kVoteK == 0 && kVoteJ * kVoteK <= 32, "a tile's rows lie in one word");
+__global__ void __launch_bounds__(256) k_vote(const __grid_constant__ VoteArgs A) {
   const GridP& g = A.g;
-  for (int64_t lin = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; lin < g.ngp; lin += (int64_t)gridDim.x * blockDim.x) {
-    const uint8_t px = A.par[0][lin], py = A.par[1][lin], pz = A.par[2][lin];
-    const bool ovf = ((px | py | pz) & 0x80) != 0;
-    double s, cf;
-    int total;
-    const int rc = vote_logic(A.min_rays, A.max_rays,
-                              [&](int i) { return (i <= 6 && !ovf) ? axis_bit(px, py, pz, i) : -1; }, s, cf, total);
-    if (rc) {
-      const int64_t slot = atomicAdd((unsigned long long*)&A.counters[C_LIST_UNDECIDED], 1ULL);
-      A.und_list[slot] = (int32_t)lin;
-      uint64_t have = 0, par = 0;
-      if (!ovf) {
-        have = 0x3FULL;
-        for (int r = 1; r <= 6; ++r) par |= (uint64_t)axis_bit(px, py, pz, r) << (r - 1);
+  const int lane = threadIdx.x & 31;
+  const int nx = (int)g.n[0], ny = (int)g.n[1], nz = (int)g.n[2];
+  const bool over = *A.over != 0;
+  const uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const uint32_t tj = w / A.tiles[0], ti = w - tj * A.tiles[0], tk = tj / A.tiles[1];
+  if (tk >= A.tiles[2]) return;
+  const int i = (int)ti * 32 + lane, j0 = (int)(tj - tk * A.tiles[1]) * kVoteJ, k0 = (int)tk * kVoteK;
+  const bool in = i < nx;
+  uint2 mx = make_uint2(0u, 0u), my[kVoteK], mz[kVoteJ];
+  {
+    const int j = j0 + lane % kVoteJ, k = k0 + lane / kVoteJ;
+    if (lane < kVoteJ * kVoteK && j < ny && k < nz) mx = A.mask[0][(int64_t)ti * ((int64_t)ny * nz) + (int64_t)k * ny + j];
+  }
+#pragma unroll
+  for (int k = 0; k < kVoteK; ++k) {
+    my[k] = make_uint2(0u, 0u);
+    if (in && k0 + k < nz) my[k] = A.mask[1][(int64_t)(j0 >> 5) * ((int64_t)nx * nz) + (int64_t)(k0 + k) * nx + i];
+    my[k].x >>= j0 & 31;
+    my[k].y >>= j0 & 31;
+  }
+#pragma unroll
+  for (int j = 0; j < kVoteJ; ++j) {
+    mz[j] = make_uint2(0u, 0u);
+    if (in && j0 + j < ny) mz[j] = A.mask[2][(int64_t)(k0 >> 5) * ((int64_t)nx * ny) + (int64_t)(j0 + j) * nx + i];
+    mz[j].x >>= k0 & 31;
+    mz[j].y >>= k0 & 31;
+  }
+#pragma unroll
+  for (int k = 0; k < kVoteK; ++k) {
+#pragma unroll
+    for (int j = 0; j < kVoteJ; ++j) {
+      const unsigned xp = __shfl_sync(0xffffffffu, mx.x, k * kVoteJ + j), xn = __shfl_sync(0xffffffffu, mx.y, k * kVoteJ + j);
+      if (!in || j0 + j >= ny || k0 + k >= nz) continue;
+      const int64_t lin = ((int64_t)(k0 + k) * ny + (j0 + j)) * nx + i;
+      const unsigned px = ((xp >> lane) & 1u) | (((xn >> lane) & 1u) << 1);
+      const unsigned py = ((my[k].x >> j) & 1u) | (((my[k].y >> j) & 1u) << 1);
+      const unsigned pz = ((mz[j].x >> k) & 1u) | (((mz[j].y >> k) & 1u) << 1);
+      bool ovf = false;
+      if (over) {
+        const int64_t Rx = (int64_t)ny * nz, Ry = (int64_t)nx * nz;
+        ovf = A.row_cnt[(int64_t)(k0 + k) * ny + (j0 + j)] > kRowCap || A.row_cnt[Rx + (int64_t)(k0 + k) * nx + i] > kRowCap ||
+              A.row_cnt[Rx + Ry + (int64_t)(j0 + j) * nx + i] > kRowCap;
       }
-      A.und_have[slot] = have;
-      A.und_par[slot] = par;
-      continue;
+      const unsigned all = px & py & pz, any = px | py | pz;
+      if (A.min_rays == 6 && !ovf && (all == 3u || any == 0u) && !(A.use_winding && 1.0 < A.conf_thresh)) {
+        A.sign[lin] = any ? 1.0 : -1.0;  // six equal rays: ratio 1 or 0, confidence 1
+        if (A.conf) A.conf[lin] = 1.0;
+      } else {
+        vote_node(A, lin, px, py, pz, ovf);
+      }
     }
-    if (A.use_winding && cf < A.conf_thresh) {
-      const int64_t slot = atomicAdd((unsigned long long*)&A.counters[C_LIST_WINDING], 1ULL);
-      A.wind_list[slot] = (int32_t)lin;
-      cf = 0.8;
-    }
-    A.sign[lin] = s;
-    if (A.conf) A.conf[lin] = cf;
   }
 }
 
@@ -383,7 +516,6 @@ struct RayArgs {
   const TriRec64* rec;
   float pad;
   int64_t max_visits;
-  const uint8_t* par[3];
   const int32_t* list;
   int min_rays, max_rays;
   double conf_thresh;
@@ -609,34 +741,49 @@ __global__ void __launch_bounds__(128) k_rays(RayArgs A, int round) {
 // built): one thread per triangle, all requested rays.  Most pairs end at a distance test of the
 // triangle's centroid from the ray's line; the rest take the tests of ray_parity, so the hits are the same.
 // Bound: that test, about 15 FP32 instructions a pair.
+constexpr int kAllRays = 128;  // requests held in shared memory at a time
 __global__ void __launch_bounds__(128) k_rays_all(RayArgs A, const float4* __restrict__ c32, int64_t nel, float reach,
                                                   int32_t* __restrict__ hit_n, double* __restrict__ hit_t) {
+  __shared__ float4 s_o[kAllRays], s_d[kAllRays];  // origin (mesh-local) and direction, .w of the first: node index
   const GridP& g = A.g;
   const int count = (int)A.rq_cnt[0];
   int64_t band = 0;
-  for (int64_t el = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; el < nel; el += (int64_t)gridDim.x * blockDim.x) {
-    const float4 c = c32[el];
-    for (int t = 0; t < count; ++t) {
-      const int64_t lin = A.list[A.req_node[t]];
+  for (int base = 0; base < count; base += kAllRays) {
+    const int m = min(kAllRays, count - base);
+    __syncthreads();
+    for (int t = threadIdx.x; t < m; t += blockDim.x) {
+      const int64_t lin = A.list[A.req_node[base + t]];
       const int64_t i = lin % g.n[0], j = (lin / g.n[0]) % g.n[1], k = lin / (g.n[0] * g.n[1]);
       const d3 p = gnode(g, i, j, k);
-      const double* dir = c_dirs + 3 * (A.req_ray[t] - 1);
-      const float dx = (float)dir[0], dy = (float)dir[1], dz = (float)dir[2];
-      const float wx = c.x - (float)(p.x - g.center[0]), wy = c.y - (float)(p.y - g.center[1]),
-                  wz = c.z - (float)(p.z - g.center[2]);
-      // distance of the centroid from the line: |w - (w . d) d|, d a unit vector
-      const float s = fmaf(wx, dx, fmaf(wy, dy, wz * dz));
-      const float qx = fmaf(-s, dx, wx), qy = fmaf(-s, dy, wy), qz = fmaf(-s, dz, wz);
-      if (fmaf(qx, qx, fmaf(qy, qy, qz * qz)) > reach * reach || s < -reach) continue;
-      const TriRec64& r = A.rec[el];
-      const d3 d = {dir[0], dir[1], dir[2]};
-      const int dec = mt32(p, d, rec_v(r, 0), rec_v(r, 1), rec_v(r, 2));
-      if (dec == 0) continue;
-      if (dec == 2) ++band;
-      double tt;
-      if (mt64(p, d, rec_v(r, 0), rec_v(r, 1), rec_v(r, 2), kEps, tt)) {
-        const int q = atomicAdd(hit_n + t, 1);
-        if (q < kRayCap) hit_t[(int64_t)t * kRayCap + q] = tt;
+      const double* dir = c_dirs + 3 * (A.req_ray[base + t] - 1);
+      s_o[t] = make_float4((float)(p.x - g.center[0]), (float)(p.y - g.center[1]), (float)(p.z - g.center[2]),
+                           __int_as_float((int)lin));
+      s_d[t] = make_float4((float)dir[0], (float)dir[1], (float)dir[2], __int_as_float(A.req_ray[base + t] - 1));
+    }
+    __syncthreads();
+    for (int64_t el = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; el < nel; el += (int64_t)gridDim.x * blockDim.x) {
+      const float4 c = c32[el];
+      for (int t = 0; t < m; ++t) {
+        const float4 o = s_o[t], d = s_d[t];
+        // distance of the centroid from the line: |w - (w . d) d|, d a unit vector
+        const float wx = c.x - o.x, wy = c.y - o.y, wz = c.z - o.z;
+        const float s = fmaf(wx, d.x, fmaf(wy, d.y, wz * d.z));
+        const float qx = fmaf(-s, d.x, wx), qy = fmaf(-s, d.y, wy), qz = fmaf(-s, d.z, wz);
+        if (fmaf(qx, qx, fmaf(qy, qy, qz * qz)) > reach * reach || s < -reach) continue;
+        const int64_t lin = __float_as_int(o.w);
+        const int64_t i = lin % g.n[0], j = (lin / g.n[0]) % g.n[1], k = lin / (g.n[0] * g.n[1]);
+        const d3 p = gnode(g, i, j, k);
+        const double* dir = c_dirs + 3 * __float_as_int(d.w);
+        const d3 dd3 = {dir[0], dir[1], dir[2]};
+        const TriRec64& r = A.rec[el];
+        const int dec = mt32(p, dd3, rec_v(r, 0), rec_v(r, 1), rec_v(r, 2));
+        if (dec == 0) continue;
+        if (dec == 2) ++band;
+        double tt;
+        if (mt64(p, dd3, rec_v(r, 0), rec_v(r, 1), rec_v(r, 2), kEps, tt)) {
+          const int q = atomicAdd(hit_n + base + t, 1);
+          if (q < kRayCap) hit_t[(int64_t)(base + t) * kRayCap + q] = tt;
+        }
       }
     }
   }
@@ -753,7 +900,7 @@ int sign_begin(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P) {
   SDF_CUDA(ctx, cudaMemsetAsync(P.row_cnt, 0, sizeof(int32_t) * (P.nrows + 1), st));
   SDF_CUDA(ctx, cudaMemsetAsync(P.row_cur, 0, sizeof(int32_t) * (P.nrows + 1), st));
   k_rows<<<grid_for(nel, 128), 128, 0, st>>>(rec, nel, g, P.Rx, P.Rx + P.Ry, false, P.row_cnt, nullptr, nullptr,
-                                             nullptr, nullptr, nullptr, ctx->d_counters);
+                                             nullptr, nullptr, ctx->d_counters);
   SDF_KERNEL(ctx);
   SDF_TRY(cub_scan_i32(ctx, P.row_cnt, P.row_off, P.nrows + 1, st, "cub_tmp_scan_sign"));
   ctx->h_scalars[S_ROW_TOTAL] = -1;
@@ -775,43 +922,40 @@ int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int 
   int32_t total;
   std::memcpy(&total, ctx->h_scalars + S_ROW_TOTAL, sizeof(int32_t));  // the low 4 bytes hold the int32
   if (total < 0) return fail(ctx, SDFGPU_ERR_CAPACITY, "more than 2^31 row hits");
-  RowHit *hits_raw, *hits;
-  unsigned long long *rkey, *rkey2;
-  int32_t *ridx, *ridx2;
+  RowHit* hits;
+  double2* where;
+  int2* info;
+  int32_t* over;
+  MaskArgs K;
   const size_t H = (size_t)std::max(total, 1);
-  SDF_TRY(scratch_t(ctx, "row_hits_raw", H, &hits_raw));
   SDF_TRY(scratch_t(ctx, "row_hits", H, &hits));
-  SDF_TRY(scratch_t(ctx, "row_key", H, &rkey));
-  SDF_TRY(scratch_t(ctx, "row_key2", H, &rkey2));
-  SDF_TRY(scratch_t(ctx, "row_idx", H, &ridx));
-  SDF_TRY(scratch_t(ctx, "row_idx2", H, &ridx2));
+  SDF_TRY(scratch_t(ctx, "row_where", H, &where));
+  SDF_TRY(scratch_t(ctx, "row_info", (size_t)nrows, &info));
+  SDF_TRY(scratch_t(ctx, "row_over", (size_t)1, &over));
+  SDF_CUDA(ctx, cudaMemsetAsync(over, 0, sizeof(int32_t), st));
+  K.nrows[0] = Rx;
+  K.nrows[1] = Ry;
+  K.nrows[2] = P.Rz;
+  K.base[0] = 0;
+  K.base[1] = Rx;
+  K.base[2] = Rx + Ry;
+  K.mbase[0] = 0;
+  for (int a = 0; a < 3; ++a) K.mbase[a + 1] = K.mbase[a] + cdiv(g.n[a], 32) * K.nrows[a];
+  SDF_TRY(scratch_t(ctx, "row_mask", (size_t)K.mbase[3], &K.mask));
   if (total > 0) {
-    k_rows<<<grid_for(nel, 128), 128, 0, st>>>(rec, nel, g, Rx, Rx + Ry, true, nullptr, row_off, row_cur, hits_raw,
-                                               rkey, ridx, ctx->d_counters);
-    SDF_KERNEL(ctx);
-    int bits = 32;
-    while (bits < 64 && (1LL << (bits - 32)) < nrows) ++bits;
-    size_t tmp_bytes = 0;
-    SDF_CUDA(ctx, cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, rkey, rkey2, ridx, ridx2, total, 0, bits, st));
-    void* tmp;
-    SDF_TRY(scratch(ctx, "cub_tmp_sign", tmp_bytes, &tmp));
-    SDF_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, rkey, rkey2, ridx, ridx2, total, 0, bits, st));
-    k_gather_rows<<<grid_for(total, 256), 256, 0, st>>>(total, ridx2, hits_raw, hits);
+    k_rows<<<grid_for(nel, 128), 128, 0, st>>>(rec, nel, g, Rx, Rx + Ry, true, nullptr, row_off, row_cur, hits, where,
+                                               ctx->d_counters);
     SDF_KERNEL(ctx);
   }
-  uint8_t *px, *py, *pz;
-  SDF_TRY(scratch_t(ctx, "par_x", (size_t)g.ngp, &px));
-  SDF_TRY(scratch_t(ctx, "par_y", (size_t)g.ngp, &py));
-  SDF_TRY(scratch_t(ctx, "par_z", (size_t)g.ngp, &pz));
-  const unsigned gp = grid_for(g.ngp, 256, 148 * 16);
+  k_row_info<<<grid_for(nrows, 256), 256, 0, st>>>(nrows, row_off, row_cnt, where, info, over);
+  SDF_KERNEL(ctx);
   SDF_MARK_ON(ctx, T_ROWS, st);
-  k_axis_parity<0><<<gp, 256, 0, st>>>(g, 0, row_off, row_cnt, hits, px);
+  K.g = g;
+  K.info = info;
+  K.hits = hits;
+  K.where = where;
+  k_row_masks<<<(unsigned)cdiv(K.mbase[3], 128), 128, 0, st>>>(K);
   SDF_KERNEL(ctx);
-  k_axis_parity<1><<<gp, 256, 0, st>>>(g, Rx, row_off, row_cnt, hits, py);
-  SDF_KERNEL(ctx);
-  k_axis_parity<2><<<gp, 256, 0, st>>>(g, Rx + Ry, row_off, row_cnt, hits, pz);
-  SDF_KERNEL(ctx);
-  SDF_MARK_ON(ctx, T_PARITY, st);
 
   int32_t *und, *wind;
   uint64_t *und_have, *und_par;
@@ -821,7 +965,12 @@ int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int 
   SDF_TRY(scratch_t(ctx, "wind_list", (size_t)g.ngp, &wind));
   VoteArgs V;
   V.g = g;
-  V.par[0] = px; V.par[1] = py; V.par[2] = pz;
+  for (int a = 0; a < 3; ++a) V.mask[a] = K.mask + K.mbase[a];
+  V.row_cnt = row_cnt;
+  V.over = over;
+  V.tiles[0] = (uint32_t)cdiv(g.n[0], 32);
+  V.tiles[1] = (uint32_t)cdiv(g.n[1], kVoteJ);
+  V.tiles[2] = (uint32_t)cdiv(g.n[2], kVoteK);
   V.min_rays = min_rays;
   V.max_rays = max_rays;
   V.conf_thresh = conf_thresh;
@@ -833,8 +982,10 @@ int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int 
   V.und_par = und_par;
   V.wind_list = wind;
   V.counters = ctx->d_counters;
-  k_vote<<<grid_for(g.ngp, 256, 148 * 16), 256, 0, st>>>(V);
+  const int64_t vote_warps = (int64_t)V.tiles[0] * V.tiles[1] * V.tiles[2];
+  k_vote<<<(unsigned)cdiv(vote_warps, 8), 256, 0, st>>>(V);
   SDF_KERNEL(ctx);
+  SDF_MARK_ON(ctx, T_PARITY, st);
   SDF_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + S_UNDECIDED, ctx->d_counters + C_LIST_UNDECIDED, sizeof(int64_t),
                                 cudaMemcpyDeviceToHost, st));
   SDF_CUDA(ctx, cudaStreamSynchronize(st));
@@ -866,7 +1017,6 @@ int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int 
     R.rec = rec;
     R.pad = (float)(2e-6 * g.E);
     R.max_visits = 2 * nel + 64;
-    R.par[0] = px; R.par[1] = py; R.par[2] = pz;
     R.list = und;
     R.min_rays = min_rays;
     R.max_rays = max_rays;
@@ -895,7 +1045,7 @@ int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int 
         SDF_TRY(scratch_t(ctx, "ray_hit_t", (size_t)nund * 36 * kRayCap, &hit_t));
         SDF_CUDA(ctx, cudaMemsetAsync(hit_n, 0, sizeof(int32_t) * nund * 36, st));
         const float reach = (float)(M.rho_max * (1.0 + 1e-5) + 4e-6 * g.E);
-        k_rays_all<<<grid_for(nel, 128, 148 * 64), 128, 0, st>>>(R, buf<float4>(ctx, "c32"), nel, reach, hit_n, hit_t);
+        k_rays_all<<<grid_for(nel, 128, 148 * 16), 128, 0, st>>>(R, buf<float4>(ctx, "c32"), nel, reach, hit_n, hit_t);
         SDF_KERNEL(ctx);
         k_rays_parity<<<grid_for(nund * 36, 64), 64, 0, st>>>(R, hit_n, hit_t);
       } else {
