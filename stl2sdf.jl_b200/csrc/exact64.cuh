@@ -120,7 +120,10 @@ __device__ inline void factor_bary(TriRec64& r) {
     if (an[1] > an[imax]) imax = 1;
     if (an[2] > an[imax]) imax = 2;
   }
-  A[imax][0] = A[imax][1] = A[imax][2] = 1.0;
+  // fixed indices throughout (row selects and swaps by compare), so that the matrix stays in registers
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    if (i == imax) A[i][0] = A[i][1] = A[i][2] = 1.0;
   r.imax = imax;
   const bool tril = A[0][1] == 0.0 && A[0][2] == 0.0 && A[1][2] == 0.0;
   const bool triu = A[1][0] == 0.0 && A[2][0] == 0.0 && A[2][1] == 0.0;
@@ -133,21 +136,29 @@ __device__ inline void factor_bary(TriRec64& r) {
     r.kind = 2;
   } else {
     r.kind = 0;
+#pragma unroll
     for (int j = 0; j < 3; ++j) {
       int p = j;
       double pm = fabs(A[j][j]);
+#pragma unroll
       for (int i = j + 1; i < 3; ++i) {
         const double v = fabs(A[i][j]);
         if (v > pm) { pm = v; p = i; }
       }
       piv[j] = p;
-      if (p != j)
-        for (int k = 0; k < 3; ++k) { const double t = A[j][k]; A[j][k] = A[p][k]; A[p][k] = t; }
+#pragma unroll
+      for (int i = j + 1; i < 3; ++i)
+        if (p == i)
+#pragma unroll
+          for (int k = 0; k < 3; ++k) { const double t = A[j][k]; A[j][k] = A[i][k]; A[i][k] = t; }
       if (A[j][j] != 0.0) {
         const double rcp = dd(1.0, A[j][j]);
+#pragma unroll
         for (int i = j + 1; i < 3; ++i) A[i][j] = dm(A[i][j], rcp);
       }
+#pragma unroll
       for (int i = j + 1; i < 3; ++i)
+#pragma unroll
         for (int k = j + 1; k < 3; ++k) A[i][k] = ds(A[i][k], dm(A[i][j], A[j][k]));
     }
   }

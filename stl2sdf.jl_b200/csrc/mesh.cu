@@ -11,6 +11,8 @@
 // trees"): 30-bit Morton codes of the triangle centroids with the triangle index in the low 32
 // bits (unique 64-bit keys), a CUB radix sort, one thread per internal node to find its range
 // and split, then a bottom-up refit with one atomic counter per internal node.
+#include <cstddef>
+
 #include <cub/cub.cuh>
 
 #include "common.cuh"
@@ -19,7 +21,12 @@ namespace sdfgpu {
 
 namespace {
 
-__global__ void k_vertex_bbox(const double* __restrict__ X, int64_t nnp, unsigned long long* bb) {
+// One set of atomics per block: with one per warp they took 35 of 44 us (0.7M vertices).
+__global__ void __launch_bounds__(256) k_vertex_bbox(const double* __restrict__ X, int64_t nnp, unsigned long long* bb) {
+  __shared__ double s_lo[8][3], s_hi[8][3];
+  __shared__ int s_bad;
+  if (threadIdx.x == 0) s_bad = 0;
+  __syncthreads();
   double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
   bool nonfinite = false;
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < nnp; v += (int64_t)gridDim.x * blockDim.x) {
@@ -35,59 +42,30 @@ __global__ void k_vertex_bbox(const double* __restrict__ X, int64_t nnp, unsigne
       lo[a] = fmin(lo[a], __shfl_down_sync(0xffffffffu, lo[a], off));
       hi[a] = fmax(hi[a], __shfl_down_sync(0xffffffffu, hi[a], off));
     }
-  }
-  const unsigned nf = __ballot_sync(0xffffffffu, nonfinite);
-  if ((threadIdx.x & 31) == 0) {
-    for (int a = 0; a < 3; ++a) {
-      atomicMin(&bb[a], dbl_ord(lo[a]));
-      atomicMax(&bb[3 + a], dbl_ord(hi[a]));
+    if ((threadIdx.x & 31) == 0) {
+      s_lo[threadIdx.x >> 5][a] = lo[a];
+      s_hi[threadIdx.x >> 5][a] = hi[a];
     }
-    if (nf) atomicOr(&bb[6], 1ULL);
   }
+  if (nonfinite) s_bad = 1;
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    const int a = threadIdx.x;
+    double l = s_lo[0][a], h = s_hi[0][a];
+    for (int w = 1; w < 8; ++w) {
+      l = fmin(l, s_lo[w][a]);
+      h = fmax(h, s_hi[w][a]);
+    }
+    atomicMin(&bb[a], dbl_ord(l));
+    atomicMax(&bb[3 + a], dbl_ord(h));
+  }
+  if (threadIdx.x == 3 && s_bad) atomicOr(&bb[6], 1ULL);
 }
 
-// Per-triangle FP64 record (dfOnTriangularMesh.jl:329-368) and the barycentric factorization.
-__global__ void k_prep(const double* __restrict__ X, int64_t nnp, const int64_t* __restrict__ IEN, int64_t nel,
-                       TriRec64* __restrict__ rec, double4* __restrict__ cent, int64_t* counters) {
-  for (int64_t el = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; el < nel; el += (int64_t)gridDim.x * blockDim.x) {
-    TriRec64 r;
-    d3 v[3];
-    for (int k = 0; k < 3; ++k) {
-      int64_t vi = IEN[3 * el + k];
-      if (vi < 1 || vi > nnp) {
-        count_add(counters, C_ERR_INDEX, 1);
-        vi = 1;
-      }
-      vi -= 1;
-      v[k] = {X[3 * vi], X[3 * vi + 1], X[3 * vi + 2]};
-      r.v[3 * k] = v[k].x; r.v[3 * k + 1] = v[k].y; r.v[3 * k + 2] = v[k].z;
-    }
-    const d3 e[3] = {v_sub(v[1], v[0]), v_sub(v[2], v[1]), v_sub(v[0], v[2])};
-    for (int j = 0; j < 3; ++j) {
-      r.L[j] = v_norm(e[j]);
-      const d3 u = v_div(e[j], r.L[j]);
-      r.u[3 * j] = u.x; r.u[3 * j + 1] = u.y; r.u[3 * j + 2] = u.z;
-    }
-    const d3 nn = v_cross(e[0], v_neg(e[2]));
-    const d3 n = v_div(nn, v_norm(nn));
-    r.n[0] = n.x; r.n[1] = n.y; r.n[2] = n.z;
-    const d3 c = v_div(v_add(v_add(v[0], v[1]), v[2]), 3.0);
-    r.bmin[0] = fmin(v[0].x, fmin(v[1].x, v[2].x));
-    r.bmin[1] = fmin(v[0].y, fmin(v[1].y, v[2].y));
-    r.bmin[2] = fmin(v[0].z, fmin(v[1].z, v[2].z));
-    r.bmax[0] = fmax(v[0].x, fmax(v[1].x, v[2].x));
-    r.bmax[1] = fmax(v[0].y, fmax(v[1].y, v[2].y));
-    r.bmax[2] = fmax(v[0].z, fmax(v[1].z, v[2].z));
-    r.pad = 0;
-    factor_bary(r);
-    rec[el] = r;
-    cent[el] = make_double4(c.x, c.y, c.z, 0.0);
-  }
-}
-
-// The FP32 record of a triangle (LeafTri, geom32.cuh), computed in FP64 from its vertices v, mesh-local,
+// The FP32 record of a triangle (LeafTri, geom32.cuh), computed in FP64 from its FP64 record, mesh-local,
 // and rounded once; id: its index, with kWeakTri when it is not fit for FP32 decisions.
-__device__ __forceinline__ LeafTri leaf_record(const double* v, int id, double cx, double cy, double cz) {
+__device__ __forceinline__ LeafTri leaf_record(const TriRec64& r, int id, double cx, double cy, double cz) {
+  const double* v = r.v;
   const double e0[3] = {v[3] - v[0], v[4] - v[1], v[5] - v[2]};
   const double e1[3] = {v[6] - v[0], v[7] - v[1], v[8] - v[2]};
   const double e2[3] = {v[6] - v[3], v[7] - v[4], v[8] - v[5]};
@@ -99,38 +77,41 @@ __device__ __forceinline__ LeafTri leaf_record(const double* v, int id, double c
   LeafTri T;
   T.a = make_float4((float)(v[0] - cx), (float)(v[1] - cy), (float)(v[2] - cz), __int_as_float(id));
   if (nn > 1e-20 * l0 * l1) {
-    const double rn = 1.0 / sqrt(nn), un[3] = {nx * rn, ny * rn, nz * rn};
-    // inward in-plane edge normals: n x (edge direction), edges a->b, b->c, c->a
-    const double* ed[3] = {e0, e2, e1};
-    const double sg[3] = {1.0, 1.0, -1.0};
+    // inward in-plane edge normals: n x (unit edge), edges a->b, b->c, c->a; with the area above 1e-10 of the
+    // edges' product, n is normal to the edges within 1e-5 and these are unit vectors within 1e-10
     double m[3][3];
+#pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const double* d = ed[k];
-      const double mx = sg[k] * (un[1] * d[2] - un[2] * d[1]), my = sg[k] * (un[2] * d[0] - un[0] * d[2]),
-                   mz = sg[k] * (un[0] * d[1] - un[1] * d[0]);
-      const double r = 1.0 / sqrt(mx * mx + my * my + mz * mz);
-      m[k][0] = mx * r; m[k][1] = my * r; m[k][2] = mz * r;
+      const double* u = r.u + 3 * k;
+      m[k][0] = r.n[1] * u[2] - r.n[2] * u[1];
+      m[k][1] = r.n[2] * u[0] - r.n[0] * u[2];
+      m[k][2] = r.n[0] * u[1] - r.n[1] * u[0];
     }
-    T.n = make_float4((float)un[0], (float)un[1], (float)un[2], (float)sqrt(l0));
-    T.m0 = make_float4((float)m[0][0], (float)m[0][1], (float)m[0][2], (float)sqrt(l2));
+    T.n = make_float4((float)r.n[0], (float)r.n[1], (float)r.n[2], (float)r.L[0]);
+    T.m0 = make_float4((float)m[0][0], (float)m[0][1], (float)m[0][2], (float)r.L[1]);
     T.m1 = make_float4((float)m[1][0], (float)m[1][1], (float)m[1][2],
                        (float)(e0[0] * m[1][0] + e0[1] * m[1][1] + e0[2] * m[1][2]));
-    T.m2 = make_float4((float)m[2][0], (float)m[2][1], (float)m[2][2], (float)sqrt(l1));
+    T.m2 = make_float4((float)m[2][0], (float)m[2][1], (float)m[2][2], (float)r.L[2]);
   } else {  // no area: the longest edge (see LeafTri)
     const int k = l0 >= l1 && l0 >= l2 ? 0 : (l1 >= l2 ? 2 : 1);  // edge a->b, c->a or b->c
-    const double* d = k == 0 ? e0 : (k == 1 ? e2 : e1);
     const double len = sqrt(k == 0 ? l0 : (k == 1 ? l2 : l1));
-    double u[3] = {1.0, 0.0, 0.0};
-    if (len > 0.0)
-      for (int q = 0; q < 3; ++q) u[q] = d[q] / len;
-    const int s = k == 1 ? 3 : 0;  // from b along b->c, else from a
+    double u[3], o[3];  // the edge's direction, and its origin: b along b->c, else a
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const double d = k == 0 ? e0[q] : (k == 1 ? e2[q] : e1[q]);
+      u[q] = len > 0.0 ? d / len : (q == 0 ? 1.0 : 0.0);
+      o[q] = k == 1 ? v[3 + q] : v[q];
+    }
     // n: the coordinate axis least along u, made normal to it
     const int j = fabs(u[0]) <= fabs(u[1]) && fabs(u[0]) <= fabs(u[2]) ? 0 : (fabs(u[1]) <= fabs(u[2]) ? 1 : 2);
+    const double uj = j == 0 ? u[0] : (j == 1 ? u[1] : u[2]);
     double un[3];
-    for (int q = 0; q < 3; ++q) un[q] = (q == j ? 1.0 : 0.0) - u[j] * u[q];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) un[q] = (q == j ? 1.0 : 0.0) - uj * u[q];
     const double rn = 1.0 / sqrt(un[0] * un[0] + un[1] * un[1] + un[2] * un[2]);
+#pragma unroll
     for (int q = 0; q < 3; ++q) un[q] *= rn;
-    T.a = make_float4((float)(v[s] - cx), (float)(v[s + 1] - cy), (float)(v[s + 2] - cz), __int_as_float(id));
+    T.a = make_float4((float)(o[0] - cx), (float)(o[1] - cy), (float)(o[2] - cz), __int_as_float(id));
     T.n = make_float4((float)un[0], (float)un[1], (float)un[2], (float)len);
     T.m0 = make_float4((float)(un[1] * u[2] - un[2] * u[1]), (float)(un[2] * u[0] - un[0] * u[2]),
                        (float)(un[0] * u[1] - un[1] * u[0]), k == 1 ? 1.f : 0.f);
@@ -140,66 +121,159 @@ __device__ __forceinline__ LeafTri leaf_record(const double* v, int id, double c
   return T;
 }
 
-// Mesh-local FP32 copies: vertices, centroid, outward-rounded box; and rho = max vertex
-// distance from the centroid (decides whether the centroid rule can miss a triangle within h).
+// The per-triangle data of a mesh, one thread per triangle: the FP64 record (dfOnTriangularMesh.jl:329-368)
+// with the barycentric factorization, the centroid, and mesh-local FP32 copies: vertices, centroid,
+// outward-rounded box and the FP32 record.
 // v32[3*el+k].w carries the global (0-based) index of vertex k; c32[el].w is 1 when the triangle
 // is well conditioned for FP32 decisions (no edge shorter than 1e-5 E, sine of the smallest
 // angle above ~1e-3, distinct vertices) and 0 when every decision on it must be made in FP64; rho_ord
-// receives rho, the same over such unfit triangles only, and their number.  tri32: the triangles' FP32
-// records (LeafTris by triangle index).
-__global__ void k_local32(const TriRec64* __restrict__ rec, const double4* __restrict__ cent,
-                          const int64_t* __restrict__ IEN, int64_t nel, double cx, double cy, double cz, double E,
-                          float4* __restrict__ v32, float4* __restrict__ c32, float4* __restrict__ box32,
-                          float4* __restrict__ tri32, unsigned long long* rho_ord) {
-  double rho = 0.0, rho_weak = 0.0;
-  unsigned weak = 0u;
-  for (int64_t el = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; el < nel; el += (int64_t)gridDim.x * blockDim.x) {
-    const TriRec64& r = rec[el];
-    const double4 c = cent[el];
-    int32_t gid[3];
-    double rt = 0.0;
-    for (int k = 0; k < 3; ++k) {
-      gid[k] = (int32_t)(IEN[3 * el + k] - 1);
-      const double x = r.v[3 * k], y = r.v[3 * k + 1], z = r.v[3 * k + 2];
-      v32[3 * el + k] = make_float4((float)(x - cx), (float)(y - cy), (float)(z - cz), __int_as_float(gid[k]));
-      const double dx = x - c.x, dy = y - c.y, dz = z - c.z;
-      rt = fmax(rt, sqrt(dx * dx + dy * dy + dz * dz));
-    }
-    rho = fmax(rho, rt);
-    double L[3], lmin = 1e300, lmax = 0.0;
-    for (int j = 0; j < 3; ++j) {
-      const int a = j, b = (j + 1) % 3;
-      const double ex = r.v[3 * b] - r.v[3 * a], ey = r.v[3 * b + 1] - r.v[3 * a + 1], ez = r.v[3 * b + 2] - r.v[3 * a + 2];
-      L[j] = sqrt(ex * ex + ey * ey + ez * ez);
-      lmin = fmin(lmin, L[j]);
-      lmax = fmax(lmax, L[j]);
-    }
-    const double ax = r.v[3] - r.v[0], ay = r.v[4] - r.v[1], az = r.v[5] - r.v[2];
-    const double bx = r.v[6] - r.v[0], by = r.v[7] - r.v[1], bz = r.v[8] - r.v[2];
-    const double nx = ay * bz - az * by, ny = az * bx - ax * bz, nz = ax * by - ay * bx;
-    const double nn = sqrt(nx * nx + ny * ny + nz * nz);
-    const bool ok = lmin > 1e-5 * E && nn > 1e-3 * lmax * lmax && gid[0] != gid[1] && gid[1] != gid[2] &&
-                    gid[0] != gid[2];
-    c32[el] = make_float4((float)(c.x - cx), (float)(c.y - cy), (float)(c.z - cz), ok ? 1.f : 0.f);
-    box32[2 * el] = make_float4(__double2float_rd(r.bmin[0] - cx), __double2float_rd(r.bmin[1] - cy),
-                                __double2float_rd(r.bmin[2] - cz), 0.f);
-    box32[2 * el + 1] = make_float4(__double2float_ru(r.bmax[0] - cx), __double2float_ru(r.bmax[1] - cy),
-                                    __double2float_ru(r.bmax[2] - cz), 0.f);
-    if (!ok) {
-      ++weak;
-      rho_weak = fmax(rho_weak, rt);
-    }
-    const LeafTri T = leaf_record(r.v, ok ? (int)el : (int)el | kWeakTri, cx, cy, cz);
-    const float4 f[5] = {T.a, T.n, T.m0, T.m1, T.m2};
+// receives rho = max vertex distance from the centroid (decides whether the centroid rule can miss a
+// triangle within h), the same over such unfit triangles only, and their number.  tri32: the triangles'
+// FP32 records (LeafTris by triangle index).  bb: k_vertex_bbox's result, from which every thread forms the
+// centre and E as the host does.
+//
+// Bound: the 544 bytes a triangle it writes.  The records go through shared memory, a warp's at a time, so
+// that each store instruction fills whole lines: written by their own threads, 16 bytes at a stride of 336, they
+// and the pass that read them back for the FP32 copies took 0.51 ms on 1.43M triangles and 2.04 ms on 5.8M
+// (B200), against 0.20 and 0.70 ms.  An odd stride in doubles keeps both sides free of bank conflicts.
+constexpr int kPrepThreads = 128;
+constexpr int kRecDoubles = sizeof(TriRec64) / 8, kRecStride = kRecDoubles + 1;
+static_assert(sizeof(TriRec64) % 16 == 0 && kRecStride % 2 == 1, "records are copied 16 bytes at a time");
+__global__ void __launch_bounds__(kPrepThreads) k_prep(const double* __restrict__ X, int64_t nnp,
+                                                       const int64_t* __restrict__ IEN, int64_t nel,
+                                                       const unsigned long long* __restrict__ bb,
+                                                       TriRec64* __restrict__ rec, double4* __restrict__ cent,
+                                                       float4* __restrict__ v32, float4* __restrict__ c32,
+                                                       float4* __restrict__ box32, float4* __restrict__ tri32,
+                                                       unsigned long long* rho_ord, int64_t* counters) {
+  __shared__ double s_rec[kPrepThreads / 32][32 * kRecStride];
+  const int lane = threadIdx.x & 31;
+  double* stage = s_rec[threadIdx.x >> 5];
+  double ctr[3], E = 0.0;
 #pragma unroll
-    for (int k = 0; k < 5; ++k) tri32[(int64_t)k * nel + el] = f[k];
+  for (int a = 0; a < 3; ++a) {
+    const double lo = ord_dbl(bb[a]), hi = ord_dbl(bb[3 + a]);
+    ctr[a] = dm(0.5, da(lo, hi));
+    E = fmax(E, fmax(ds(hi, ctr[a]), ds(ctr[a], lo)));
   }
+  double rho2 = 0.0, rho2_weak = 0.0;
+  unsigned weak = 0u;
+  for (int64_t base = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) - lane; base < nel;
+       base += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t el = base + lane;
+    const int count = (int)min((int64_t)32, nel - base);
+    TriRec64 r;
+    if (lane < count) {
+      d3 v[3];
+      int32_t gid[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        int64_t vi = IEN[3 * el + k];
+        if (vi < 1 || vi > nnp) {
+          count_add(counters, C_ERR_INDEX, 1);
+          vi = 1;
+        }
+        vi -= 1;
+        gid[k] = (int32_t)vi;
+        v[k] = {X[3 * vi], X[3 * vi + 1], X[3 * vi + 2]};
+        r.v[3 * k] = v[k].x; r.v[3 * k + 1] = v[k].y; r.v[3 * k + 2] = v[k].z;
+      }
+      const d3 e[3] = {v_sub(v[1], v[0]), v_sub(v[2], v[1]), v_sub(v[0], v[2])};
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        r.L[j] = v_norm(e[j]);
+        const d3 u = v_div(e[j], r.L[j]);
+        r.u[3 * j] = u.x; r.u[3 * j + 1] = u.y; r.u[3 * j + 2] = u.z;
+      }
+      const d3 nn = v_cross(e[0], v_neg(e[2]));
+      const double area2 = v_norm(nn);
+      const d3 n = v_div(nn, area2);
+      r.n[0] = n.x; r.n[1] = n.y; r.n[2] = n.z;
+      const d3 c = v_div(v_add(v_add(v[0], v[1]), v[2]), 3.0);
+      r.bmin[0] = fmin(v[0].x, fmin(v[1].x, v[2].x));
+      r.bmin[1] = fmin(v[0].y, fmin(v[1].y, v[2].y));
+      r.bmin[2] = fmin(v[0].z, fmin(v[1].z, v[2].z));
+      r.bmax[0] = fmax(v[0].x, fmax(v[1].x, v[2].x));
+      r.bmax[1] = fmax(v[0].y, fmax(v[1].y, v[2].y));
+      r.bmax[2] = fmax(v[0].z, fmax(v[1].z, v[2].z));
+      r.pad = 0;
+      cent[el] = make_double4(c.x, c.y, c.z, 0.0);
+      double rt2 = 0.0;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const double dx = v[k].x - c.x, dy = v[k].y - c.y, dz = v[k].z - c.z;
+        rt2 = fmax(rt2, dx * dx + dy * dy + dz * dz);
+      }
+      rho2 = fmax(rho2, rt2);
+      const double lmin = fmin(r.L[0], fmin(r.L[1], r.L[2])), lmax = fmax(r.L[0], fmax(r.L[1], r.L[2]));
+      const bool ok = lmin > 1e-5 * E && area2 > 1e-3 * lmax * lmax && gid[0] != gid[1] && gid[1] != gid[2] &&
+                      gid[0] != gid[2];
+      if (!ok) {
+        ++weak;
+        rho2_weak = fmax(rho2_weak, rt2);
+      }
+      c32[el] = make_float4((float)(c.x - ctr[0]), (float)(c.y - ctr[1]), (float)(c.z - ctr[2]), ok ? 1.f : 0.f);
+      const LeafTri T = leaf_record(r, ok ? (int)el : (int)el | kWeakTri, ctr[0], ctr[1], ctr[2]);
+      const float4 f[5] = {T.a, T.n, T.m0, T.m1, T.m2};
+#pragma unroll
+      for (int k = 0; k < 5; ++k) tri32[(int64_t)k * nel + el] = f[k];
+      // vertices and box, staged: 3 and 2 float4 a triangle
+      float4* f4 = reinterpret_cast<float4*>(stage);
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        f4[3 * lane + k] = make_float4((float)(v[k].x - ctr[0]), (float)(v[k].y - ctr[1]), (float)(v[k].z - ctr[2]),
+                                       __int_as_float(gid[k]));
+      f4[96 + 2 * lane] = make_float4(__double2float_rd(r.bmin[0] - ctr[0]), __double2float_rd(r.bmin[1] - ctr[1]),
+                                      __double2float_rd(r.bmin[2] - ctr[2]), 0.f);
+      f4[96 + 2 * lane + 1] = make_float4(__double2float_ru(r.bmax[0] - ctr[0]), __double2float_ru(r.bmax[1] - ctr[1]),
+                                          __double2float_ru(r.bmax[2] - ctr[2]), 0.f);
+      factor_bary(r);
+    }
+    __syncwarp();
+    {
+      const float4* f4 = reinterpret_cast<const float4*>(stage);
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        if (32 * k + lane < 3 * count) v32[3 * base + 32 * k + lane] = f4[32 * k + lane];
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        if (32 * k + lane < 2 * count) box32[2 * base + 32 * k + lane] = f4[96 + 32 * k + lane];
+    }
+    __syncwarp();
+    if (lane < count) {
+      double* o = stage + kRecStride * lane;
+#pragma unroll
+      for (int q = 0; q < 9; ++q) {
+        o[q] = r.v[q];
+        o[9 + q] = r.u[q];
+        o[30 + q] = r.A[q];
+      }
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        o[18 + q] = r.L[q];
+        o[21 + q] = r.n[q];
+        o[24 + q] = r.bmin[q];
+        o[27 + q] = r.bmax[q];
+      }
+      o[39] = __hiloint2double(r.imax, r.kind);
+      o[40] = __hiloint2double(r.pad, r.piv);
+      o[41] = 0.0;
+    }
+    __syncwarp();
+    double2* out = reinterpret_cast<double2*>(rec + base);
+    for (int q = lane; q < count * (kRecDoubles / 2); q += 32) {
+      const int s = 2 * q + q / (kRecDoubles / 2);
+      out[q] = make_double2(stage[s], stage[s + 1]);
+    }
+    __syncwarp();
+  }
+  double rho = sqrt(rho2), rho_weak = sqrt(rho2_weak);
   for (int off = 16; off > 0; off >>= 1) {
     rho = fmax(rho, __shfl_down_sync(0xffffffffu, rho, off));
     rho_weak = fmax(rho_weak, __shfl_down_sync(0xffffffffu, rho_weak, off));
     weak += __shfl_down_sync(0xffffffffu, weak, off);
   }
-  if ((threadIdx.x & 31) == 0) {
+  if (lane == 0) {
     atomicMax(rho_ord, dbl_ord(rho * (1.0 + 1e-12)));
     if (weak) {
       atomicMax(rho_ord + 1, dbl_ord(rho_weak * (1.0 + 1e-12)));
@@ -207,6 +281,11 @@ __global__ void k_local32(const TriRec64* __restrict__ rec, const double4* __res
     }
   }
 }
+static_assert(offsetof(TriRec64, u) == 9 * 8 && offsetof(TriRec64, L) == 18 * 8 && offsetof(TriRec64, n) == 21 * 8 &&
+                  offsetof(TriRec64, bmin) == 24 * 8 && offsetof(TriRec64, bmax) == 27 * 8 && offsetof(TriRec64, A) == 30 * 8 &&
+                  offsetof(TriRec64, kind) == 39 * 8 && offsetof(TriRec64, imax) == 39 * 8 + 4 &&
+                  offsetof(TriRec64, piv) == 40 * 8 && offsetof(TriRec64, pad) == 40 * 8 + 4 && kRecDoubles == 42,
+              "k_prep stages the record by double");
 
 __device__ __forceinline__ unsigned expand_bits10(unsigned v) {
   v = (v * 0x00010001u) & 0xFF0000FFu;
@@ -643,20 +722,25 @@ int mesh_upload_and_build(sdfgpu_ctx* ctx, const double* X, int64_t nnp, const i
   SDF_TRY(scratch_t(ctx, "box32", (size_t)nel * 2, &box32));
   SDF_TRY(scratch_t(ctx, "bbox", 10, &bb));
 
-  unsigned long long init[8];
-  for (int a = 0; a < 3; ++a) { init[a] = ~0ULL; init[3 + a] = 0ULL; }
-  init[6] = 0ULL;
-  init[7] = 0ULL;  // rho (ordered encoding of 0.0 is > 0; reset below)
+  float4* tri32;
+  SDF_TRY(scratch_t(ctx, "tri32", (size_t)nel * 5, &tri32));
+
+  // box, non-finite flag; rho, rho of the unfit triangles, their number (0 is below the encoding of every
+  // non-negative double)
+  unsigned long long init[10] = {~0ULL, ~0ULL, ~0ULL};
   SDF_CUDA(ctx, cudaMemsetAsync(ctx->d_counters, 0, sizeof(int64_t) * C_NUM, st));
   SDF_CUDA(ctx, cudaMemcpyAsync(bb, init, sizeof(init), cudaMemcpyHostToDevice, st));
-  k_vertex_bbox<<<grid_for(nnp, 256, 148 * 8), 256, 0, st>>>(dX, nnp, bb);
+  k_vertex_bbox<<<grid_for(nnp, 256, 148 * 4), 256, 0, st>>>(dX, nnp, bb);
   SDF_KERNEL(ctx);
-  k_prep<<<grid_for(nel, 128), 128, 0, st>>>(dX, nnp, dIEN, nel, rec, cent, ctx->d_counters);
+  k_prep<<<grid_for(nel, kPrepThreads), kPrepThreads, 0, st>>>(dX, nnp, dIEN, nel, bb, rec, cent, v32, c32, box32, tri32,
+                                                              bb + 7, ctx->d_counters);
   SDF_KERNEL(ctx);
-  unsigned long long hbb[8];
+  SDF_CUDA(ctx, cudaEventRecord(ctx->ev_mesh, st));
+  unsigned long long hbb[10];
   int64_t hcnt[C_NUM];
   SDF_CUDA(ctx, cudaMemcpyAsync(hbb, bb, sizeof(hbb), cudaMemcpyDeviceToHost, st));
   SDF_CUDA(ctx, cudaMemcpyAsync(hcnt, ctx->d_counters, sizeof(hcnt), cudaMemcpyDeviceToHost, st));
+  SDF_CUDA(ctx, cudaEventRecord(ctx->ev[5], st));
   SDF_CUDA(ctx, cudaStreamSynchronize(st));
   if (hbb[6]) return fail(ctx, SDFGPU_ERR_INVALID_ARGUMENT, "mesh vertices must be finite");
   if (hcnt[C_ERR_INDEX]) return fail(ctx, SDFGPU_ERR_INVALID_ARGUMENT, "IEN holds an index outside 1..nnp");
@@ -672,25 +756,11 @@ int mesh_upload_and_build(sdfgpu_ctx* ctx, const double* X, int64_t nnp, const i
     E = std::max(E, std::max(M.bmax[a] - M.center[a], M.center[a] - M.bmin[a]));
   }
   M.E = E;
-
-  // rho, rho of the unfit triangles, their number: 0 is below the encoding of every non-negative double
-  SDF_CUDA(ctx, cudaMemsetAsync(bb + 7, 0, 3 * sizeof(unsigned long long), st));
-  float4* tri32;
-  SDF_TRY(scratch_t(ctx, "tri32", (size_t)nel * 5, &tri32));
-  k_local32<<<grid_for(nel, 128), 128, 0, st>>>(rec, cent, dIEN, nel, M.center[0], M.center[1], M.center[2], M.E, v32,
-                                                 c32, box32, tri32, bb + 7);
-  SDF_KERNEL(ctx);
-
-  SDF_CUDA(ctx, cudaEventRecord(ctx->ev_mesh, st));
+  M.rho_max = ord_dbl(hbb[7]);
+  M.n_weak = (int64_t)hbb[9];
+  M.rho_weak = M.n_weak ? ord_dbl(hbb[8]) : 0.0;
   if (eager) SDF_TRY(ensure_tree(ctx, eager > 1));
   ctx->tree_used = 0;
-  unsigned long long hrho[3];
-  SDF_CUDA(ctx, cudaMemcpyAsync(hrho, bb + 7, sizeof(hrho), cudaMemcpyDeviceToHost, st));
-  SDF_CUDA(ctx, cudaEventRecord(ctx->ev[5], st));
-  SDF_CUDA(ctx, cudaStreamSynchronize(st));
-  M.rho_max = ord_dbl(hrho[0]);
-  M.n_weak = (int64_t)hrho[2];
-  M.rho_weak = M.n_weak ? ord_dbl(hrho[1]) : 0.0;
   float ms = 0.f;
   SDF_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev[4], ctx->ev[5]));
   ctx->stats.ms_mesh = ms;
