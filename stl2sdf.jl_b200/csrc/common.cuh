@@ -259,7 +259,7 @@ int run_nearest_points(sdfgpu_ctx* ctx, const GridP& g, double* d_dist);
 // dist_fold runs one mesh's fold, dist_knn its 3-nearest-vertex fallback, dist_fold_multi the
 // folds of many prepared meshes together.
 struct DistPlan {
-  alignas(16) unsigned char fold[512];      // the fold kernel's arguments (near.cu: those of its stage)
+  alignas(16) unsigned char fold[768];      // the fold kernel's arguments (near.cu: those of its stage)
   alignas(16) unsigned char knn_args[640];  // the fallback kernel's arguments (when knn)
   alignas(16) unsigned char unb[512];       // unbounded / learned: the search's arguments (UnbArgs)
   bool unbounded = false;                   // the plan is an unbounded search (unb), not a fold

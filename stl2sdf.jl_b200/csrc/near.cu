@@ -44,10 +44,17 @@ struct NearArgs {
   LeafTris tri;         // FP32 records by triangle index
   const TriRec64* rec;
   const double4* cent;
+  const float4* box32;  // mesh-local outward-rounded boxes
+  const float4* c32;    // and centroids
   int64_t nel;
   bool ref;             // the reference rule, else the true minimum
   double reach;         // box growth: h plus the margin
   double ih;            // 1 / h
+  // the grid in FP32: node = ihf * (mesh-local coordinate) + bo, within rm cells; mesh-local node
+  // coordinates o32 + hf * node; the near nodes' distance, with the FP32 error of a box and a node in it
+  float ihf, hf, bo[3], rm, o32[3], limb;
+  float mk;             // see k_near_scatter
+  uint64_t* mask;       // per triangle: the nodes of its box that its second scatter looks at
   float lim2, eD;       // squared FP32 distance of a near node; error of the FP32 distances
   float E;
   double rho;           // the mesh's largest vertex-to-centroid distance (edges are at most 2 rho)
@@ -61,10 +68,12 @@ struct NearArgs {
   int32_t* hidx;        // per near node: its hard index, or -1
   int32_t* hard_n;
   int32_t* hard;        // near indices of hard nodes
+  int32_t* unbounded_n; // hard nodes whose hbound is not known from their slots
   uint8_t* tflag;       // tiles with hard nodes
+  uint8_t* tcand;       // tiles in which a candidate of a hard node can have its centroid
   int64_t tn[3];
   float* hbound;        // per hard node: bound on the distances that matter to its fold
-  int32_t* hcnt;        // its candidates within it
+  int32_t* hcnt;        // its candidates within it (listed if they fit)
   int64_t* hoff;        // their place in the pool, -1: none
   int32_t* pool;
   unsigned long long* pool_n;
@@ -84,45 +93,92 @@ __device__ __forceinline__ bool near_range(const NearArgs& A, int a, double x0, 
   return lo <= hi;
 }
 
+// Node of axis a at a mesh-local coordinate, in FP32 (within A.rm), moved by `off`, clamped to one node beyond
+// the grid.
+__device__ __forceinline__ float node32(const NearArgs& A, int a, float x, float off) {
+  return fminf(fmaxf(fmaf(x, A.ihf, A.bo[a]) + off, -1.f), (float)A.g.N[a] + 1.f);
+}
+
 // kFill false: every node's smallest squared distance, over the nodes near each triangle.  kFill true:
 // each near node's triangles within the band of its minimum.  A thread per triangle: the boxes of one
-// mesh differ little in size, and the triangle's frame stays in registers.  Bound: instruction issue
-// (about 60 per pair), half of the pairs beyond h.
+// mesh differ little in size, and the triangle's frame stays in registers.  The nodes within h of the
+// triangle's box (a chord per grid row) are the bits of a 64-bit mask, so a warp takes as many steps as its
+// largest count, about half of the box's nodes.  The first scatter keeps the bits of the pairs that were
+// within the band of the node's minimum at that time; it only falls, so the second needs no others: about
+// two pairs a triangle instead of thirty.  Triangles of more than 64 nodes go through 64 at a time, both
+// times.  Bound: instruction issue, about 70 a pair.  Both scatters, 1.4M triangles of which a third of a
+// node is near, and 5.8M: 0.43 -> 0.30 and 1.9 -> 1.22 ms (B200) against all
+// nodes of the box in both.
 template <bool kFill>
 __global__ void __launch_bounds__(128) k_near_scatter(const __grid_constant__ NearArgs A) {
   const GridP& g = A.g;
-  const float hf = (float)g.h;
   for (int64_t el = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; el < A.nel; el += (int64_t)gridDim.x * blockDim.x) {
-    const TriRec64& r = A.rec[el];
-    int lo[3], hi[3];
+    uint64_t kept = 0;
+    if (kFill) {
+      kept = A.mask[el];
+      if (!kept) continue;
+    }
+    const float4 b0 = A.box32[2 * el], b1 = A.box32[2 * el + 1];
+    const float blo[3] = {b0.x, b0.y, b0.z}, bhi[3] = {b1.x, b1.y, b1.z};
+    const float grow = fmaf(A.limb, A.ihf, A.rm);
+    int lo[3], n[3];
     bool any = true;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const double v0 = r.v[a], v1 = r.v[3 + a], v2 = r.v[6 + a];
-      any = any && near_range(A, a, fmin(v0, fmin(v1, v2)) - A.reach, fmax(v0, fmax(v1, v2)) + A.reach, lo[a], hi[a]);
+      lo[a] = max((int)ceilf(node32(A, a, blo[a], -grow)), 0);
+      n[a] = min((int)floorf(node32(A, a, bhi[a], grow)), (int)g.N[a]) - lo[a] + 1;
+      any = any && n[a] > 0;
     }
-    if (!any) continue;
-    const LeafTri T = A.tri.load((int)el);
-    // the record's vertex a: v1, or the end of the longest edge of a triangle without area
-    const int s = T.m2.w < 0.f && T.m0.w != 0.f ? 3 : 0;
-    const LeafView V = leaf_view(T, f3(T.a));  // from points a + d
-    // nodes relative to a: FP64 differences rounded once, then FP32 steps along x
-    const float x0 = (float)(g.o[0] + g.h * (double)lo[0] - r.v[s]);
-    for (int k = lo[2]; k <= hi[2]; ++k) {
-      const float z = (float)(g.o[2] + g.h * (double)gidx(g, 2, k) - r.v[s + 2]);
-      for (int j = lo[1]; j <= hi[1]; ++j) {
-        const float y = (float)(g.o[1] + g.h * (double)j - r.v[s + 1]);
-        const int64_t row = g.n[0] * (j + g.n[1] * (int64_t)k);
-        for (int i = lo[0]; i <= hi[0]; ++i) {
-          const float d2 = view_d2(V, make_float3(fmaf(hf, (float)(i - lo[0]), x0), y, z));
+    uint64_t next = 0;
+    if (any) {
+      const LeafTri T = A.tri.load((int)el);
+      // the record's vertex a: v1, or the end of the longest edge of a triangle without area
+      const double* va = A.rec[el].v + (T.m2.w < 0.f && T.m0.w != 0.f ? 3 : 0);
+      const LeafView V = leaf_view(T, f3(T.a));  // from points a + d
+      // nodes relative to a: an FP64 difference rounded once, then FP32 steps
+      const float x0 = (float)(g.o[0] + g.h * (double)lo[0] - va[0]), y0 = (float)(g.o[1] + g.h * (double)lo[1] - va[1]),
+                  z0 = (float)(g.o[2] + g.h * (double)gidx(g, 2, lo[2]) - va[2]);
+      const int rows = n[1] * n[2], per = max(64 / n[0], 1);  // near_applies keeps n[0] below 16
+      const float inx = 1.f / (float)n[0], iny = 1.f / (float)n[1];
+      const float limb2 = A.limb * A.limb;
+#pragma unroll 1
+      for (int row0 = 0; row0 < rows; row0 += per) {
+        uint64_t bits = kept;
+        if (!kFill || rows > per) {
+          bits = 0;
+          int at = 0;
+          const int row1 = min(rows, row0 + per);
+          int k = (int)(((float)row0 + 0.5f) * iny), j = row0 - k * n[1];
+#pragma unroll 1
+          for (int r = row0; r < row1; ++r, at += n[0]) {
+            const float y = fmaf(A.hf, (float)(lo[1] + j), A.o32[1]), z = fmaf(A.hf, (float)(lo[2] + k), A.o32[2]);
+            const float dy = fmaxf(fmaxf(blo[1] - y, y - bhi[1]), 0.f), dz = fmaxf(fmaxf(blo[2] - z, z - bhi[2]), 0.f);
+            const float rem = limb2 - dy * dy - dz * dz;
+            if (rem >= 0.f) {
+              const float half = fmaf(sqrt_approx(rem) * (1.f + 1e-5f), A.ihf, A.rm);
+              const int i0 = max((int)ceilf(node32(A, 0, blo[0], -half)), lo[0]) - lo[0];
+              const int i1 = min((int)floorf(node32(A, 0, bhi[0], half)) - lo[0], n[0] - 1);
+              if (i1 >= i0) bits |= ((2ull << (i1 - i0)) - 1ull) << (at + i0);
+            }
+            if (++j == n[1]) { j = 0; ++k; }
+          }
+        }
+        while (bits) {
+          const int b = __ffsll((long long)bits) - 1;
+          bits &= bits - 1ull;
+          const int br = (int)(((float)b + 0.5f) * inx), i = b - br * n[0], r = row0 + br;
+          const int k = (int)(((float)r + 0.5f) * iny), j = r - k * n[1];
+          const float d2 = view_d2(V, make_float3(fmaf(A.hf, (float)i, x0), fmaf(A.hf, (float)j, y0), fmaf(A.hf, (float)k, z0)));
           if (!(d2 <= A.lim2)) continue;
-          const int64_t lin = row + i;
+          const int64_t lin = lo[0] + i + g.n[0] * (lo[1] + j + g.n[1] * (int64_t)(lo[2] + k));
           const uint32_t m = __ldcg(A.m2 + lin);
           if (!kFill) {
+            // (sqrt(m) + 2 eD)^2 with sqrt(m) at most the near nodes' distance
+            if (d2 <= fmaf(__uint_as_float(m), 1.f + 4e-6f, A.mk)) next |= 1ull << b;
             if (__float_as_uint(d2) < m) atomicMin(A.m2 + lin, __float_as_uint(d2));
           } else {
-            const float b = sqrt_approx(__uint_as_float(m)) * (1.f + 1e-6f) + 2.f * A.eD;
-            if (d2 > b * b) continue;
+            const float w = sqrt_approx(__uint_as_float(m)) * (1.f + 1e-6f) + 2.f * A.eD;
+            if (d2 > w * w) continue;
             const int32_t q = A.map[lin];
             const int c = atomicAdd(A.cnt + q, 1);
             if (c < kSlots) A.slot[(int64_t)q * kSlots + c] = __float_as_int(T.a.w);
@@ -130,28 +186,54 @@ __global__ void __launch_bounds__(128) k_near_scatter(const __grid_constant__ Ne
         }
       }
     }
+    if (!kFill) A.mask[el] = next;  // of several masks: whether any has a bit
   }
 }
 
-// Lists the near nodes; all others get h.
-__global__ void k_near_nodes(const __grid_constant__ NearArgs A) {
+// Lists the near nodes; all others get h.  A block takes kNodes nodes a thread and one place in the list for
+// them: an atomic per warp on the list's length took 0.31 ms for 33M nodes, this 0.11 (B200).  Bound: 12
+// bytes a node.
+constexpr int kNodes = 8, kNodesThreads = 256;
+__global__ void __launch_bounds__(kNodesThreads) k_near_nodes(const __grid_constant__ NearArgs A) {
+  __shared__ int s_n[kNodesThreads / 32], s_first;
   const GridP& g = A.g;
-  const int lane = threadIdx.x & 31;
-  for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < g.ngp; base += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t lin = base + threadIdx.x;
-    const bool in = lin < g.ngp;
-    const bool near = in && A.m2[lin] != 0x7f7f7f7fu;
-    if (in && !near) A.dist[lin] = g.h;
-    const unsigned mask = __ballot_sync(0xffffffffu, near);
-    if (!mask) continue;
-    int first = 0;
-    if (lane == 0) first = atomicAdd(A.near_n, __popc(mask));
-    first = __shfl_sync(0xffffffffu, first, 0);
-    if (near) {
-      const int q = first + __popc(mask & ((1u << lane) - 1u));
-      A.map[lin] = q;
-      A.node[q] = (int32_t)lin;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int64_t base = blockIdx.x * (int64_t)(kNodes * kNodesThreads); base < g.ngp;
+       base += (int64_t)gridDim.x * (kNodes * kNodesThreads)) {
+    unsigned near = 0u;
+    int before[kNodes], total = 0;  // near nodes of this warp before mine
+#pragma unroll
+    for (int q = 0; q < kNodes; ++q) {
+      const int64_t lin = base + q * kNodesThreads + threadIdx.x;
+      const bool in = lin < g.ngp, is = in && A.m2[lin] != 0x7f7f7f7fu;
+      if (in && !is) A.dist[lin] = g.h;
+      const unsigned mask = __ballot_sync(0xffffffffu, is);
+      before[q] = total + __popc(mask & ((1u << lane) - 1u));
+      total += __popc(mask);
+      near |= (unsigned)is << q;
     }
+    if (lane == 0) s_n[w] = total;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int sum = 0;
+#pragma unroll
+      for (int v = 0; v < kNodesThreads / 32; ++v) {
+        const int c = s_n[v];
+        s_n[v] = sum;
+        sum += c;
+      }
+      s_first = sum ? atomicAdd(A.near_n, sum) : 0;
+    }
+    __syncthreads();
+    const int first = s_first + s_n[w];
+#pragma unroll
+    for (int q = 0; q < kNodes; ++q)
+      if ((near >> q) & 1u) {
+        const int64_t lin = base + q * kNodesThreads + threadIdx.x;
+        A.map[lin] = first + before[q];
+        A.node[first + before[q]] = (int32_t)lin;
+      }
+    __syncthreads();
   }
 }
 
@@ -199,8 +281,13 @@ __global__ void __launch_bounds__(128) k_near_resolve(const __grid_constant__ Ne
     const int n = A.cnt[q];
     bool hard = n < 1 || n > kSlots;
     for (int s = 0; s < n && !hard; ++s) hard = (slot[s] & kWeakTri) != 0;
-    double m = INFINITY;
-    if (!hard) {
+    double m = INFINITY, nearest = INFINITY;  // nearest: a squared distance of a triangle fit for FP32 decisions
+    if (hard) {
+      for (int s = 0; s < min(n, kSlots); ++s) {
+        int feat;
+        if ((slot[s] & kWeakTri) == 0) nearest = fmin(nearest, near64(A.rec, slot[s], p, tol2, feat));
+      }
+    } else {
       // the ties, as in lane_filter (unbounded.cuh)
       double best = 1e300, lim = 1e300;
       int left = 0;
@@ -218,6 +305,7 @@ __global__ void __launch_bounds__(128) k_near_resolve(const __grid_constant__ Ne
         }
         slot[left++] = (int)((unsigned)t | (unsigned)(feat < 0 ? 7 : feat) << kFeatShift);
       }
+      nearest = best;
       // in ascending triangle index
       double Vc = INFINITY, Fprev = INFINITY;
       int dependent = 0, last = -1;
@@ -266,9 +354,20 @@ __global__ void __launch_bounds__(128) k_near_resolve(const __grid_constant__ Ne
       A.hard[hq] = q;
       A.hidx[q] = hq;
       A.hcnt[hq] = 0;
-      A.hbound[hq] = INFINITY;
-      const int64_t i = lin % g.n[0], j = (lin / g.n[0]) % g.n[1], k = lin / (g.n[0] * g.n[1]);
-      A.tflag[((k >> kTileShift) * A.tn[1] + (j >> kTileShift)) * A.tn[0] + (i >> kTileShift)] = 1;
+      A.hbound[hq] = __double2float_ru(sqrt(nearest) + 4.0 * A.rho + 4.0 * tol);
+      if (isinf(nearest)) atomicAdd(A.unbounded_n, 1);
+      const int64_t at[3] = {lin % g.n[0], (lin / g.n[0]) % g.n[1], lin / (g.n[0] * g.n[1])};
+      A.tflag[((at[2] >> kTileShift) * A.tn[1] + (at[1] >> kTileShift)) * A.tn[0] + (at[0] >> kTileShift)] = 1;
+      const double rc = (A.ref ? A.rball : A.reach + A.rho) * A.ih + (double)A.rm + 1.0;
+      int t0[3], t1[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        t0[a] = max((int)((double)at[a] - rc), 0) >> kTileShift;
+        t1[a] = (int)fmin((double)at[a] + rc, (double)g.N[a]) >> kTileShift;
+      }
+      for (int z = t0[2]; z <= t1[2]; ++z)
+        for (int y = t0[1]; y <= t1[1]; ++y)
+          for (int x = t0[0]; x <= t1[0]; ++x) A.tcand[((int64_t)z * A.tn[1] + y) * A.tn[0] + x] = 1;
       continue;
     }
     A.dist[lin] = m > g.h ? g.h : m;  // clamp (dfOnTriangularMesh.jl:202-206)
@@ -293,17 +392,33 @@ __device__ __forceinline__ bool hard_candidate(const NearArgs& A, int64_t t, con
          p.y <= r.bmax[1] + A.reach && p.z >= r.bmin[2] - A.reach && p.z <= r.bmax[2] + A.reach;
 }
 
-// The hard nodes' candidates that matter: every triangle visits the flagged tiles its candidate region
-// reaches.  A step assigns at most the distance to the farthest point of its triangle, so the fold ends
-// at or below U = min over the triangles fit for FP32 decisions of (their distance + 2 rho); a value that
-// can be the result comes from a triangle within U, and whether its feet improve the minimum depends on
-// values up to U + 2 rho.  kPhase 0: that bound per node; 1: the candidates within it counted; 2: listed.
+// The hard nodes' candidates that matter: the triangles with their centroid in a tile where a hard node can
+// have candidates visit the tiles with hard nodes that their candidate region reaches.  A step assigns at
+// most the distance to the farthest point of its triangle, so the fold ends at or below U = min over the
+// triangles fit for FP32 decisions of (their distance + 2 rho); a value that can be the result comes from
+// a triangle within U, and whether its feet improve the minimum depends on values up to U + 2 rho.
+// k_near_resolve has that bound from a node's slots, unless all of them are unfit.  kPhase 0: it is found
+// for those nodes (else returns at once); 1: the candidates within it counted (returns at once when every
+// node can have kHardCap places); 2: listed.  Bound: 16 bytes and one flag a triangle; three passes that each
+// formed the triangles' regions in FP64 took 0.81 ms on 5.8M triangles, this 0.09 (B200).
+__device__ __forceinline__ bool hard_uniform(int n_hard) { return (int64_t)n_hard * kHardCap <= kHardPool; }
+
 template <int kPhase>
 __global__ void __launch_bounds__(128) k_hard_collect(const __grid_constant__ NearArgs A) {
   if (*A.hard_n == 0) return;
+  if (kPhase == 0 && *A.unbounded_n == 0) return;
+  if (kPhase == 1 && hard_uniform(*A.hard_n)) return;
   const GridP& g = A.g;
   const double tol = 1e-9 * (double)A.E;
   for (int64_t el = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; el < A.nel; el += (int64_t)gridDim.x * blockDim.x) {
+    {
+      const float4 c = A.c32[el];
+      const float f[3] = {node32(A, 0, c.x, 0.f), node32(A, 1, c.y, 0.f), node32(A, 2, c.z, 0.f)};
+      int t[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) t[a] = min(max((int)f[a], 0), (int)g.N[a]) >> kTileShift;
+      if (!A.tcand[((int64_t)t[2] * A.tn[1] + t[1]) * A.tn[0] + t[0]]) continue;
+    }
     int lo[3], hi[3];
     bool any = true;
     if (A.ref) {
@@ -343,7 +458,8 @@ __global__ void __launch_bounds__(128) k_hard_collect(const __grid_constant__ Ne
                 if (kPhase == 1) {
                   atomicAdd(A.hcnt + hq, 1);
                 } else if (A.hoff[hq] >= 0) {
-                  A.pool[A.hoff[hq] + atomicAdd(A.hcnt + hq, 1)] = (int32_t)el;
+                  const int c = atomicAdd(A.hcnt + hq, 1);
+                  if (c < kHardCap) A.pool[A.hoff[hq] + c] = (int32_t)el;
                 }
               }
         }
@@ -356,7 +472,9 @@ __global__ void k_hard_place(const __grid_constant__ NearArgs A) {
   for (int hq = blockIdx.x * blockDim.x + threadIdx.x; hq < n_hard; hq += gridDim.x * blockDim.x) {
     const int c = A.hcnt[hq];
     int64_t off = -1;
-    if (c <= kHardCap) {
+    if (hard_uniform(n_hard)) {
+      off = (int64_t)hq * kHardCap;
+    } else if (c <= kHardCap) {
       off = (int64_t)atomicAdd(A.pool_n, (unsigned long long)c);
       if (off + c > kHardPool) off = -1;
     }
@@ -395,8 +513,8 @@ __global__ void __launch_bounds__(128) k_hard_replay(const __grid_constant__ Nea
         ++fp64;
       }
     };
-    if (A.hoff[hq] >= 0) {
-      const int n = A.hcnt[hq];
+    const int n = A.hcnt[hq];
+    if (A.hoff[hq] >= 0 && n <= kHardCap) {
       int *list = s_list[w], *sorted = A.pool + A.hoff[hq];
       for (int s = lane; s < n; s += 32) list[s] = sorted[s];
       __syncwarp();
@@ -424,14 +542,15 @@ __global__ void __launch_bounds__(128) k_hard_replay(const __grid_constant__ Nea
 }  // namespace
 
 // Whether near_distances takes this call: triangles of at most 1.5 (reference rule) or 4 cells from their
-// centroid, the mesh near the coordinate origin (see unb_mesh), and few and small triangles unfit for
-// FP32 decisions, each of which sends the nodes nearest to it to the replay.
+// centroid, the mesh near the coordinate origin (see unb_mesh), mesh and grid within 1e5 cells of the mesh's
+// centre (FP32 node indices within half a cell, and a box's rows within a mask), and few and small triangles
+// unfit for FP32 decisions, each of which sends the nodes nearest to it to the replay.
 bool near_applies(const sdfgpu_ctx* ctx, const GridP& g, int mode) {
   const MeshDev& M = ctx->mesh;
   double off = 0.0;
   for (int a = 0; a < 3; ++a) off = std::max(off, std::fabs(M.center[a]));
   const double rho = M.rho_max * (1.0 + 1e-9) + 1e-6 * g.E;
-  return off <= 64.0 * M.E && rho < (mode == SDFGPU_MODE_REF_RULE ? 1.5 : 4.0) * g.h && M.rho_weak <= 1.5 * g.h &&
+  return off <= 64.0 * M.E && g.E <= 1e5 * g.h && rho < (mode == SDFGPU_MODE_REF_RULE ? 1.5 : 4.0) * g.h && M.rho_weak <= 1.5 * g.h &&
          M.n_weak <= M.nel / 64;
 }
 
@@ -447,6 +566,8 @@ int near_prepare(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, Dist
   A.tri = LeafTris{buf<float4>(ctx, "tri32"), M.nel};
   A.rec = buf<TriRec64>(ctx, "rec");
   A.cent = buf<double4>(ctx, "cent64");
+  A.box32 = buf<float4>(ctx, "box32");
+  A.c32 = buf<float4>(ctx, "c32");
   A.nel = M.nel;
   A.ref = mode == SDFGPU_MODE_REF_RULE;
   // FP32 distances in the triangle's own frame: every rounding is relative to |p - a| + the edges, at most
@@ -457,6 +578,17 @@ int near_prepare(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, Dist
   A.reach = lim * (1.0 + 1e-9) + 1e-9 * g.E;
   A.ih = 1.0 / g.h;
   A.E = (float)g.E;
+  A.ihf = (float)A.ih;
+  A.hf = (float)g.h;
+  for (int a = 0; a < 3; ++a) {
+    const double o = g.o[a] + g.h * (double)gidx(g, a, 0) - M.center[a];  // mesh-local
+    A.o32[a] = (float)o;
+    A.bo[a] = (float)(-o * A.ih);
+  }
+  // FP32 coordinates of boxes and nodes are within 3 roundings of E each
+  A.limb = (float)(lim * (1.0 + 1e-6) + 1e-6 * g.E);
+  A.rm = (float)(2e-6 * g.E * A.ih + 1e-4);
+  A.mk = (float)(4.1 * A.eD * lim + 4.1 * A.eD * A.eD);
   A.rho = M.rho_max;
   const double sr = 2.5 * g.h;
   A.r2 = sr * sr;
@@ -468,21 +600,24 @@ int near_prepare(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, Dist
     A.tn[a] = (g.n[a] >> kTileShift) + 1;
     tiles *= A.tn[a];
   }
-  int32_t* counts;  // near nodes, hard nodes
+  int32_t* counts;  // near nodes, hard nodes, hard nodes without a bound
   SDF_TRY(scratch_t(ctx, "near_m2", (size_t)g.ngp, &A.m2));
   SDF_TRY(scratch_t(ctx, "near_map", (size_t)g.ngp, &A.map));
   SDF_TRY(scratch_t(ctx, "near_node", (size_t)g.ngp, &A.node));
-  SDF_TRY(scratch_t(ctx, "near_counts", 2, &counts));
-  SDF_TRY(scratch_t(ctx, "near_tflag", (size_t)tiles, &A.tflag));
+  SDF_TRY(scratch_t(ctx, "near_counts", 3, &counts));
+  SDF_TRY(scratch_t(ctx, "near_tflag", (size_t)tiles * 2, &A.tflag));
+  SDF_TRY(scratch_t(ctx, "near_mask", (size_t)M.nel, &A.mask));
+  A.tcand = A.tflag + tiles;
   A.near_n = counts;
   A.hard_n = counts + 1;
+  A.unbounded_n = counts + 2;
   SDF_CUDA(ctx, cudaMemsetAsync(A.m2, 0x7f, sizeof(uint32_t) * g.ngp, st));  // 3.39e38
-  SDF_CUDA(ctx, cudaMemsetAsync(counts, 0, 2 * sizeof(int32_t), st));
-  SDF_CUDA(ctx, cudaMemsetAsync(A.tflag, 0, (size_t)tiles, st));
+  SDF_CUDA(ctx, cudaMemsetAsync(counts, 0, 3 * sizeof(int32_t), st));
+  SDF_CUDA(ctx, cudaMemsetAsync(A.tflag, 0, (size_t)tiles * 2, st));
   const unsigned gt = grid_for(M.nel, 128, 148 * 64);
   k_near_scatter<false><<<gt, 128, 0, st>>>(A);
   SDF_KERNEL(ctx);
-  k_near_nodes<<<grid_for(g.ngp, 256, 148 * 16), 256, 0, st>>>(A);
+  k_near_nodes<<<grid_for(cdiv(g.ngp, kNodes), kNodesThreads, 148 * 16), kNodesThreads, 0, st>>>(A);
   SDF_KERNEL(ctx);
   int32_t n_near = 0;
   SDF_CUDA(ctx, cudaMemcpyAsync(&n_near, A.near_n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));

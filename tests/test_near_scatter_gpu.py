@@ -116,3 +116,18 @@ def test_adaptive_rays_of_few_and_many_nodes(gpu_ctx, n, drop):
     s, c = gpu_ctx.signs(o, h, N)
     ref = oracle.signs(V, F, o, h, N)
     assert np.array_equal(s, ref["sign"]) and np.array_equal(c, ref["conf"])
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("size", [0.1, 0.6, 1.4])
+@pytest.mark.parametrize("cones", [40, 4000])
+def test_separate_cones(gpu_ctx, cones, size, mode):
+    """Open cones whose apex is the nearest point of most nodes around them, the case that replays the
+    reference's fold: a few such nodes, and more than fit the fixed places of their candidate lists."""
+    rng = np.random.default_rng(cones)
+    a = rng.uniform(0, 1, (cones, 1, 3))
+    ring = a + size / 66.0 * rng.normal(0, 0.3, (cones, 3, 3)) + size / 66.0 * rng.normal(0, 0.5, (cones, 1, 3))
+    X = np.concatenate([a, ring], 1).reshape(-1, 3)
+    b = 4 * np.arange(cones)[:, None] + 1
+    F = np.concatenate([b + np.array([[0, 1, 2]]), b + np.array([[0, 2, 3]]), b + np.array([[0, 3, 1]])], 0)
+    check(gpu_ctx, X, F, 1.0 / 64.0, mode)
