@@ -306,6 +306,7 @@ int launch_combine(sdfgpu_ctx* ctx, int64_t ngp, const double* d_dist, const dou
 struct SignPlan {
   int64_t Rx = 0, Ry = 0, Rz = 0, nrows = 0;
   int32_t *row_cnt = nullptr, *row_off = nullptr, *row_cur = nullptr;
+  uint32_t* row_flags = nullptr;
 };
 int sign_begin(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P);
 int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int max_rays, double conf_thresh,

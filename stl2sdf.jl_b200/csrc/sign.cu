@@ -24,6 +24,7 @@
 //     per node with a fixed-order block reduction.
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -167,14 +168,34 @@ __device__ __forceinline__ bool axis_range2(const GridP& g, int a, double x0, do
   return lo <= hi;
 }
 
-template <int AX>
-__device__ __forceinline__ void tri_rows(const GridP& g, const TriRec64& r, bool fill, int64_t row_base,
-                                         int32_t* row_cnt, const int32_t* row_off, int32_t* row_cur, RowHit* hits,
-                                         double2* where, int64_t& nhit, int64_t& nband) {
+struct RowArgs {
+  GridP g;
+  const TriRec64* rec;
+  const float4* box32;
+  int64_t nel;
+  int chunk;            // triangles per block, a multiple of kRowThreads
+  float ihf, bo[3], rm;  // node = ihf * (mesh-local FP32 coordinate) + bo, within rm cells
+  int64_t base_y, base_z;
+  int32_t* row_cnt;
+  const int32_t* row_off;
+  int32_t* row_cur;
+  RowHit* hits;
+  double2* where;
+  uint32_t* flags;      // a byte per triangle: the axes on which it has hits
+  int64_t* counters;
+};
+
+template <int AX, bool kFill>
+__device__ __forceinline__ bool tri_rows(const RowArgs& A, const TriRec64& r, int64_t& nhit, int64_t& nband) {
+  const GridP& g = A.g;
   const int b = AX == 0 ? 1 : 0, c = AX == 2 ? 1 : 2;
+  const int64_t row_base = AX == 0 ? 0 : (AX == 1 ? A.base_y : A.base_z);
   int64_t b0, b1, c0, c1;
-  if (!axis_range2(g, b, r.bmin[b], r.bmax[b], b0, b1)) return;
-  if (!axis_range2(g, c, r.bmin[c], r.bmax[c], c0, c1)) return;
+  if (!axis_range2(g, b, fmin(r.v[b], fmin(r.v[3 + b], r.v[6 + b])), fmax(r.v[b], fmax(r.v[3 + b], r.v[6 + b])), b0, b1))
+    return false;
+  if (!axis_range2(g, c, fmin(r.v[c], fmin(r.v[3 + c], r.v[6 + c])), fmax(r.v[c], fmax(r.v[3 + c], r.v[6 + c])), c0, c1))
+    return false;
+  bool hit = false;
   for (int64_t jc = c0; jc <= c1; ++jc) {
     const double oc = da(g.o[c], dm(g.h, (double)gidx(g, c, jc)));
     for (int64_t jb = b0; jb <= b1; ++jb) {
@@ -182,14 +203,18 @@ __device__ __forceinline__ void tri_rows(const GridP& g, const TriRec64& r, bool
       const int64_t row = row_base + jc * g.n[b] + jb;
       const int dec = row_test32<AX>(r, ob, oc);
       if (dec == 0) continue;
-      if (!fill) {
+      if (!kFill) {
         if (dec == 2) ++nband;  // inside the FP32 band: the FP64 test decides
-        if (dec == 1 || row_test<AX>(r, ob, oc, nullptr)) { atomicAdd(&row_cnt[row], 1); ++nhit; }
+        if (dec == 1 || row_test<AX>(r, ob, oc, nullptr)) {
+          atomicAdd(&A.row_cnt[row], 1);
+          ++nhit;
+          hit = true;
+        }
       } else {
         RowHit R;
         if (row_test<AX>(r, ob, oc, &R)) {  // the hit's FP64 constants (and the band's decision)
-          const int32_t pos = row_off[row] + atomicAdd(&row_cur[row], 1);
-          hits[pos] = R;
+          const int32_t pos = A.row_off[row] + atomicAdd(&A.row_cur[row], 1);
+          A.hits[pos] = R;
           // the hit's coordinate, and a bound on |t - (coordinate - xa)| over the row's nodes: t is formed
           // from terms of these absolute sums by at most a dozen roundings, f's own error among them
           const double x0 = g.o[AX] + g.h * (double)gidx(g, AX, 0), x1 = g.o[AX] + g.h * (double)gidx(g, AX, g.N[AX]);
@@ -197,30 +222,82 @@ __device__ __forceinline__ void tri_rows(const GridP& g, const TriRec64& r, bool
           const double sum = fabs(R.P) + fabs(R.fa) * (fabs(R.K1) + S * fabs(R.ea)) +
                              fabs(R.fb) * (fabs(R.K2) + S * fabs(R.eb));
           const double x = R.v1a + row_t<AX>(R, R.v1a), e = 7.2e-15 * (fabs(R.f) * sum + S + fabs(R.v1a));
-          where[pos] = make_double2(x, e);
+          A.where[pos] = make_double2(x, e);
         }
       }
     }
   }
+  return hit;
 }
 
-__global__ void k_rows(const TriRec64* __restrict__ rec, int64_t nel, GridP g, int64_t base_y, int64_t base_z,
-                       bool fill, int32_t* row_cnt, const int32_t* row_off, int32_t* row_cur, RowHit* hits,
-                       double2* where, int64_t* counters) {
-  int64_t nhit = 0, nband = 0;
-  for (int64_t el = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; el < nel; el += (int64_t)gridDim.x * blockDim.x) {
-    const TriRec64 r = rec[el];
-    tri_rows<0>(g, r, fill, 0, row_cnt, row_off, row_cur, hits, where, nhit, nband);
-    tri_rows<1>(g, r, fill, base_y, row_cnt, row_off, row_cur, hits, where, nhit, nband);
-    tri_rows<2>(g, r, fill, base_z, row_cnt, row_off, row_cur, hits, where, nhit, nband);
+// The row hits: counted per row, then (kFill) written to their places.  A block lists its triangles per
+// axis -- those with a row of the grid across their box (FP32, with a margin), in the second pass those
+// that had hits -- and works the lists off, so that the warps of the FP64 part are full whatever share of
+// the triangles reaches a row.  Measured for both passes on 1.4M and 5.8M triangles (B200): 106 and 428 us,
+// against 209 and 800 with a thread per triangle for all axes.  Bound: the latency of the records' reads.
+constexpr int kRowThreads = 128, kRowChunk = 8 * kRowThreads;
+
+template <bool kFill>
+__global__ void __launch_bounds__(kRowThreads) k_rows(const __grid_constant__ RowArgs A) {
+  __shared__ uint16_t s_list[3][kRowChunk];
+  __shared__ uint32_t s_flag[kRowChunk / 4];
+  __shared__ int s_n[3];
+  const int lane = threadIdx.x & 31;
+  const int64_t first = (int64_t)blockIdx.x * A.chunk;
+  const int m = (int)min((int64_t)A.chunk, A.nel - first);
+  if (threadIdx.x < 3) s_n[threadIdx.x] = 0;
+  for (int t = threadIdx.x; t < A.chunk / 4; t += kRowThreads)
+    s_flag[t] = kFill && 4 * t < m ? A.flags[first / 4 + t] : 0u;
+  __syncthreads();
+  for (int t0 = 0; t0 < m; t0 += kRowThreads) {
+    const int t = t0 + threadIdx.x;
+    unsigned want = 0u;  // axes whose rows may meet the triangle
+    if (t < m) {
+      if (kFill) {
+        want = (s_flag[t >> 2] >> (8 * (t & 3))) & 7u;
+      } else {
+        const float4 b0 = A.box32[2 * (first + t)], b1 = A.box32[2 * (first + t) + 1];
+        const float lo[3] = {b0.x, b0.y, b0.z}, hi[3] = {b1.x, b1.y, b1.z};
+        bool some[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          const float f0 = fmaf(lo[a], A.ihf, A.bo[a]) - A.rm, f1 = fmaf(hi[a], A.ihf, A.bo[a]) + A.rm;
+          some[a] = !(floorf(f1) < ceilf(f0) || f1 < 0.f || f0 > (float)A.g.N[a]);
+        }
+        want = (unsigned)(some[1] && some[2]) | (unsigned)(some[0] && some[2]) << 1 | (unsigned)(some[0] && some[1]) << 2;
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const unsigned in = __ballot_sync(0xffffffffu, (want >> a) & 1u);
+      if (!in) continue;
+      int at = 0;
+      if (lane == 0) at = atomicAdd(&s_n[a], __popc(in));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if ((want >> a) & 1u) s_list[a][at + __popc(in & ((1u << lane) - 1u))] = (uint16_t)t;
+    }
   }
-  if (!fill) {
+  __syncthreads();
+  int64_t nhit = 0, nband = 0;
+  auto axis = [&](auto ax) {
+    constexpr int AX = decltype(ax)::value;
+    for (int q = threadIdx.x; q < s_n[AX]; q += kRowThreads) {
+      const int t = s_list[AX][q];
+      if (tri_rows<AX, kFill>(A, A.rec[first + t], nhit, nband)) atomicOr(&s_flag[t >> 2], 1u << (8 * (t & 3) + AX));
+    }
+  };
+  axis(std::integral_constant<int, 0>());
+  axis(std::integral_constant<int, 1>());
+  axis(std::integral_constant<int, 2>());
+  if (!kFill) {
+    __syncthreads();
+    for (int t = threadIdx.x; 4 * t < m; t += kRowThreads) A.flags[first / 4 + t] = s_flag[t];
     for (int off = 16; off > 0; off >>= 1) {
       nhit += __shfl_down_sync(0xffffffffu, nhit, off);
       nband += __shfl_down_sync(0xffffffffu, nband, off);
     }
-    if ((threadIdx.x & 31) == 0 && nhit) count_add(counters, C_ROW_HITS, nhit);
-    if ((threadIdx.x & 31) == 0 && nband) count_add(counters, C_SIGN_BAND, nband);
+    if (lane == 0 && nhit) count_add(A.counters, C_ROW_HITS, nhit);
+    if (lane == 0 && nband) count_add(A.counters, C_SIGN_BAND, nband);
   }
 }
 
@@ -885,10 +962,32 @@ int upload_directions(sdfgpu_ctx* ctx, const double* dirs) {
   return 0;
 }
 
+static RowArgs row_args(sdfgpu_ctx* ctx, const GridP& g, const SignPlan& P) {
+  const MeshDev& M = ctx->mesh;
+  RowArgs A{};
+  A.g = g;
+  A.rec = buf<TriRec64>(ctx, "rec");
+  A.box32 = buf<float4>(ctx, "box32");
+  A.nel = M.nel;
+  // few triangles: a block for each kRowThreads of them, so that they fill the GPU; many: full warps
+  A.chunk = kRowThreads * (int)std::min<int64_t>(kRowChunk / kRowThreads, 1 + M.nel / (kRowThreads * 148 * 8));
+  const double ih = 1.0 / g.h;
+  A.ihf = (float)ih;
+  for (int a = 0; a < 3; ++a) A.bo[a] = (float)((M.center[a] - (g.o[a] + g.h * (double)gidx(g, a, 0))) * ih);
+  A.rm = (float)(2e-6 * g.E * ih + 1e-4);
+  A.base_y = P.Rx;
+  A.base_z = P.Rx + P.Ry;
+  A.row_cnt = P.row_cnt;
+  A.row_off = P.row_off;
+  A.row_cur = P.row_cur;
+  A.flags = P.row_flags;
+  A.counters = ctx->d_counters;
+  return A;
+}
+
 int sign_begin(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P) {
   cudaStream_t st = ctx->sign_stream;
   const int64_t nel = ctx->mesh.nel;
-  const TriRec64* rec = buf<TriRec64>(ctx, "rec");
   P.Rx = g.n[1] * g.n[2];
   P.Ry = g.n[0] * g.n[2];
   P.Rz = g.n[0] * g.n[1];
@@ -899,8 +998,9 @@ int sign_begin(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P) {
   SDF_TRY(scratch_t(ctx, "row_cur", (size_t)P.nrows + 1, &P.row_cur));
   SDF_CUDA(ctx, cudaMemsetAsync(P.row_cnt, 0, sizeof(int32_t) * (P.nrows + 1), st));
   SDF_CUDA(ctx, cudaMemsetAsync(P.row_cur, 0, sizeof(int32_t) * (P.nrows + 1), st));
-  k_rows<<<grid_for(nel, 128), 128, 0, st>>>(rec, nel, g, P.Rx, P.Rx + P.Ry, false, P.row_cnt, nullptr, nullptr,
-                                             nullptr, nullptr, ctx->d_counters);
+  SDF_TRY(scratch_t(ctx, "row_flags", (size_t)cdiv(nel, 4), &P.row_flags));
+  const RowArgs A = row_args(ctx, g, P);
+  k_rows<false><<<(unsigned)cdiv(nel, A.chunk), kRowThreads, 0, st>>>(A);
   SDF_KERNEL(ctx);
   SDF_TRY(cub_scan_i32(ctx, P.row_cnt, P.row_off, P.nrows + 1, st, "cub_tmp_scan_sign"));
   ctx->h_scalars[S_ROW_TOTAL] = -1;
@@ -917,7 +1017,7 @@ int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int 
   const int64_t nel = M.nel;
   const TriRec64* rec = buf<TriRec64>(ctx, "rec");
   const int64_t Rx = P.Rx, Ry = P.Ry, nrows = P.nrows;
-  int32_t *row_cnt = P.row_cnt, *row_off = P.row_off, *row_cur = P.row_cur;
+  int32_t *row_cnt = P.row_cnt, *row_off = P.row_off;
   SDF_CUDA(ctx, cudaEventSynchronize(ctx->ev_rows));
   int32_t total;
   std::memcpy(&total, ctx->h_scalars + S_ROW_TOTAL, sizeof(int32_t));  // the low 4 bytes hold the int32
@@ -943,8 +1043,10 @@ int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int 
   for (int a = 0; a < 3; ++a) K.mbase[a + 1] = K.mbase[a] + cdiv(g.n[a], 32) * K.nrows[a];
   SDF_TRY(scratch_t(ctx, "row_mask", (size_t)K.mbase[3], &K.mask));
   if (total > 0) {
-    k_rows<<<grid_for(nel, 128), 128, 0, st>>>(rec, nel, g, Rx, Rx + Ry, true, nullptr, row_off, row_cur, hits, where,
-                                               ctx->d_counters);
+    RowArgs A = row_args(ctx, g, P);
+    A.hits = hits;
+    A.where = where;
+    k_rows<true><<<(unsigned)cdiv(nel, A.chunk), kRowThreads, 0, st>>>(A);
     SDF_KERNEL(ctx);
   }
   k_row_info<<<grid_for(nrows, 256), 256, 0, st>>>(nrows, row_off, row_cnt, where, info, over);
