@@ -173,7 +173,8 @@ struct RowArgs {
   const TriRec64* rec;
   const float4* box32;
   int64_t nel;
-  int chunk;            // triangles per block, a multiple of kRowThreads
+  int chunk;            // triangles per block, a multiple of 32
+  int lanes;            // threads per triangle and axis, a power of two; times gridDim.z blocks
   float ihf, bo[3], rm;  // node = ihf * (mesh-local FP32 coordinate) + bo, within rm cells
   int64_t base_y, base_z;
   int32_t* row_cnt;
@@ -181,12 +182,14 @@ struct RowArgs {
   int32_t* row_cur;
   RowHit* hits;
   double2* where;
-  uint32_t* flags;      // a byte per triangle: the axes on which it has hits
+  int32_t* hrow;
+  uint32_t* flags[3];   // per axis a bit per triangle: whether it has hits
   int64_t* counters;
 };
 
 template <int AX, bool kFill>
-__device__ __forceinline__ bool tri_rows(const RowArgs& A, const TriRec64& r, int64_t& nhit, int64_t& nband) {
+__device__ __forceinline__ bool tri_rows(const RowArgs& A, const TriRec64& r, uint32_t sub, uint32_t stride, int64_t& nhit,
+                                         int64_t& nband) {
   const GridP& g = A.g;
   const int b = AX == 0 ? 1 : 0, c = AX == 2 ? 1 : 2;
   const int64_t row_base = AX == 0 ? 0 : (AX == 1 ? A.base_y : A.base_z);
@@ -196,34 +199,35 @@ __device__ __forceinline__ bool tri_rows(const RowArgs& A, const TriRec64& r, in
   if (!axis_range2(g, c, fmin(r.v[c], fmin(r.v[3 + c], r.v[6 + c])), fmax(r.v[c], fmax(r.v[3 + c], r.v[6 + c])), c0, c1))
     return false;
   bool hit = false;
-  for (int64_t jc = c0; jc <= c1; ++jc) {
-    const double oc = da(g.o[c], dm(g.h, (double)gidx(g, c, jc)));
-    for (int64_t jb = b0; jb <= b1; ++jb) {
-      const double ob = da(g.o[b], dm(g.h, (double)gidx(g, b, jb)));
-      const int64_t row = row_base + jc * g.n[b] + jb;
-      const int dec = row_test32<AX>(r, ob, oc);
-      if (dec == 0) continue;
-      if (!kFill) {
-        if (dec == 2) ++nband;  // inside the FP32 band: the FP64 test decides
-        if (dec == 1 || row_test<AX>(r, ob, oc, nullptr)) {
-          atomicAdd(&A.row_cnt[row], 1);
-          ++nhit;
-          hit = true;
-        }
-      } else {
-        RowHit R;
-        if (row_test<AX>(r, ob, oc, &R)) {  // the hit's FP64 constants (and the band's decision)
-          const int32_t pos = A.row_off[row] + atomicAdd(&A.row_cur[row], 1);
-          A.hits[pos] = R;
-          // the hit's coordinate, and a bound on |t - (coordinate - xa)| over the row's nodes: t is formed
-          // from terms of these absolute sums by at most a dozen roundings, f's own error among them
-          const double x0 = g.o[AX] + g.h * (double)gidx(g, AX, 0), x1 = g.o[AX] + g.h * (double)gidx(g, AX, g.N[AX]);
-          const double S = fmax(fabs(x0 - R.v1a), fabs(x1 - R.v1a));
-          const double sum = fabs(R.P) + fabs(R.fa) * (fabs(R.K1) + S * fabs(R.ea)) +
-                             fabs(R.fb) * (fabs(R.K2) + S * fabs(R.eb));
-          const double x = R.v1a + row_t<AX>(R, R.v1a), e = 7.2e-15 * (fabs(R.f) * sum + S + fabs(R.v1a));
-          A.where[pos] = make_double2(x, e);
-        }
+  const uint32_t nb = (uint32_t)(b1 - b0 + 1), rows = nb * (uint32_t)(c1 - c0 + 1);
+  for (uint32_t q = sub; q < rows; q += stride) {
+    const uint32_t qc = q / nb;
+    const int64_t jc = c0 + qc, jb = b0 + (q - qc * nb);
+    const double oc = da(g.o[c], dm(g.h, (double)gidx(g, c, jc))), ob = da(g.o[b], dm(g.h, (double)gidx(g, b, jb)));
+    const int64_t row = row_base + jc * g.n[b] + jb;
+    const int dec = row_test32<AX>(r, ob, oc);
+    if (dec == 0) continue;
+    if (!kFill) {
+      if (dec == 2) ++nband;  // inside the FP32 band: the FP64 test decides
+      if (dec == 1 || row_test<AX>(r, ob, oc, nullptr)) {
+        atomicAdd(&A.row_cnt[row], 1);
+        ++nhit;
+        hit = true;
+      }
+    } else {
+      RowHit R;
+      if (row_test<AX>(r, ob, oc, &R)) {  // the hit's FP64 constants (and the band's decision)
+        const int32_t pos = A.row_off[row] + atomicAdd(&A.row_cur[row], 1);
+        A.hits[pos] = R;
+        // the hit's coordinate, and a bound on |t - (coordinate - xa)| over the row's nodes: t is formed
+        // from terms of these absolute sums by at most a dozen roundings, f's own error among them
+        const double x0 = g.o[AX] + g.h * (double)gidx(g, AX, 0), x1 = g.o[AX] + g.h * (double)gidx(g, AX, g.N[AX]);
+        const double S = fmax(fabs(x0 - R.v1a), fabs(x1 - R.v1a));
+        const double sum = fabs(R.P) + fabs(R.fa) * (fabs(R.K1) + S * fabs(R.ea)) +
+                           fabs(R.fb) * (fabs(R.K2) + S * fabs(R.eb));
+        const double x = R.v1a + row_t<AX>(R, R.v1a), e = 7.2e-15 * (fabs(R.f) * sum + S + fabs(R.v1a));
+        A.where[pos] = make_double2(x, e);
+        A.hrow[pos] = (int32_t)row;
       }
     }
   }
@@ -235,26 +239,30 @@ __device__ __forceinline__ bool tri_rows(const RowArgs& A, const TriRec64& r, in
 // that had hits -- and works the lists off, so that the warps of the FP64 part are full whatever share of
 // the triangles reaches a row.  Measured for both passes on 1.4M and 5.8M triangles (B200): 106 and 428 us,
 // against 209 and 800 with a thread per triangle for all axes.  Bound: the latency of the records' reads.
+// Meshes too small to fill the GPU that way get a block per axis (gridDim.y) and several threads and blocks
+// (gridDim.z) for the rows of one triangle: 5k triangles on 149k nodes 54 -> 14 us.
 constexpr int kRowThreads = 128, kRowChunk = 8 * kRowThreads;
 
 template <bool kFill>
 __global__ void __launch_bounds__(kRowThreads) k_rows(const __grid_constant__ RowArgs A) {
   __shared__ uint16_t s_list[3][kRowChunk];
-  __shared__ uint32_t s_flag[kRowChunk / 4];
+  __shared__ uint32_t s_flag[3][kRowChunk / 32];
   __shared__ int s_n[3];
   const int lane = threadIdx.x & 31;
   const int64_t first = (int64_t)blockIdx.x * A.chunk;
   const int m = (int)min((int64_t)A.chunk, A.nel - first);
+  const unsigned axes = gridDim.y == 1 ? 7u : 1u << blockIdx.y;
   if (threadIdx.x < 3) s_n[threadIdx.x] = 0;
-  for (int t = threadIdx.x; t < A.chunk / 4; t += kRowThreads)
-    s_flag[t] = kFill && 4 * t < m ? A.flags[first / 4 + t] : 0u;
+  for (int t = threadIdx.x; t < 3 * (kRowChunk / 32); t += kRowThreads) s_flag[0][t] = 0u;
   __syncthreads();
   for (int t0 = 0; t0 < m; t0 += kRowThreads) {
     const int t = t0 + threadIdx.x;
     unsigned want = 0u;  // axes whose rows may meet the triangle
     if (t < m) {
       if (kFill) {
-        want = (s_flag[t >> 2] >> (8 * (t & 3))) & 7u;
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+          if ((axes >> a) & 1u) want |= ((A.flags[a][(first + t) >> 5] >> (t & 31)) & 1u) << a;
       } else {
         const float4 b0 = A.box32[2 * (first + t)], b1 = A.box32[2 * (first + t) + 1];
         const float lo[3] = {b0.x, b0.y, b0.z}, hi[3] = {b1.x, b1.y, b1.z};
@@ -264,7 +272,7 @@ __global__ void __launch_bounds__(kRowThreads) k_rows(const __grid_constant__ Ro
           const float f0 = fmaf(lo[a], A.ihf, A.bo[a]) - A.rm, f1 = fmaf(hi[a], A.ihf, A.bo[a]) + A.rm;
           some[a] = !(floorf(f1) < ceilf(f0) || f1 < 0.f || f0 > (float)A.g.N[a]);
         }
-        want = (unsigned)(some[1] && some[2]) | (unsigned)(some[0] && some[2]) << 1 | (unsigned)(some[0] && some[1]) << 2;
+        want = axes & ((unsigned)(some[1] && some[2]) | (unsigned)(some[0] && some[2]) << 1 | (unsigned)(some[0] && some[1]) << 2);
       }
     }
 #pragma unroll
@@ -281,9 +289,11 @@ __global__ void __launch_bounds__(kRowThreads) k_rows(const __grid_constant__ Ro
   int64_t nhit = 0, nband = 0;
   auto axis = [&](auto ax) {
     constexpr int AX = decltype(ax)::value;
-    for (int q = threadIdx.x; q < s_n[AX]; q += kRowThreads) {
+    const uint32_t L = (uint32_t)A.lanes, sub = threadIdx.x & (L - 1u);
+    for (int q = threadIdx.x / L; q < s_n[AX]; q += kRowThreads / L) {
       const int t = s_list[AX][q];
-      if (tri_rows<AX, kFill>(A, A.rec[first + t], nhit, nband)) atomicOr(&s_flag[t >> 2], 1u << (8 * (t & 3) + AX));
+      if (tri_rows<AX, kFill>(A, A.rec[first + t], sub + L * blockIdx.z, L * gridDim.z, nhit, nband))
+        atomicOr(&s_flag[AX][t >> 5], 1u << (t & 31));
     }
   };
   axis(std::integral_constant<int, 0>());
@@ -291,7 +301,8 @@ __global__ void __launch_bounds__(kRowThreads) k_rows(const __grid_constant__ Ro
   axis(std::integral_constant<int, 2>());
   if (!kFill) {
     __syncthreads();
-    for (int t = threadIdx.x; 4 * t < m; t += kRowThreads) A.flags[first / 4 + t] = s_flag[t];
+    for (int t = threadIdx.x; t < 3 * (kRowChunk / 32); t += kRowThreads)
+      if (s_flag[0][t]) atomicOr(A.flags[t / (kRowChunk / 32)] + (first >> 5) + t % (kRowChunk / 32), s_flag[0][t]);
     for (int off = 16; off > 0; off >>= 1) {
       nhit += __shfl_down_sync(0xffffffffu, nhit, off);
       nband += __shfl_down_sync(0xffffffffu, nband, off);
@@ -301,35 +312,38 @@ __global__ void __launch_bounds__(kRowThreads) k_rows(const __grid_constant__ Ro
   }
 }
 
-// Per row: the first hit, and their number with two flags.  Hits certainly within eps / 4 of one another
-// are one hit to every node outside their bounds: all but the first get a negative bound (its magnitude
-// stays), and kRowOdd says whether the number of distinct hits is odd.  kRowClose: two hits of the row
-// are neither that close nor certainly more than eps apart, or there are too many of them to compare
-// (then over[0] counts the row too).
-constexpr int kRowClose = 1 << 30, kRowOdd = 1 << 29, kRowCount = kRowOdd - 1;
-__global__ void k_row_info(int64_t nrows, const int32_t* __restrict__ row_off, const int32_t* __restrict__ row_cnt,
-                           double2* __restrict__ where, int2* __restrict__ info, int32_t* __restrict__ over) {
-  for (int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; row < nrows; row += (int64_t)gridDim.x * blockDim.x) {
-    const int off = row_off[row], n = row_cnt[row];
-    bool close = n > kRowCap;
-    if (close) atomicAdd(over, 1);
-    int distinct = n;
-    for (int a = 1; a < n && !close; ++a) {
-      const double2 p = where[off + a];
-      bool same = false;
-      for (int b = 0; b < a && !close; ++b) {
-        const double2 q = where[off + b];
-        const double gap = fabs(p.x - q.x), e = 2.0 * (p.y + fabs(q.y));
-        const bool near = gap + e < 0.25 * kEps;
-        same = same || near;
-        close = !near && !(gap > kEps + e);
+// Per row two flags, from its hits, a thread per hit against those before it.  Hits certainly within eps / 4
+// of one another are one hit to every node outside their bounds: all but the first get a negative bound (its
+// magnitude stays), and kRowOdd says whether their number is odd.  kRowClose: two hits of the row are neither
+// that close nor certainly more than eps apart, or there are too many of them to compare (then over[0] counts
+// the row too).  A thread per row took 61 us where rows have up to a few dozen hits (131k triangles, 24k rows),
+// this 6 us (B200).
+constexpr unsigned kRowClose = 1u, kRowOdd = 2u;
+__global__ void k_hit_info(int64_t total, const int32_t* __restrict__ hrow, const int32_t* __restrict__ row_off,
+                           const int32_t* __restrict__ row_cnt, double2* __restrict__ where, uint32_t* __restrict__ flag,
+                           int32_t* __restrict__ over) {
+  for (int64_t h = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; h < total; h += (int64_t)gridDim.x * blockDim.x) {
+    const int row = hrow[h], off = row_off[row], n = row_cnt[row], a = (int)(h - off);
+    if (n > kRowCap) {
+      if (a == 0) {
+        atomicAdd(over, 1);
+        atomicOr(flag + row, kRowClose);
       }
-      if (same) {
-        where[off + a].y = -p.y;
-        --distinct;
-      }
+      continue;
     }
-    info[row] = make_int2(off, n | (close ? kRowClose : 0) | ((distinct & 1) ? kRowOdd : 0));
+    const double px = where[h].x, py = fabs(where[h].y);
+    bool same = false, close = false;
+    for (int b = 0; b < a; ++b) {
+      const double gap = fabs(px - where[off + b].x), e = 2.0 * (py + fabs(where[off + b].y));
+      const bool near = gap + e < 0.25 * kEps;
+      same = same || near;
+      close = close || (!near && !(gap > kEps + e));
+    }
+    if (close) atomicOr(flag + row, kRowClose);
+    if (same) {
+      where[h].y = -py;
+      atomicXor(flag + row, kRowOdd);
+    }
   }
 }
 
@@ -374,7 +388,8 @@ struct MaskArgs {
   GridP g;
   int64_t nrows[3], base[3];  // rows along x, y, z, and the first of each among all rows
   int64_t mbase[4];           // first mask word of each axis, and their number
-  const int2* info;
+  const int32_t *off, *cnt;   // per row: its first hit, their number
+  const uint32_t* flag;       // and flags (k_hit_info)
   const RowHit* hits;
   const double2* where;
   uint2* mask;  // per axis [word of 32 nodes][row]: bits of the +AX and of the -AX ray
@@ -386,17 +401,19 @@ template <int AX>
 __device__ __forceinline__ void row_mask(const MaskArgs& A, int64_t q) {
   const GridP& g = A.g;
   const int64_t word = q / A.nrows[AX], row = q - word * A.nrows[AX];
-  const int2 in = A.info[A.base[AX] + row];
-  const int n = in.y & kRowCount;
+  const int64_t r0 = A.base[AX] + row;
+  const int n = A.cnt[r0];
   uint2 m = make_uint2(0u, 0u);
   if (n > 0 && n <= kRowCap) {
     const int first = (int)(word * 32), last = (int)min((int64_t)31, g.n[AX] - 1 - first);  // this word's nodes
-    unsigned exact = (in.y & kRowClose) ? 0xffffffffu : 0u;
+    const int off = A.off[r0];
+    const unsigned flag = A.flag[r0];
+    unsigned exact = (flag & kRowClose) ? 0xffffffffu : 0u;
     if (!exact) {
       const double o = g.o[AX] + g.h * (double)gidx(g, AX, 0), inv = 1.0 / g.h;
       const double slack = fabs(g.o[AX]) * inv + (double)g.n[AX] + 1.0;
       for (int a = 0; a < n; ++a) {
-        const double2 c = A.where[in.x + a];
+        const double2 c = A.where[off + a];
         // the hit in nodes from the row's first, and the half width of the window around it in which t's
         // sign against eps is open (eps, t's bound, and the roundings of this line and of the nodes)
         const double r = (c.x - o) * inv;
@@ -407,13 +424,13 @@ __device__ __forceinline__ void row_mask(const MaskArgs& A, int64_t q) {
         if (!signbit(c.y)) m.x ^= below;
         if (hi >= lo) exact |= (0xffffffffu >> (31 - hi)) & ~below;
       }
-      m.y = (in.y & kRowOdd) ? ~m.x : m.x;
+      m.y = (((unsigned)n & 1u) ^ ((flag & kRowOdd) ? 1u : 0u)) ? ~m.x : m.x;
     }
     exact &= 0xffffffffu >> (31 - last);
     while (exact) {
       const int b = __ffs(exact) - 1;
       exact &= exact - 1u;
-      const unsigned par = row_parity<AX>(A.hits + in.x, n, da(g.o[AX], dm(g.h, (double)gidx(g, AX, first + b))));
+      const unsigned par = row_parity<AX>(A.hits + off, n, da(g.o[AX], dm(g.h, (double)gidx(g, AX, first + b))));
       m.x = (m.x & ~(1u << b)) | ((par & 1u) << b);
       m.y = (m.y & ~(1u << b)) | ((par >> 1) << b);
     }
@@ -969,8 +986,6 @@ static RowArgs row_args(sdfgpu_ctx* ctx, const GridP& g, const SignPlan& P) {
   A.rec = buf<TriRec64>(ctx, "rec");
   A.box32 = buf<float4>(ctx, "box32");
   A.nel = M.nel;
-  // few triangles: a block for each kRowThreads of them, so that they fill the GPU; many: full warps
-  A.chunk = kRowThreads * (int)std::min<int64_t>(kRowChunk / kRowThreads, 1 + M.nel / (kRowThreads * 148 * 8));
   const double ih = 1.0 / g.h;
   A.ihf = (float)ih;
   for (int a = 0; a < 3; ++a) A.bo[a] = (float)((M.center[a] - (g.o[a] + g.h * (double)gidx(g, a, 0))) * ih);
@@ -980,9 +995,23 @@ static RowArgs row_args(sdfgpu_ctx* ctx, const GridP& g, const SignPlan& P) {
   A.row_cnt = P.row_cnt;
   A.row_off = P.row_off;
   A.row_cur = P.row_cur;
-  A.flags = P.row_flags;
+  for (int a = 0; a < 3; ++a) A.flags[a] = P.row_flags + a * cdiv(M.nel, 32);
   A.counters = ctx->d_counters;
   return A;
+}
+
+// The launch shape: as many threads per triangle and axis as fill the GPU, up to half the rows that the
+// mesh's largest triangle can meet; one block for all axes where the triangles alone fill it.
+static dim3 row_grid(const sdfgpu_ctx* ctx, RowArgs& A) {
+  const MeshDev& M = ctx->mesh;
+  const double side = std::min(2.0 * M.rho_max / A.g.h + 1.0, 64.0);
+  const int64_t threads = 148 * 2048;
+  int64_t per = 1;
+  while (2 * per <= 0.5 * side * side && M.nel * 3 * 2 * per <= threads) per *= 2;
+  A.lanes = (int)std::min<int64_t>(per, kRowThreads);
+  const int64_t z = per / A.lanes, y = M.nel * 3 <= threads ? 3 : 1;
+  A.chunk = 32 * (int)std::min<int64_t>(kRowChunk / 32, 1 + M.nel * y * z / (32 * 148 * 8));
+  return dim3((unsigned)cdiv(M.nel, A.chunk), (unsigned)y, (unsigned)z);
 }
 
 int sign_begin(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P) {
@@ -998,9 +1027,11 @@ int sign_begin(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P) {
   SDF_TRY(scratch_t(ctx, "row_cur", (size_t)P.nrows + 1, &P.row_cur));
   SDF_CUDA(ctx, cudaMemsetAsync(P.row_cnt, 0, sizeof(int32_t) * (P.nrows + 1), st));
   SDF_CUDA(ctx, cudaMemsetAsync(P.row_cur, 0, sizeof(int32_t) * (P.nrows + 1), st));
-  SDF_TRY(scratch_t(ctx, "row_flags", (size_t)cdiv(nel, 4), &P.row_flags));
-  const RowArgs A = row_args(ctx, g, P);
-  k_rows<false><<<(unsigned)cdiv(nel, A.chunk), kRowThreads, 0, st>>>(A);
+  SDF_TRY(scratch_t(ctx, "row_flags", (size_t)cdiv(nel, 32) * 3, &P.row_flags));
+  SDF_CUDA(ctx, cudaMemsetAsync(P.row_flags, 0, sizeof(uint32_t) * cdiv(nel, 32) * 3, st));
+  RowArgs A = row_args(ctx, g, P);
+  const dim3 grid = row_grid(ctx, A);
+  k_rows<false><<<grid, kRowThreads, 0, st>>>(A);
   SDF_KERNEL(ctx);
   SDF_TRY(cub_scan_i32(ctx, P.row_cnt, P.row_off, P.nrows + 1, st, "cub_tmp_scan_sign"));
   ctx->h_scalars[S_ROW_TOTAL] = -1;
@@ -1024,15 +1055,16 @@ int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int 
   if (total < 0) return fail(ctx, SDFGPU_ERR_CAPACITY, "more than 2^31 row hits");
   RowHit* hits;
   double2* where;
-  int2* info;
-  int32_t* over;
+  int32_t *hrow, *over;
+  uint32_t* row_flag;
   MaskArgs K;
   const size_t H = (size_t)std::max(total, 1);
   SDF_TRY(scratch_t(ctx, "row_hits", H, &hits));
   SDF_TRY(scratch_t(ctx, "row_where", H, &where));
-  SDF_TRY(scratch_t(ctx, "row_info", (size_t)nrows, &info));
-  SDF_TRY(scratch_t(ctx, "row_over", (size_t)1, &over));
-  SDF_CUDA(ctx, cudaMemsetAsync(over, 0, sizeof(int32_t), st));
+  SDF_TRY(scratch_t(ctx, "row_hrow", H, &hrow));
+  SDF_TRY(scratch_t(ctx, "row_flag", (size_t)nrows + 1, &row_flag));  // and the number of overfull rows
+  over = reinterpret_cast<int32_t*>(row_flag + nrows);
+  SDF_CUDA(ctx, cudaMemsetAsync(row_flag, 0, sizeof(uint32_t) * (nrows + 1), st));
   K.nrows[0] = Rx;
   K.nrows[1] = Ry;
   K.nrows[2] = P.Rz;
@@ -1046,14 +1078,18 @@ int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int 
     RowArgs A = row_args(ctx, g, P);
     A.hits = hits;
     A.where = where;
-    k_rows<true><<<(unsigned)cdiv(nel, A.chunk), kRowThreads, 0, st>>>(A);
+    A.hrow = hrow;
+    const dim3 grid = row_grid(ctx, A);
+    k_rows<true><<<grid, kRowThreads, 0, st>>>(A);
+    SDF_KERNEL(ctx);
+    k_hit_info<<<grid_for(total, 128), 128, 0, st>>>(total, hrow, row_off, row_cnt, where, row_flag, over);
     SDF_KERNEL(ctx);
   }
-  k_row_info<<<grid_for(nrows, 256), 256, 0, st>>>(nrows, row_off, row_cnt, where, info, over);
-  SDF_KERNEL(ctx);
   SDF_MARK_ON(ctx, T_ROWS, st);
   K.g = g;
-  K.info = info;
+  K.off = row_off;
+  K.cnt = row_cnt;
+  K.flag = row_flag;
   K.hits = hits;
   K.where = where;
   k_row_masks<<<(unsigned)cdiv(K.mbase[3], 128), 128, 0, st>>>(K);

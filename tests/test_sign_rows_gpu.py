@@ -85,3 +85,13 @@ def test_slabs(gpu_ctx):
     plane = int((N[0] + 1) * (N[1] + 1))
     for k0, k1 in [(0, 0), (1, 5), (6, 20)]:
         assert np.array_equal(gpu_ctx.sdf_slab(o, h, N, k0, k1), whole[k0 * plane:(k1 + 1) * plane])
+
+
+@pytest.mark.parametrize("nel", [12, 36, 96, 120])
+@pytest.mark.parametrize("nodes", [12, 40, 97])
+def test_triangles_over_many_rows(gpu_ctx, nel, nodes):
+    """Few triangles, each across up to nodes^2 rows, so that several threads and blocks share one."""
+    rng = np.random.default_rng(nel)
+    X, F = boxes([(lo, lo + rng.uniform(0.2, 0.6, 3)) for lo in rng.uniform(0.0, 0.4, (nel // 12, 3))])
+    st = check(gpu_ctx, X, F, (-0.011, -0.017, -0.013), 1.1 / nodes, (nodes, nodes - 3, nodes // 2))
+    assert st["row_hits"] > 0
