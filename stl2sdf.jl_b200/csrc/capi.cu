@@ -184,9 +184,10 @@ int reset_counters(sdfgpu_ctx* ctx) {
 
 int finish_counters(sdfgpu_ctx* ctx, const GridP& g) {
   const int64_t tile_pairs = ctx->h_counters[C_TILE_PAIRS], band = ctx->h_counters[C_BAND];  // counted on the host
-  SDF_CUDA(ctx, cudaMemcpyAsync(ctx->h_counters, ctx->d_counters, sizeof(int64_t) * C_NUM, cudaMemcpyDeviceToHost,
-                                ctx->stream));
+  SDF_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + S_COUNTERS, ctx->d_counters, sizeof(int64_t) * C_NUM,
+                                cudaMemcpyDeviceToHost, ctx->stream));
   SDF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  std::memcpy(ctx->h_counters, ctx->h_scalars + S_COUNTERS, sizeof(int64_t) * C_NUM);
   ctx->h_counters[C_TILE_PAIRS] = tile_pairs;
   ctx->h_counters[C_BAND] += band;
   sdfgpu_stats& s = ctx->stats;
@@ -244,10 +245,13 @@ int run_all(sdfgpu_ctx* ctx, const GridP& g, bool want_dist, bool want_sign, int
   }
   SDF_TRY(reset_counters(ctx));
   ctx->launches = 0;
-  for (int i = 0; i < T_NUM; ++i) SDF_MARK(ctx, i);
+  SDF_MARK(ctx, T_DIST0);
+  if (!(want_dist && want_sign) || defer)  // else every stage records its own
+    for (int i = 0; i < T_NUM; ++i) SDF_MARK(ctx, i);
   // The sign stage runs on its own stream, forked after the counters are cleared: its row counting
-  // is enqueued first, the distance stage next (its one host wait covers the row count too), and
-  // the rest of the sign stage while the distance fold runs.  The join precedes the combine.
+  // is enqueued first, the distance stage's lists next (its one host wait covers the row count too),
+  // then the rest of the sign stage up to the vote, whose chain of small kernels is the longer one on small
+  // meshes, and the distance fold beside it.  The join precedes the combine.
   cudaStream_t ss = ctx->sign_stream;
   SignPlan P;
   bool forked = false;
@@ -267,17 +271,19 @@ int run_all(sdfgpu_ctx* ctx, const GridP& g, bool want_dist, bool want_sign, int
       SDF_MARK_ON(ctx, T_SIGN0, ss);
       SDF_TRY(sign_begin(ctx, g, P));
     }
-    if (want_dist) {
-      if (defer)  // a batch runs the fold later, together with other meshes'
-        SDF_TRY(dist_prepare(ctx, g, mode, d_dist, d_xp, *defer, learned));
-      else
-        SDF_TRY(run_distances(ctx, g, mode, learned, d_dist, d_xp));
+    // Rays past the 36th are never cast, so every max_rays >= 44 gives the same votes as 44.
+    const int max_eff = max_rays > 44 ? 44 : max_rays;
+    const std::function<int()> vote = [&]() -> int {
+      return want_sign ? sign_vote(ctx, g, P, min_rays, max_eff, conf, use_winding, d_sign, d_conf) : 0;
+    };
+    if (want_dist && !defer) {
+      SDF_TRY(run_distances(ctx, g, mode, learned, d_dist, d_xp, vote));
+    } else {
+      if (want_dist) SDF_TRY(dist_prepare(ctx, g, mode, d_dist, d_xp, *defer, learned));  // a batch runs the fold later
+      SDF_TRY(vote());
     }
     SDF_MARK(ctx, T_DIST1);
     if (want_sign) {
-      for (int i = T_ROWS; i <= T_PARITY; ++i) SDF_MARK_ON(ctx, i, ss);
-      // Rays past the 36th are never cast, so every max_rays >= 44 gives the same votes as 44.
-      const int max_eff = max_rays > 44 ? 44 : max_rays;
       SDF_TRY(sign_finish(ctx, g, P, min_rays, max_eff, conf, use_winding, d_sign, d_conf));
       SDF_MARK_ON(ctx, T_SIGN1, ss);
     }

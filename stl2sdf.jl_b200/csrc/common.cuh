@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <functional>
 #include <map>
 #include <string>
 #include <unordered_map>
@@ -164,7 +165,9 @@ enum Stage : int { T_DIST0 = 0, T_TILES, T_FOLD, T_DIST1, T_ROWS, T_PARITY, T_SI
 
 // Slots of ctx->h_scalars: device counts read back to size the next stage.  Page-locked, so the
 // read is an asynchronous copy the host waits for only when it needs the value.
-enum Scalar : int { S_ROW_TOTAL = 0, S_UNDECIDED, S_WINDING, S_NUM = 8 };
+// S_UNDECIDED and S_WINDING are read in one copy; S_MESH: the mesh's scalars (mesh.cu).
+enum Scalar : int { S_ROW_TOTAL = 0, S_UNDECIDED, S_WINDING, S_NEAR, S_MESH = 8, S_COUNTERS = 18, S_NUM = S_COUNTERS + C_NUM };
+static_assert(C_LIST_WINDING == C_LIST_UNDECIDED + 1 && S_WINDING == S_UNDECIDED + 1, "the lists' lengths are read together");
 
 #define SDF_TRY(expr)          \
   do {                         \
@@ -250,7 +253,10 @@ int mesh_upload_and_build(sdfgpu_ctx* ctx, const double* X, int64_t nnp, const i
                           bool device_ptrs);
 int ensure_ine(sdfgpu_ctx* ctx);
 int ensure_tree(sdfgpu_ctx* ctx, bool boxes);
-int run_distances(sdfgpu_ctx* ctx, const GridP& g, int mode, int use_learned, double* d_dist, double* d_xp);
+// `between` (may be empty) runs once the host has waited for the stage's lists and before their use is
+// enqueued, or after an unbounded search has been.
+int run_distances(sdfgpu_ctx* ctx, const GridP& g, int mode, int use_learned, double* d_dist, double* d_xp,
+                  const std::function<int()>& between = {});
 // Exact unbounded distances of a sparse grid's nodes, one thread per node (learned.cu).
 int run_nearest_points(sdfgpu_ctx* ctx, const GridP& g, double* d_dist);
 
@@ -299,16 +305,21 @@ int unb_multi(sdfgpu_ctx* ctx, const void* d_items, const int64_t* d_off, int co
               unsigned long long* heads, int64_t grid, cudaStream_t st);
 int launch_combine(sdfgpu_ctx* ctx, int64_t ngp, const double* d_dist, const double* d_sign, double* d_sdf,
                    cudaStream_t st);
-// The sign stage in two parts on ctx->sign_stream: sign_begin enqueues the axis-row counting and
-// returns without waiting; sign_finish waits for that count and enqueues the rest (lists, parities,
-// vote, adaptive rays, winding).  Between the two the caller can enqueue the distance stage, which
-// then overlaps the sign stage on the GPU.  d_sign / d_conf receive the results.
+// The sign stage in three parts on ctx->sign_stream: sign_begin enqueues the axis-row counting and
+// returns without waiting; sign_vote waits for that count and enqueues the row masks and the vote;
+// sign_finish waits for the vote's lists and does the rest (adaptive rays, winding).  Between them the
+// caller can enqueue the distance stage, which then overlaps the sign stage on the GPU.  d_sign /
+// d_conf receive the results.
 struct SignPlan {
   int64_t Rx = 0, Ry = 0, Rz = 0, nrows = 0;
   int32_t *row_cnt = nullptr, *row_off = nullptr, *row_cur = nullptr;
   uint32_t* row_flags = nullptr;
+  int32_t *und = nullptr, *wind = nullptr;  // undecided nodes, and those for the winding number
+  uint64_t *und_have = nullptr, *und_par = nullptr;
 };
 int sign_begin(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P);
+int sign_vote(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int max_rays, double conf_thresh,
+              int use_winding, double* d_sign, double* d_conf);
 int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int max_rays, double conf_thresh,
                 int use_winding, double* d_sign, double* d_conf);
 int run_combine(sdfgpu_ctx* ctx, const GridP& g, const double* d_dist, const double* d_sign, double* d_sdf);

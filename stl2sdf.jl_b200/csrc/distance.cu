@@ -645,7 +645,8 @@ int unb_setup(sdfgpu_ctx* ctx, const GridP& g, int use_learned, double* d_dist, 
 
 }  // namespace
 
-int run_distances(sdfgpu_ctx* ctx, const GridP& g, int mode, int use_learned, double* d_dist, double* d_xp) {
+int run_distances(sdfgpu_ctx* ctx, const GridP& g, int mode, int use_learned, double* d_dist, double* d_xp,
+                  const std::function<int()>& between) {
   cudaStream_t st = ctx->stream;
   if (mode == SDFGPU_MODE_UNBOUNDED) {
     UnbArgs A;
@@ -677,19 +678,21 @@ int run_distances(sdfgpu_ctx* ctx, const GridP& g, int mode, int use_learned, do
     }
     SDF_KERNEL(ctx);
     SDF_MARK(ctx, T_FOLD);
-    return 0;
+    return between ? between() : 0;
   }
 
   DistPlan P;
   if (!d_xp && !ctx->tune_tiles && near_applies(ctx, g, mode)) {
     SDF_TRY(near_prepare(ctx, g, mode, d_dist, P));
     SDF_MARK(ctx, T_TILES);
+    if (between) SDF_TRY(between());
     SDF_TRY(near_run(ctx, P));
     SDF_MARK(ctx, T_FOLD);
     return 0;
   }
   SDF_TRY(dist_prepare(ctx, g, mode, d_dist, d_xp, P));
   SDF_MARK(ctx, T_TILES);
+  if (between) SDF_TRY(between());
   SDF_TRY(dist_fold(ctx, P));
   SDF_MARK(ctx, T_FOLD);
   if (P.knn) SDF_TRY(dist_knn(ctx, P, st, true));

@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_prep(const double* __restrict_
                                                        TriRec64* __restrict__ rec, double4* __restrict__ cent,
                                                        float4* __restrict__ v32, float4* __restrict__ c32,
                                                        float4* __restrict__ box32, float4* __restrict__ tri32,
-                                                       unsigned long long* rho_ord, int64_t* counters) {
+                                                       unsigned long long* bad, unsigned long long* rho_ord) {
   __shared__ double s_rec[kPrepThreads / 32][32 * kRecStride];
   const int lane = threadIdx.x & 31;
   double* stage = s_rec[threadIdx.x >> 5];
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_prep(const double* __restrict_
       for (int k = 0; k < 3; ++k) {
         int64_t vi = IEN[3 * el + k];
         if (vi < 1 || vi > nnp) {
-          count_add(counters, C_ERR_INDEX, 1);
+          atomicOr(bad, 2ULL);
           vi = 1;
         }
         vi -= 1;
@@ -725,25 +725,24 @@ int mesh_upload_and_build(sdfgpu_ctx* ctx, const double* X, int64_t nnp, const i
   float4* tri32;
   SDF_TRY(scratch_t(ctx, "tri32", (size_t)nel * 5, &tri32));
 
-  // box, non-finite flag; rho, rho of the unfit triangles, their number (0 is below the encoding of every
-  // non-negative double)
+  // box; flags: 1 a vertex not finite, 2 an index out of range; rho, rho of the unfit triangles, their
+  // number (0 is below the encoding of every non-negative double)
   unsigned long long init[10] = {~0ULL, ~0ULL, ~0ULL};
-  SDF_CUDA(ctx, cudaMemsetAsync(ctx->d_counters, 0, sizeof(int64_t) * C_NUM, st));
   SDF_CUDA(ctx, cudaMemcpyAsync(bb, init, sizeof(init), cudaMemcpyHostToDevice, st));
   k_vertex_bbox<<<grid_for(nnp, 256, 148 * 4), 256, 0, st>>>(dX, nnp, bb);
   SDF_KERNEL(ctx);
   k_prep<<<grid_for(nel, kPrepThreads), kPrepThreads, 0, st>>>(dX, nnp, dIEN, nel, bb, rec, cent, v32, c32, box32, tri32,
-                                                              bb + 7, ctx->d_counters);
+                                                              bb + 6, bb + 7);
   SDF_KERNEL(ctx);
   SDF_CUDA(ctx, cudaEventRecord(ctx->ev_mesh, st));
-  unsigned long long hbb[10];
-  int64_t hcnt[C_NUM];
-  SDF_CUDA(ctx, cudaMemcpyAsync(hbb, bb, sizeof(hbb), cudaMemcpyDeviceToHost, st));
-  SDF_CUDA(ctx, cudaMemcpyAsync(hcnt, ctx->d_counters, sizeof(hcnt), cudaMemcpyDeviceToHost, st));
+  static_assert(S_COUNTERS - S_MESH >= sizeof(init) / sizeof(init[0]), "the mesh's scalars have page-locked slots");
+  SDF_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + S_MESH, bb, sizeof(init), cudaMemcpyDeviceToHost, st));
   SDF_CUDA(ctx, cudaEventRecord(ctx->ev[5], st));
   SDF_CUDA(ctx, cudaStreamSynchronize(st));
-  if (hbb[6]) return fail(ctx, SDFGPU_ERR_INVALID_ARGUMENT, "mesh vertices must be finite");
-  if (hcnt[C_ERR_INDEX]) return fail(ctx, SDFGPU_ERR_INVALID_ARGUMENT, "IEN holds an index outside 1..nnp");
+  unsigned long long hbb[10];
+  std::memcpy(hbb, ctx->h_scalars + S_MESH, sizeof(hbb));
+  if (hbb[6] & 1) return fail(ctx, SDFGPU_ERR_INVALID_ARGUMENT, "mesh vertices must be finite");
+  if (hbb[6] & 2) return fail(ctx, SDFGPU_ERR_INVALID_ARGUMENT, "IEN holds an index outside 1..nnp");
 
   MeshDev& M = ctx->mesh;
   M.nnp = nnp;

@@ -600,28 +600,30 @@ int near_prepare(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, Dist
     A.tn[a] = (g.n[a] >> kTileShift) + 1;
     tiles *= A.tn[a];
   }
-  int32_t* counts;  // near nodes, hard nodes, hard nodes without a bound
+  int32_t* counts;  // near nodes, hard nodes, hard nodes without a bound; the pool's length
   SDF_TRY(scratch_t(ctx, "near_m2", (size_t)g.ngp, &A.m2));
   SDF_TRY(scratch_t(ctx, "near_map", (size_t)g.ngp, &A.map));
   SDF_TRY(scratch_t(ctx, "near_node", (size_t)g.ngp, &A.node));
-  SDF_TRY(scratch_t(ctx, "near_counts", 3, &counts));
+  SDF_TRY(scratch_t(ctx, "near_counts", 6, &counts));
   SDF_TRY(scratch_t(ctx, "near_tflag", (size_t)tiles * 2, &A.tflag));
   SDF_TRY(scratch_t(ctx, "near_mask", (size_t)M.nel, &A.mask));
   A.tcand = A.tflag + tiles;
   A.near_n = counts;
   A.hard_n = counts + 1;
   A.unbounded_n = counts + 2;
+  A.pool_n = reinterpret_cast<unsigned long long*>(counts + 4);
   SDF_CUDA(ctx, cudaMemsetAsync(A.m2, 0x7f, sizeof(uint32_t) * g.ngp, st));  // 3.39e38
-  SDF_CUDA(ctx, cudaMemsetAsync(counts, 0, 3 * sizeof(int32_t), st));
+  SDF_CUDA(ctx, cudaMemsetAsync(counts, 0, 6 * sizeof(int32_t), st));
   SDF_CUDA(ctx, cudaMemsetAsync(A.tflag, 0, (size_t)tiles * 2, st));
   const unsigned gt = grid_for(M.nel, 128, 148 * 64);
   k_near_scatter<false><<<gt, 128, 0, st>>>(A);
   SDF_KERNEL(ctx);
   k_near_nodes<<<grid_for(cdiv(g.ngp, kNodes), kNodesThreads, 148 * 16), kNodesThreads, 0, st>>>(A);
   SDF_KERNEL(ctx);
-  int32_t n_near = 0;
-  SDF_CUDA(ctx, cudaMemcpyAsync(&n_near, A.near_n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+  SDF_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + S_NEAR, A.near_n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   SDF_CUDA(ctx, cudaStreamSynchronize(st));
+  int32_t n_near;
+  std::memcpy(&n_near, ctx->h_scalars + S_NEAR, sizeof(n_near));
   SDF_TRY(scratch_t(ctx, "near_cnt", (size_t)n_near, &A.cnt));
   SDF_TRY(scratch_t(ctx, "near_slot", (size_t)n_near * kSlots, &A.slot));
   SDF_TRY(scratch_t(ctx, "near_hidx", (size_t)n_near, &A.hidx));
@@ -630,7 +632,6 @@ int near_prepare(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, Dist
   SDF_TRY(scratch_t(ctx, "near_hcnt", (size_t)n_near, &A.hcnt));
   SDF_TRY(scratch_t(ctx, "near_hoff", (size_t)n_near, &A.hoff));
   SDF_TRY(scratch_t(ctx, "near_pool", (size_t)kHardPool, &A.pool));
-  SDF_TRY(scratch_t(ctx, "near_pool_n", 1, &A.pool_n));
   std::memcpy(Pl.fold, &A, sizeof(A));
   Pl.g = g;
   Pl.nonempty = n_near;
@@ -651,7 +652,6 @@ int near_run(sdfgpu_ctx* ctx, const DistPlan& Pl) {
   k_near_resolve<<<grid_for(n, 128, 148 * 32), 128, 0, st>>>(A);
   SDF_KERNEL(ctx);
   // these return at once when no node is hard
-  SDF_CUDA(ctx, cudaMemsetAsync(A.pool_n, 0, sizeof(unsigned long long), st));
   k_hard_collect<0><<<gt, 128, 0, st>>>(A);
   SDF_KERNEL(ctx);
   k_hard_collect<1><<<gt, 128, 0, st>>>(A);

@@ -1041,12 +1041,9 @@ int sign_begin(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P) {
   return 0;
 }
 
-int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int max_rays, double conf_thresh,
-                int use_winding, double* d_sign, double* d_conf) {
+int sign_vote(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int max_rays, double conf_thresh,
+              int use_winding, double* d_sign, double* d_conf) {
   cudaStream_t st = ctx->sign_stream;
-  const MeshDev& M = ctx->mesh;
-  const int64_t nel = M.nel;
-  const TriRec64* rec = buf<TriRec64>(ctx, "rec");
   const int64_t Rx = P.Rx, Ry = P.Ry, nrows = P.nrows;
   int32_t *row_cnt = P.row_cnt, *row_off = P.row_off;
   SDF_CUDA(ctx, cudaEventSynchronize(ctx->ev_rows));
@@ -1095,12 +1092,10 @@ int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int 
   k_row_masks<<<(unsigned)cdiv(K.mbase[3], 128), 128, 0, st>>>(K);
   SDF_KERNEL(ctx);
 
-  int32_t *und, *wind;
-  uint64_t *und_have, *und_par;
-  SDF_TRY(scratch_t(ctx, "und_list", (size_t)g.ngp, &und));
-  SDF_TRY(scratch_t(ctx, "und_have", (size_t)g.ngp, &und_have));
-  SDF_TRY(scratch_t(ctx, "und_par", (size_t)g.ngp, &und_par));
-  SDF_TRY(scratch_t(ctx, "wind_list", (size_t)g.ngp, &wind));
+  SDF_TRY(scratch_t(ctx, "und_list", (size_t)g.ngp, &P.und));
+  SDF_TRY(scratch_t(ctx, "und_have", (size_t)g.ngp, &P.und_have));
+  SDF_TRY(scratch_t(ctx, "und_par", (size_t)g.ngp, &P.und_par));
+  SDF_TRY(scratch_t(ctx, "wind_list", (size_t)g.ngp, &P.wind));
   VoteArgs V;
   V.g = g;
   for (int a = 0; a < 3; ++a) V.mask[a] = K.mask + K.mbase[a];
@@ -1115,17 +1110,28 @@ int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int 
   V.use_winding = use_winding;
   V.sign = d_sign;
   V.conf = d_conf;
-  V.und_list = und;
-  V.und_have = und_have;
-  V.und_par = und_par;
-  V.wind_list = wind;
+  V.und_list = P.und;
+  V.und_have = P.und_have;
+  V.und_par = P.und_par;
+  V.wind_list = P.wind;
   V.counters = ctx->d_counters;
   const int64_t vote_warps = (int64_t)V.tiles[0] * V.tiles[1] * V.tiles[2];
   k_vote<<<(unsigned)cdiv(vote_warps, 8), 256, 0, st>>>(V);
   SDF_KERNEL(ctx);
   SDF_MARK_ON(ctx, T_PARITY, st);
-  SDF_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + S_UNDECIDED, ctx->d_counters + C_LIST_UNDECIDED, sizeof(int64_t),
+  SDF_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + S_UNDECIDED, ctx->d_counters + C_LIST_UNDECIDED, 2 * sizeof(int64_t),
                                 cudaMemcpyDeviceToHost, st));
+  return 0;
+}
+
+int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int max_rays, double conf_thresh,
+                int use_winding, double* d_sign, double* d_conf) {
+  cudaStream_t st = ctx->sign_stream;
+  const MeshDev& M = ctx->mesh;
+  const int64_t nel = M.nel;
+  const TriRec64* rec = buf<TriRec64>(ctx, "rec");
+  int32_t *und = P.und, *wind = P.wind;
+  uint64_t *und_have = P.und_have, *und_par = P.und_par;
   SDF_CUDA(ctx, cudaStreamSynchronize(st));
   const int64_t nund = ctx->h_scalars[S_UNDECIDED];
   if (nund > 0) {
@@ -1195,9 +1201,11 @@ int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int 
     SDF_KERNEL(ctx);
   }
   if (use_winding) {
-    SDF_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + S_WINDING, ctx->d_counters + C_LIST_WINDING, sizeof(int64_t),
-                                  cudaMemcpyDeviceToHost, st));
-    SDF_CUDA(ctx, cudaStreamSynchronize(st));
+    if (nund > 0) {  // their votes may have added to the list
+      SDF_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + S_WINDING, ctx->d_counters + C_LIST_WINDING, sizeof(int64_t),
+                                    cudaMemcpyDeviceToHost, st));
+      SDF_CUDA(ctx, cudaStreamSynchronize(st));
+    }
     const int64_t nw = ctx->h_scalars[S_WINDING];
     if (nw > 0) {
       const int nchunks = (int)cdiv(nel, kWindChunk);
