@@ -23,6 +23,7 @@
 //   * Nodes left with confidence < threshold sum the winding number over all triangles, one CTA
 //     per node with a fixed-order block reduction.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <type_traits>
 
@@ -31,13 +32,14 @@
 namespace sdfgpu {
 
 __constant__ double c_dirs[36 * 3];
+__constant__ float c_dirs32[36 * 3];  // the same, rounded
 
 namespace {
 
 constexpr double kEps = 1e-8;  // check_ray_inside_bvh default (:118), passed to MT (:132)
 constexpr int kRowCap = 64;    // hits per row a node sorts in registers/local memory
 constexpr int kRayCap = 256;   // hits per generic ray
-constexpr int64_t kAllPairsNodes = 64;  // undecided nodes whose rays may test every triangle
+constexpr int kAllPairsNodes = 24;  // undecided nodes whose rays test every triangle
 constexpr int kStack = 64;
 
 // A row hit: the Möller–Trumbore constants of one triangle for one grid row, from which each node
@@ -834,49 +836,65 @@ __global__ void __launch_bounds__(128) k_rays(RayArgs A, int round) {
 // The rays of a few undecided nodes against every triangle, without the LBVH (which then need not be
 // built): one thread per triangle, all requested rays.  Most pairs end at a distance test of the
 // triangle's centroid from the ray's line; the rest take the tests of ray_parity, so the hits are the same.
-// Bound: that test, about 15 FP32 instructions a pair.
-constexpr int kAllRays = 128;  // requests held in shared memory at a time
-__global__ void __launch_bounds__(128) k_rays_all(RayArgs A, const float4* __restrict__ c32, int64_t nel, float reach,
-                                                  int32_t* __restrict__ hit_n, double* __restrict__ hit_t) {
-  __shared__ float4 s_o[kAllRays], s_d[kAllRays];  // origin (mesh-local) and direction, .w of the first: node index
+// The node's terms are formed once for its rays, whose directions are constant operands.  Bound: the test's
+// 7 instructions a pair; 24 rays of one node against 1.4M and 5.8M triangles 45 and 112 us (B200),
+// against 61 and 240 with origins and directions read from shared memory a pair.
+constexpr int kRayGroup = 6;
+__global__ void __launch_bounds__(128) k_rays_all(const __grid_constant__ RayArgs A, int nund, const float4* __restrict__ c32,
+                                                  int64_t nel, float reach, float lim2, int32_t* __restrict__ hit_n,
+                                                  double* __restrict__ hit_t) {
+  __shared__ float4 s_o[kAllPairsNodes];  // origin (mesh-local), .w: node index
+  __shared__ unsigned long long s_want[kAllPairsNodes];
   const GridP& g = A.g;
-  const int count = (int)A.rq_cnt[0];
   int64_t band = 0;
-  for (int base = 0; base < count; base += kAllRays) {
-    const int m = min(kAllRays, count - base);
-    __syncthreads();
-    for (int t = threadIdx.x; t < m; t += blockDim.x) {
-      const int64_t lin = A.list[A.req_node[base + t]];
-      const int64_t i = lin % g.n[0], j = (lin / g.n[0]) % g.n[1], k = lin / (g.n[0] * g.n[1]);
-      const d3 p = gnode(g, i, j, k);
-      const double* dir = c_dirs + 3 * (A.req_ray[base + t] - 1);
-      s_o[t] = make_float4((float)(p.x - g.center[0]), (float)(p.y - g.center[1]), (float)(p.z - g.center[2]),
-                           __int_as_float((int)lin));
-      s_d[t] = make_float4((float)dir[0], (float)dir[1], (float)dir[2], __int_as_float(A.req_ray[base + t] - 1));
-    }
-    __syncthreads();
-    for (int64_t el = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; el < nel; el += (int64_t)gridDim.x * blockDim.x) {
-      const float4 c = c32[el];
-      for (int t = 0; t < m; ++t) {
-        const float4 o = s_o[t], d = s_d[t];
-        // distance of the centroid from the line: |w - (w . d) d|, d a unit vector
-        const float wx = c.x - o.x, wy = c.y - o.y, wz = c.z - o.z;
-        const float s = fmaf(wx, d.x, fmaf(wy, d.y, wz * d.z));
-        const float qx = fmaf(-s, d.x, wx), qy = fmaf(-s, d.y, wy), qz = fmaf(-s, d.z, wz);
-        if (fmaf(qx, qx, fmaf(qy, qy, qz * qz)) > reach * reach || s < -reach) continue;
+  for (int q = threadIdx.x; q < nund; q += blockDim.x) {
+    const int64_t lin = A.list[q];
+    const int64_t i = lin % g.n[0], j = (lin / g.n[0]) % g.n[1], k = lin / (g.n[0] * g.n[1]);
+    const d3 p = gnode(g, i, j, k);
+    s_o[q] = make_float4((float)(p.x - g.center[0]), (float)(p.y - g.center[1]), (float)(p.z - g.center[2]),
+                         __int_as_float((int)lin));
+    s_want[q] = 0ULL;
+  }
+  __syncthreads();
+  const int count = (int)A.rq_cnt[0];
+  for (int t = threadIdx.x; t < count; t += blockDim.x)
+    atomicOr(&s_want[A.req_node[t]], 1ULL << (A.req_ray[t] - 1));
+  __syncthreads();
+  for (int64_t el = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; el < nel; el += (int64_t)gridDim.x * blockDim.x) {
+    const float4 c = c32[el];
+    for (int q = 0; q < nund; ++q) {
+      const unsigned long long want = s_want[q];
+      if (!want) continue;
+      const float4 o = s_o[q];
+      // squared distance of the centroid from the line: |w|^2 - (w . d)^2, d a unit vector
+      const float wx = c.x - o.x, wy = c.y - o.y, wz = c.z - o.z, ww = fmaf(wx, wx, fmaf(wy, wy, fmaf(wz, wz, -lim2)));
+      unsigned long long pass = 0ULL;
+#pragma unroll
+      for (int r0 = 0; r0 < 36; r0 += kRayGroup) {
+        constexpr unsigned kGroup = (1u << kRayGroup) - 1u;
+        if (!((unsigned)(want >> r0) & kGroup)) continue;
+        unsigned in = 0u;
+#pragma unroll
+        for (int r = 0; r < kRayGroup; ++r) {
+          const float s = fmaf(wx, c_dirs32[3 * (r0 + r)], fmaf(wy, c_dirs32[3 * (r0 + r) + 1], wz * c_dirs32[3 * (r0 + r) + 2]));
+          in |= (unsigned)(!(fmaf(-s, s, ww) > 0.f) && !(s < -reach)) << r;
+        }
+        pass |= (unsigned long long)in << r0;
+      }
+      for (pass &= want; pass; pass &= pass - 1ULL) {
+        const int ray = __ffsll((long long)pass) - 1;
         const int64_t lin = __float_as_int(o.w);
         const int64_t i = lin % g.n[0], j = (lin / g.n[0]) % g.n[1], k = lin / (g.n[0] * g.n[1]);
         const d3 p = gnode(g, i, j, k);
-        const double* dir = c_dirs + 3 * __float_as_int(d.w);
-        const d3 dd3 = {dir[0], dir[1], dir[2]};
+        const d3 dir = {c_dirs[3 * ray], c_dirs[3 * ray + 1], c_dirs[3 * ray + 2]};
         const TriRec64& r = A.rec[el];
-        const int dec = mt32(p, dd3, rec_v(r, 0), rec_v(r, 1), rec_v(r, 2));
+        const int dec = mt32(p, dir, rec_v(r, 0), rec_v(r, 1), rec_v(r, 2));
         if (dec == 0) continue;
         if (dec == 2) ++band;
         double tt;
-        if (mt64(p, dd3, rec_v(r, 0), rec_v(r, 1), rec_v(r, 2), kEps, tt)) {
-          const int q = atomicAdd(hit_n + base + t, 1);
-          if (q < kRayCap) hit_t[(int64_t)(base + t) * kRayCap + q] = tt;
+        if (mt64(p, dir, rec_v(r, 0), rec_v(r, 1), rec_v(r, 2), kEps, tt)) {
+          const int h = atomicAdd(hit_n + q * 36 + ray, 1);
+          if (h < kRayCap) hit_t[(int64_t)(q * 36 + ray) * kRayCap + h] = tt;
         }
       }
     }
@@ -889,12 +907,12 @@ __global__ void __launch_bounds__(128) k_rays_all(RayArgs A, const float4* __res
 __global__ void k_rays_parity(RayArgs A, const int32_t* __restrict__ hit_n, double* __restrict__ hit_t) {
   const int count = (int)A.rq_cnt[0];
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
-    const int n = hit_n[t];
+    const int at = A.req_node[t] * 36 + A.req_ray[t] - 1, n = hit_n[at];
     int parity = 0;
     if (n > kRayCap) {
       count_add(A.counters, C_ERR_CAPACITY, 1);
     } else if (n > 0) {
-      double* ts = hit_t + (int64_t)t * kRayCap;
+      double* ts = hit_t + (int64_t)at * kRayCap;
       for (int a = 1; a < n; ++a) {
         const double v = ts[a];
         int b = a;
@@ -976,6 +994,9 @@ __global__ void k_combine(int64_t n, const double* __restrict__ dist, const doub
 
 int upload_directions(sdfgpu_ctx* ctx, const double* dirs) {
   SDF_CUDA(ctx, cudaMemcpyToSymbolAsync(c_dirs, dirs, sizeof(double) * 108, 0, cudaMemcpyHostToDevice, ctx->stream));
+  float d32[108];
+  for (int q = 0; q < 108; ++q) d32[q] = (float)dirs[q];
+  SDF_CUDA(ctx, cudaMemcpyToSymbolAsync(c_dirs32, d32, sizeof(d32), 0, cudaMemcpyHostToDevice, ctx->stream));
   return 0;
 }
 
@@ -1147,9 +1168,11 @@ int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int 
     SDF_TRY(scratch_t(ctx, "rq_cnt", (size_t)kRounds + 1, &rq_cnt));
     SDF_CUDA(ctx, cudaMemsetAsync(done, 0, (size_t)nund, st));
     SDF_CUDA(ctx, cudaMemsetAsync(rq_cnt, 0, sizeof(int64_t) * (kRounds + 1), st));
-    // Few (ray, triangle) pairs: all of them, at about 0.5 ps each (24 rays x 1.4M triangles in 20 us)
-    // instead of walks of the LBVH whose latency (0.28 ms there) and build (0.6 ms) they would pay for.
-    const bool all_pairs = nund <= kAllPairsNodes && (double)nund * 30.0 * (double)nel <= 4.0e8;
+    // Few nodes: their rays against all triangles, about 19 ps a node and triangle (0.11 ms for one node and
+    // 5.8M triangles), instead of walks of the LBVH, which take 0.28 ms by their latency and the build that
+    // nothing else in such a call needs (0.47 ms for 1.4M triangles, 0.33 ns a triangle): the sides meet at
+    // about 20 nodes for many triangles, and at more for few.
+    const bool all_pairs = nund <= kAllPairsNodes;
     if (!all_pairs) {
       SDF_TRY(ensure_tree(ctx, false));
       SDF_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_bvh, 0));  // the adaptive rays walk the LBVH
@@ -1188,8 +1211,11 @@ int sign_finish(sdfgpu_ctx* ctx, const GridP& g, SignPlan& P, int min_rays, int 
         SDF_TRY(scratch_t(ctx, "ray_hit_n", (size_t)nund * 36, &hit_n));
         SDF_TRY(scratch_t(ctx, "ray_hit_t", (size_t)nund * 36 * kRayCap, &hit_t));
         SDF_CUDA(ctx, cudaMemsetAsync(hit_n, 0, sizeof(int32_t) * nund * 36, st));
-        const float reach = (float)(M.rho_max * (1.0 + 1e-5) + 4e-6 * g.E);
-        k_rays_all<<<grid_for(nel, 128, 148 * 16), 128, 0, st>>>(R, buf<float4>(ctx, "c32"), nel, reach, hit_n, hit_t);
+        // a hit triangle's centroid is within rho of the line: with the errors of the FP32 coordinates in
+        // it (4e-6 E), and of |w|^2 - (w . d)^2 (|w| at most 3.5 E: below 1e-5 E^2)
+        const double rho = M.rho_max * (1.0 + 1e-5) + 4e-6 * g.E, lim2 = rho * rho + 1.5e-5 * g.E * g.E;
+        k_rays_all<<<grid_for(nel, 128, 148 * 16), 128, 0, st>>>(R, (int)nund, buf<float4>(ctx, "c32"), nel,
+                                                                 (float)std::sqrt(lim2), (float)lim2, hit_n, hit_t);
         SDF_KERNEL(ctx);
         k_rays_parity<<<grid_for(nund * 36, 64), 64, 0, st>>>(R, hit_n, hit_t);
       } else {
