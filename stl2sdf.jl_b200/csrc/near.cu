@@ -107,10 +107,11 @@ __device__ __forceinline__ float node32(const NearArgs& A, int a, float x, float
 // within the band of the node's minimum at that time; it only falls, so the second needs no others: about
 // two pairs a triangle instead of thirty.  Triangles of more than 64 nodes go through 64 at a time, both
 // times.  Bound: instruction issue, about 70 a pair.  Both scatters, 1.4M triangles of which a third of a
-// node is near, and 5.8M: 0.43 -> 0.30 and 1.9 -> 1.22 ms (B200) against all
+// node is near, and 5.8M: 0.43 -> 0.27 and 1.9 -> 1.11 ms (B200) against all
 // nodes of the box in both.
+// 64 registers (8 blocks an SM) for the latency of the triangles' reads: 10% below the compiler's 80.
 template <bool kFill>
-__global__ void __launch_bounds__(128) k_near_scatter(const __grid_constant__ NearArgs A) {
+__global__ void __launch_bounds__(128, 8) k_near_scatter(const __grid_constant__ NearArgs A) {
   const GridP& g = A.g;
   for (int64_t el = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; el < A.nel; el += (int64_t)gridDim.x * blockDim.x) {
     uint64_t kept = 0;
@@ -269,7 +270,7 @@ __device__ __noinline__ void step_values(const TriRec64* __restrict__ rec, int t
 }
 
 // One thread per near node: the result from its ties, or a place in the hard list.
-__global__ void __launch_bounds__(128) k_near_resolve(const __grid_constant__ NearArgs A) {
+__global__ void __launch_bounds__(128, 6) k_near_resolve(const __grid_constant__ NearArgs A) {
   const GridP& g = A.g;
   const int n_near = *A.near_n;
   const double tol = 1e-9 * (double)A.E, tol2 = tol * tol;
