@@ -453,6 +453,8 @@ int sdfgpu_sdf_batch_ex(sdfgpu_ctx* ctx, sdfgpu_batch_item* items, int64_t count
     sdfgpu_ctx* w = nullptr;
     if (create_context(&o, &w, false) != SDFGPU_OK)
       return fail(ctx, SDFGPU_ERR_CUDA, std::string("batch worker: ") + sdfgpu_last_error(nullptr));
+    if (!ctx->worker_hints) ctx->worker_hints = std::make_shared<ScratchHints>();
+    w->hints = ctx->worker_hints;
     ctx->workers.push_back(w);
   }
   BatchJob J;

@@ -6,6 +6,8 @@
 
 #include <functional>
 #include <map>
+#include <memory>
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -105,6 +107,12 @@ struct DevBuf {
   size_t cap = 0;
 };
 
+// The largest size that any worker of a batch has asked for, per scratch buffer (see scratch()).
+struct ScratchHints {
+  std::mutex mu;
+  std::unordered_map<std::string, size_t> bytes;
+};
+
 }  // namespace sdfgpu
 
 struct sdfgpu_ctx {
@@ -134,6 +142,7 @@ struct sdfgpu_ctx {
   int64_t* h_scalars = nullptr;          // page-locked host slots for sizing reads (see Scalar)
   std::string ns;                        // prefix of every scratch-buffer name (batch items keep their own)
   std::vector<sdfgpu_ctx*> workers;      // batch workers (batch.cu), created on first use
+  std::shared_ptr<sdfgpu::ScratchHints> hints, worker_hints;  // a worker's, and those of this context's workers
   std::map<int64_t, uint32_t> tuned;     // autotuner: (size class, mode) -> packed tile or brick (batch.cu)
 };
 
