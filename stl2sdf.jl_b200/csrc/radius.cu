@@ -118,18 +118,23 @@ __device__ __forceinline__ void acc_to_a(const float acc[8][4], uint32_t a[4][4]
 // ---- training (mma.sync m16n8k16, FP16 operands, FP32 accumulate) ------------------------------
 //
 // One step = k_train_step + k_train_reduce.  k_train_step: every CTA takes kTS samples of the
-// step's batch (4 warps x 32).  A warp runs the forward of its 32 samples as three 64-wide GEMM
+// step's batch (8 warps x 16).  A warp runs the forward of its 16 samples as three 64-wide GEMM
 // layers on the tensor cores (the inference kernel's fragments), the loss and dL/dy, then the
 // backward input gradients dZ3 -> dZ2 -> dZ1 as two more GEMMs (dH = dZ W, W read transposed from
 // shared memory), staging every activation and every dZ in shared memory as FP16.  Then each warp
-// forms a 16-row slice of every weight gradient dW = dZ^T H as GEMMs over the CTA's kTS samples,
+// forms half of a 16-row slice of every weight gradient dW = dZ^T H as GEMMs over the CTA's kTS samples,
 // and the CTA writes its partial gradient (and partial loss) to global memory.  k_train_reduce sums
 // the partials of all CTAs in a fixed order (deterministic), rescales, and applies Adam.
 //
 // dL/dy is carried scaled by kGyScale instead of 1/B so the FP16 dZ stay in range; the reduce
 // multiplies by 1 / (kGyScale B).  dZ beyond the FP16 range are clamped (only possible far from a
 // trained state; the gradient then stays finite).
+//
+// Bound: the latency of one CTA's chain (a step has too few samples to fill the GPU): loading the weights,
+// five GEMMs, and the gradients over the samples.  With eight warps instead of four, each chain link is half
+// as long: 24.9 -> 18.5 us a step (B200, 51 steps of the default training).
 constexpr int kTS = 128;                 // samples per CTA
+constexpr int kTrainThreads = 2 * kTS;
 constexpr float kGyScale = 1.f / 256.f;  // per-sample dL/dy scale inside the step
 constexpr int kLd1 = kIn + 8;            // shared-memory row strides in halves (padding against bank conflicts)
 constexpr int kLdH = kHid + 8;
@@ -147,8 +152,8 @@ struct TrainSmem {
   __half D1[kTS * kLdH];   // per sample: dZ1, dZ2, dZ3 (scaled by kGyScale)
   __half D2[kTS * kLdH];
   __half D3[kTS * kLdH];
-  float gw4[4][kHid];
-  float red[4][2];         // per warp: sum of dL/dy (b4) and of the loss terms
+  float gw4[kTrainThreads / 32][kHid];
+  float red[kTrainThreads / 32][2];         // per warp: sum of dL/dy (b4) and of the loss terms
 };
 
 __device__ __forceinline__ uint32_t pack_hh(__half lo, __half hi) {
@@ -206,15 +211,16 @@ __device__ __forceinline__ void mask_by(float acc[8][4], const __half* H, int r0
   }
 }
 
-// dW rows [16 w, 16 w + 16) of one layer: sum over the CTA's kTS samples of dZ[s][out] H[s][in]
-// (A = dZ^T, B = H), written to the CTA's partial at offW (row stride K).
+// dW rows [16 (w % 4), 16 (w % 4) + 16) and columns 8 NT (w / 4) to 8 NT (w / 4 + 1) of one layer: sum over
+// the CTA's kTS samples of dZ[s][out] H[s][in] (A = dZ^T, B = H), written to the CTA's partial at offW (row
+// stride K).
 template <int NT>
 __device__ __forceinline__ void wgrad_rows(const __half* D, const __half* H, int ldh, int K, int w, int g, int t,
                                            float* out) {
   float acc[NT][4];
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-  const int o = 16 * w + g;
+  const int o = 16 * (w & 3) + g, c0 = 8 * NT * (w >> 2);
 #pragma unroll 2
   for (int kk = 0; kk < kTS / 16; ++kk) {
     const int s0 = 16 * kk + 2 * t;
@@ -224,7 +230,7 @@ __device__ __forceinline__ void wgrad_rows(const __half* D, const __half* H, int
                            pack_hh(D[(s0 + 8) * kLdH + o + 8], D[(s0 + 9) * kLdH + o + 8])};
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-      const int n = 8 * nt + g;
+      const int n = c0 + 8 * nt + g;
       const uint32_t bf[2] = {pack_hh(H[s0 * ldh + n], H[(s0 + 1) * ldh + n]),
                               pack_hh(H[(s0 + 8) * ldh + n], H[(s0 + 9) * ldh + n])};
       mma16816(acc[nt], a, bf);
@@ -232,7 +238,7 @@ __device__ __forceinline__ void wgrad_rows(const __half* D, const __half* H, int
   }
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt) {
-    const int c = 8 * nt + 2 * t;
+    const int c = c0 + 8 * nt + 2 * t;
     out[o * K + c] = acc[nt][0];
     out[o * K + c + 1] = acc[nt][1];
     out[(o + 8) * K + c] = acc[nt][2];
@@ -243,15 +249,17 @@ __device__ __forceinline__ void wgrad_rows(const __half* D, const __half* H, int
 // Forward, loss and backward of kTS samples per CTA; writes the CTA's partial gradient.  Sample q of
 // the step is X[perm[off + q]] (perm may be NULL: X[q]); samples q >= B contribute nothing.
 // dhat_out / loss_out (nullable) receive the per-sample network output and loss term.
-__global__ void __launch_bounds__(128) k_train_step(const float* __restrict__ P, const float* __restrict__ X,
+__global__ void __launch_bounds__(kTrainThreads) k_train_step(const float* __restrict__ P, const float* __restrict__ X,
                                                     const float* __restrict__ T, const int32_t* __restrict__ perm,
                                                     int64_t off, int64_t B, float* __restrict__ partial,
                                                     float* __restrict__ dhat_out, float* __restrict__ loss_out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TrainSmem& S = *reinterpret_cast<TrainSmem*>(smem_raw);
-  for (int q = threadIdx.x; q < kHid * kIn; q += blockDim.x)
+#pragma unroll
+  for (int q = threadIdx.x; q < kHid * kIn; q += kTrainThreads)
     S.W1[(q / kIn) * kLd1 + q % kIn] = __float2half_rn(P[kOffW1 + q]);
-  for (int q = threadIdx.x; q < kHid * kHid; q += blockDim.x) {
+#pragma unroll
+  for (int q = threadIdx.x; q < kHid * kHid; q += kTrainThreads) {
     S.W2[(q / kHid) * kLdH + q % kHid] = __float2half_rn(P[kOffW2 + q]);
     S.W3[(q / kHid) * kLdH + q % kHid] = __float2half_rn(P[kOffW3 + q]);
   }
@@ -264,8 +272,8 @@ __global__ void __launch_bounds__(128) k_train_step(const float* __restrict__ P,
   if (threadIdx.x == 0) S.b4 = P[kOffB4];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int64_t cbase = (int64_t)blockIdx.x * kTS;
-  {  // features of this warp's 32 samples
-    const int sl = 32 * warp + lane;
+  if (threadIdx.x < kTS) {  // the samples' features
+    const int sl = threadIdx.x;
     const int64_t q = cbase + sl;
     float x0 = 0.f, x1 = 0.f, x2 = 0.f;
     if (q < B) {
@@ -282,9 +290,8 @@ __global__ void __launch_bounds__(128) k_train_step(const float* __restrict__ P,
 #pragma unroll
   for (int nt = 0; nt < 8; ++nt) gw4[nt][0] = gw4[nt][1] = 0.f;
   float gb4 = 0.f, lsum = 0.f;
-#pragma unroll 1
-  for (int mt = 0; mt < 2; ++mt) {
-    const int r0 = 32 * warp + 16 * mt + g;  // this thread's rows r0 and r0 + 8 (CTA-local samples)
+  {
+    const int r0 = 16 * warp + g;  // this thread's rows r0 and r0 + 8 (CTA-local samples)
     uint32_t a1[2][4];
 #pragma unroll
     for (int kc = 0; kc < 2; ++kc) {
@@ -385,22 +392,25 @@ __global__ void __launch_bounds__(128) k_train_step(const float* __restrict__ P,
   }
   __syncthreads();
   float* out = partial + (int64_t)blockIdx.x * kPart;
-  wgrad_rows<8>(S.D3, S.H2, kLdH, kHid, warp, g, t, out + kOffW3);
-  wgrad_rows<8>(S.D2, S.H1, kLdH, kHid, warp, g, t, out + kOffW2);
-  wgrad_rows<4>(S.D1, S.H0, kLd1, kIn, warp, g, t, out + kOffW1);
+  wgrad_rows<kHid / 16>(S.D3, S.H2, kLdH, kHid, warp, g, t, out + kOffW3);
+  wgrad_rows<kHid / 16>(S.D2, S.H1, kLdH, kHid, warp, g, t, out + kOffW2);
+  wgrad_rows<kIn / 16>(S.D1, S.H0, kLd1, kIn, warp, g, t, out + kOffW1);
   for (int q = threadIdx.x; q < 3 * kHid; q += blockDim.x) {  // bias gradients: sums of dZ over the samples
     const int layer = q / kHid, o = q % kHid;
     const __half* D = layer == 0 ? S.D1 : (layer == 1 ? S.D2 : S.D3);
     float s = 0.f;
+#pragma unroll 16
     for (int sl = 0; sl < kTS; ++sl) s += __half2float(D[sl * kLdH + o]);
     out[(layer == 0 ? kOffB1 : (layer == 1 ? kOffB2 : kOffB3)) + o] = s;
   }
-  if (threadIdx.x < kHid)
-    out[kOffW4 + threadIdx.x] =
-        S.gw4[0][threadIdx.x] + S.gw4[1][threadIdx.x] + S.gw4[2][threadIdx.x] + S.gw4[3][threadIdx.x];
+  auto warps = [](auto at) {  // the sum over the warps, pairwise
+    static_assert(kTrainThreads == 256, "eight warps");
+    return ((at(0) + at(1)) + (at(2) + at(3))) + ((at(4) + at(5)) + (at(6) + at(7)));
+  };
+  if (threadIdx.x < kHid) out[kOffW4 + threadIdx.x] = warps([&](int w) { return S.gw4[w][threadIdx.x]; });
   if (threadIdx.x == 0) {
-    out[kOffB4] = S.red[0][0] + S.red[1][0] + S.red[2][0] + S.red[3][0];
-    out[kParams] = S.red[0][1] + S.red[1][1] + S.red[2][1] + S.red[3][1];
+    out[kOffB4] = warps([&](int w) { return S.red[w][0]; });
+    out[kParams] = warps([&](int w) { return S.red[w][1]; });
   }
 }
 
@@ -575,7 +585,7 @@ int mlp_eval_host(sdfgpu_ctx* ctx, const float* params, const float* xn, const f
   SDF_CUDA(ctx, cudaMemcpyAsync(dX, xn, sizeof(float) * 3 * B, cudaMemcpyHostToDevice, st));
   if (target) SDF_CUDA(ctx, cudaMemcpyAsync(dT, target, sizeof(float) * B, cudaMemcpyHostToDevice, st));
   SDF_TRY(train_smem_attr(ctx));
-  k_train_step<<<nparts, 128, sizeof(TrainSmem), st>>>(dP, dX, dT, nullptr, 0, B, part, YH, nullptr);
+  k_train_step<<<nparts, kTrainThreads, sizeof(TrainSmem), st>>>(dP, dX, dT, nullptr, 0, B, part, YH, nullptr);
   SDF_KERNEL(ctx);
   k_train_reduce<<<(kPart + 255) / 256, 256, 0, st>>>(part, nparts, B, dP, nullptr, nullptr, 0, 0.f, 0.f, 0.f, G, dl);
   SDF_KERNEL(ctx);
@@ -653,7 +663,7 @@ int train_radius(sdfgpu_ctx* ctx, int coarse_n, int steps, int batch, float lr, 
   float b1t = 1.f, b2t = 1.f;
   for (int it = 0; it < steps; ++it) {
     const int64_t off = (it % per_epoch) * B;
-    k_train_step<<<nparts, 128, sizeof(TrainSmem), st>>>(P, X, T, dperm, off, B, part, nullptr, nullptr);
+    k_train_step<<<nparts, kTrainThreads, sizeof(TrainSmem), st>>>(P, X, T, dperm, off, B, part, nullptr, nullptr);
     SDF_KERNEL(ctx);
     b1t *= 0.9f;
     b2t *= 0.999f;
@@ -663,7 +673,7 @@ int train_radius(sdfgpu_ctx* ctx, int coarse_n, int steps, int batch, float lr, 
     SDF_KERNEL(ctx);
   }
   // final loss over the first batch of the shuffle
-  k_train_step<<<nparts, 128, sizeof(TrainSmem), st>>>(P, X, T, dperm, 0, B, part, nullptr, nullptr);
+  k_train_step<<<nparts, kTrainThreads, sizeof(TrainSmem), st>>>(P, X, T, dperm, 0, B, part, nullptr, nullptr);
   SDF_KERNEL(ctx);
   k_train_reduce<<<(kPart + 255) / 256, 256, 0, st>>>(part, nparts, B, P, nullptr, nullptr, 0, 0.f, 0.f, 0.f, nullptr,
                                                        dl);
