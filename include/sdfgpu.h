@@ -109,11 +109,11 @@ typedef struct sdfgpu_stats {
                                      build runs beside the next call's distance stage */
   int64_t launches;               /* kernels of this library launched by the last call (CUB excluded) */
   int64_t mesh_launches;          /* same, for the last set_mesh */
-  double ms_tiles;                /* (tile, triangle) pair build + sort */
-  double ms_fold;                 /* tile fold kernel (the distance hot loop) */
-  double ms_rows;                 /* axis-row hit lists (count, fill, sort) */
-  double ms_parity;               /* the three axis-parity kernels */
-  double ms_vote;                 /* vote + adaptive rays + winding */
+  double ms_tiles;                /* nearest distances and near nodes of the scatter, or (tile, triangle) pair build + sort */
+  double ms_fold;                 /* the near nodes' results, the tile fold kernel or the unbounded search */
+  double ms_rows;                 /* axis-row hit lists (count, fill) and their flags */
+  double ms_parity;               /* the rows' parity masks and the vote */
+  double ms_vote;                 /* adaptive rays + winding */
   int64_t certified_nodes;        /* learned radius: nodes whose bounded search certified the result */
   double radius_loss;             /* final training loss of the radius network */
   int64_t bvh_visits;             /* LBVH nodes opened by the unbounded search (one per warp and node) */

@@ -48,7 +48,6 @@ enum Counter : int {
   C_UNB_FALLBACK,
   C_ERR_CAPACITY,   // per-thread buffer overflow
   C_ERR_STACK,      // traversal stack overflow
-  C_ERR_INDEX,      // mesh index out of range
   C_LIST_UNDECIDED, // length of the undecided-node list
   C_LIST_WINDING,   // length of the winding list
   C_CERTIFIED,      // learned radius: nodes certified by the bounded search

@@ -21,7 +21,8 @@
 //
 // Work: the (triangle, node) pairs of the triangles' boxes grown by h -- about 27 a triangle where
 // triangles are small against h -- against the 64 nodes of every tile each triangle's 2.5 h ball reaches.
-// Whole field calls on a B200, tile fold -> scatter: 16.8M nodes, 1.4M triangles, reference rule 7.25 ->
+// Whole field calls on a B200, tile fold -> scatter with the other stages alike (all nodes of the boxes in both
+// scatters; the kernels' comments have what the masks gave): 16.8M nodes, 1.4M triangles, reference rule 7.25 ->
 // 3.61 ms; 33M nodes, 5.8M triangles, true minimum 25.6 -> 16.3 ms; 590k nodes, 131k triangles 1.33 ->
 // 0.77 ms; level at 149k nodes and 5k triangles (0.52 ms, launches).
 #include <algorithm>
