@@ -213,7 +213,8 @@ class Context:
         return int(s.value or 0)
 
     def set_mesh(self, X, IEN, key=None):
-        """X: (nnp, 3) float64; IEN: (nel, 3) int64 1-based (vertex-major = 3 x n column-major)."""
+        """X: (nnp, 3) float64; IEN: (nel, 3) int64 1-based (vertex-major = 3 x n column-major).
+        key: returns at once when it is the resident mesh's."""
         if key is not None and key == self._mesh_key:
             return
         X = np.ascontiguousarray(X, np.float64).reshape(-1, 3)
