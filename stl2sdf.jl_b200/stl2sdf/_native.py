@@ -219,12 +219,13 @@ class Context:
             return
         X = np.ascontiguousarray(X, np.float64).reshape(-1, 3)
         IEN = np.ascontiguousarray(IEN, np.int64).reshape(-1, 3)
+        self._mesh_key = None  # a refused mesh leaves the context without one
         self._check(lib().sdfgpu_set_mesh(self._p, _d(X), X.shape[0], _i(IEN), IEN.shape[0]))
         self._mesh_key = key
 
     def set_mesh_device(self, x_ptr: int, nnp: int, ien_ptr: int, nel: int):
-        self._check(lib().sdfgpu_set_mesh_device(self._p, ctypes.c_void_p(x_ptr), nnp, ctypes.c_void_p(ien_ptr), nel))
         self._mesh_key = None
+        self._check(lib().sdfgpu_set_mesh_device(self._p, ctypes.c_void_p(x_ptr), nnp, ctypes.c_void_p(ien_ptr), nel))
 
     def distances(self, origin, h, N, mode=MODE_REF_RULE, want_xp=False, learned=False, out=None):
         N = np.ascontiguousarray(N, np.int64)

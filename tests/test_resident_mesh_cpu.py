@@ -14,8 +14,14 @@ from stl2sdf import MeshGrid, _native
 class Recorder:
     def __init__(self):
         self.meshes = []
+        self.refuse = False
+
+    def sdfgpu_set_mesh_device(self, ctx, X, nnp, IEN, nel):
+        return 1
 
     def sdfgpu_set_mesh(self, ctx, X, nnp, IEN, nel):
+        if self.refuse:
+            return 1
         self.meshes.append(np.ctypeslib.as_array(ctypes.cast(X, ctypes.POINTER(ctypes.c_double)), (nnp, 3)).copy())
         return 0
 
@@ -43,3 +49,19 @@ def test_a_mesh_of_the_same_size_at_a_freed_address_is_a_new_mesh(recorded):
             ctx.set_mesh(mesh.vertex_rows(), mesh.triangle_rows(), key=mesh._key)
         del mesh
     assert [m[0, 0] for m in rec.meshes] == [k + 1.0 for k in range(50)]
+
+
+@pytest.mark.parametrize("device", [False, True])
+def test_a_refused_mesh_leaves_none_resident(recorded, device):
+    rec, ctx = recorded
+    mesh, bad = (MeshGrid.TriangularMesh(np.eye(3) * s, IEN) for s in (1.0, 2.0))
+    ctx.set_mesh(mesh.vertex_rows(), mesh.triangle_rows(), key=mesh._key)
+    rec.refuse = True
+    with pytest.raises(_native.SdfGpuError):
+        if device:
+            ctx.set_mesh_device(0, 3, 0, 1)
+        else:
+            ctx.set_mesh(bad.vertex_rows(), bad.triangle_rows(), key=bad._key)
+    rec.refuse = False
+    ctx.set_mesh(mesh.vertex_rows(), mesh.triangle_rows(), key=mesh._key)
+    assert len(rec.meshes) == 2  # uploaded again
