@@ -210,8 +210,8 @@ __global__ void __launch_bounds__(kRbfThreads) k_rbf_update(int64_t n, double* _
 }
 
 // The coarse nodes within the cut-off of every fine index along each axis: the first one, the squared
-// FP32 differences the distance is formed from (beyond the last: too large to pass) and the factors
-// exp(-(dx / sigma)^2).
+// FP32 differences the distance is formed from (beyond the last: NaN; a square that overflows is an ordinary
+// tap that no distance bound admits) and the factors exp(-(dx / sigma)^2).
 struct EvalAxis {
   int32_t first[3];  // offset of the axis in the arrays below
   const int32_t* start;
@@ -222,7 +222,7 @@ __global__ void k_rbf_taps(Axis3 fine, Axis3 coarse, double h, double sigma, flo
                            int32_t* __restrict__ start, float* __restrict__ d2, double* __restrict__ g) {
   const int a = blockIdx.y;
   const double inv_s2 = 1.0 / (sigma * sigma);
-  const float reach = maxd * maxd * 1.0001f;
+  const double reach = (double)maxd * (double)maxd * 1.0001;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < fine.n[a]; i += (int64_t)gridDim.x * blockDim.x) {
     const float p = fine.x[a][i];
     const int64_t m = (int64_t)floor(((double)p - (double)coarse.x[a][0]) / h);
@@ -231,19 +231,19 @@ __global__ void k_rbf_taps(Axis3 fine, Axis3 coarse, double h, double sigma, flo
     int n = 0;
     int64_t first = 0;
     for (int64_t c = lo; c <= hi && n < kTaps; ++c) {
-      const float d = __fsub_rn(p, coarse.x[a][c]), q = __fmul_rn(d, d);
-      if (q > reach) {
+      const float d = __fsub_rn(p, coarse.x[a][c]);
+      if ((double)d * (double)d > reach) {
         if (n > 0) break;  // past the cut-off
         continue;
       }
       if (n == 0) first = c;
-      d2[at * kTaps + n] = q;
+      d2[at * kTaps + n] = __fmul_rn(d, d);
       g[at * kTaps + n] = exp(-((double)d * (double)d) * inv_s2);
       ++n;
     }
     start[at] = (int32_t)first;
     for (; n < kTaps; ++n) {
-      d2[at * kTaps + n] = INFINITY;
+      d2[at * kTaps + n] = NAN;
       g[at * kTaps + n] = 0.0;
     }
   }
@@ -285,13 +285,13 @@ __global__ void __launch_bounds__(kRbfThreads) k_rbf_eval(Axis3 fine, Axis3 coar
 #pragma unroll 1
     for (int kz = 0; kz < kTaps; ++kz) {
       const float dz2 = E.d2[iz * kTaps + kz];
-      if (dz2 == INFINITY) break;  // past the axis' taps
+      if (isnan(dz2)) break;  // past the axis' taps
       if (!(dz2 <= smax)) continue;
       const double gz = E.g[iz * kTaps + kz];
 #pragma unroll 1
       for (int ky = 0; ky < kTaps; ++ky) {
         const float dy2 = E.d2[iy * kTaps + ky];
-        if (dy2 == INFINITY) break;
+        if (isnan(dy2)) break;
         if (!(__fadd_rn(dy2, dz2) <= smax)) continue;  // rounding is monotone: no x can pass
         const double* row = wxy + ((cz + kz) * cny + ky) * cnx;
         double sum = 0.0;
@@ -453,8 +453,9 @@ extern "C" int sdfgpu_rbf_smoothing(sdfgpu_ctx* ctx, const double aabb_min[3], c
     res = std::sqrt(rr);
     weights = x;
   }
-  // per-axis taps of the fine points; smax: the largest float whose correctly rounded square root is
-  // within maxd (the root is monotone), so the terms are those of "sqrt(s) <= maxd"
+  // per-axis taps of the fine points; smax: the largest finite float whose correctly rounded square root is
+  // within maxd (the root is monotone), so the terms are those of "sqrt(s) <= maxd" (a sum s that overflows
+  // is an infinite distance, whose term is 0 where maxd is infinite too)
   EvalAxis E;
   E.first[0] = 0;
   E.first[1] = (int32_t)nf[0];
@@ -470,8 +471,8 @@ extern "C" int sdfgpu_rbf_smoothing(sdfgpu_ctx* ctx, const double aabb_min[3], c
   E.start = tstart;
   E.d2 = td2;
   E.g = tg;
-  float smax = maxd * maxd;
-  while (std::sqrt(std::nextafter(smax, INFINITY)) <= maxd) smax = std::nextafter(smax, INFINITY);
+  float smax = std::min(maxd * maxd, FLT_MAX);
+  while (smax < FLT_MAX && std::sqrt(std::nextafter(smax, INFINITY)) <= maxd) smax = std::nextafter(smax, INFINITY);
   while (smax > 0.f && std::sqrt(smax) > maxd) smax = std::nextafter(smax, 0.f);
   k_rbf_taps<<<dim3(grid_for(std::max(nf[0], std::max(nf[1], nf[2])), 128), 3), 128, 0, st>>>(
       af, ac, cell_size, sigma, maxd, R, E, tstart, td2, tg);

@@ -125,3 +125,18 @@ def test_gpu_products_across_tiles_and_cutoffs(gpu_ctx, N, thr):
         b32 = rbf.process_vector(d)
         if its < d.size:
             assert np.linalg.norm(K @ w - b32) <= 1.05 * np.sqrt(np.finfo(np.float32).eps) * np.linalg.norm(b32)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cell,N", [(1e-18, (5, 4, 3)), (6e18, (9, 4, 3)), (1e19, (9, 8, 7)), (5e19, (5, 4, 3)),
+                                    (9e37, (3, 2, 3)), (2e38, (1, 1, 1))])
+def test_gpu_cells_at_the_ends_of_the_fp32_range(gpu_ctx, cell, N):
+    """Cut-offs whose square, or which themselves, overflow FP32: the call returns, and the terms are those of
+    the FP32 distances."""
+    o, amax, N, h = _grid(N, cell)
+    d = np.random.default_rng(5).normal(size=int(np.prod(N + 1)))
+    with np.errstate(over="ignore"):
+        ref = rbf.evaluate(rbf.fine_axes(o, amax, N, 2)[0], rbf.coarse_axes(o, amax, N), rbf.process_vector(d), h, 1e-3,
+                           k=min(d.size, 400))
+    got, _, _, _ = gpu_ctx.rbf_smoothing(o, amax, N, h, d, interpolation=False, smooth=2)
+    assert np.max(np.abs(got - ref)) <= 4e-6 * np.max(np.abs(ref))  # as above
