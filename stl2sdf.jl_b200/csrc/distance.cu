@@ -362,7 +362,7 @@ __global__ void k_fill_empty(GridP g, const int32_t* __restrict__ tile_cnt, doub
     node_ijk(g, lin, i, j, k);
     const int64_t tile = (k / g.t[2] * g.nt[1] + j / g.t[1]) * g.nt[0] + i / g.t[0];
     if (tile_cnt[tile] != 0) continue;
-    dist[lin] = g.h;
+    dist[lin] = fmin(g.h, kBig);  // the fold's initial minimum, where the cells are larger
     status[lin] = 0;
     if (xp) {
       xp[3 * lin] = 0.0;

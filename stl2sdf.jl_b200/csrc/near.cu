@@ -3,7 +3,8 @@
 // triangles to the nodes within one cell of them instead of candidate lists.
 //
 // Every result is clamped to h (:202-206), and every value the fold can assign for a triangle is at
-// least its true distance, so a node farther than h from all triangles gets h.  For the others let D be
+// least its true distance, so a node farther than h from all triangles gets h (or kBig, the fold's initial
+// minimum, where the cells are larger than that).  For the others let D be
 // the smallest true distance.  A candidate's step (:101-176) assigns, given the running minimum m,
 //   its plane distance when p projects inside;
 //   otherwise F, the smallest distance to a foot on its edges, when F < m;
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(kNodesThreads) k_near_nodes(const __grid_const
     for (int q = 0; q < kNodes; ++q) {
       const int64_t lin = base + q * kNodesThreads + threadIdx.x;
       const bool in = lin < g.ngp, is = in && A.m2[lin] != 0x7f7f7f7fu;
-      if (in && !is) A.dist[lin] = g.h;
+      if (in && !is) A.dist[lin] = fmin(g.h, kBig);
       const unsigned mask = __ballot_sync(0xffffffffu, is);
       before[q] = total + __popc(mask & ((1u << lane) - 1u));
       total += __popc(mask);
@@ -283,7 +284,7 @@ __global__ void __launch_bounds__(128, 6) k_near_resolve(const __grid_constant__
     const int n = A.cnt[q];
     bool hard = n < 1 || n > kSlots;
     for (int s = 0; s < n && !hard; ++s) hard = (slot[s] & kWeakTri) != 0;
-    double m = INFINITY, nearest = INFINITY;  // nearest: a squared distance of a triangle fit for FP32 decisions
+    double m = kBig, nearest = INFINITY;  // nearest: a squared distance of a triangle fit for FP32 decisions
     if (hard) {
       for (int s = 0; s < min(n, kSlots); ++s) {
         int feat;

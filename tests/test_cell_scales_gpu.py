@@ -1,0 +1,52 @@
+"""Every distance mode at cell sizes around 1e10, the reference's initial minimum (abs(-1.0e10),
+src/SignedDistances/dfOnTriangularMesh.jl:31), every node against the FP64 oracle, bit for bit: above it a node
+that no triangle comes closer to keeps that minimum, whether or not it has candidates."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import oracle
+from workloads import synthetic
+
+pytestmark = pytest.mark.gpu
+
+
+
+def check(ctx, h, cells, mode, want_xp, away=0.0):
+    """A sphere whose triangles reach `cells` cells from their centroids, `away` radii from the origin."""
+    V, F = synthetic.icosphere(3, jitter=0.1, seed=5)
+    T = V[F - 1]
+    V = V * (cells * h / np.linalg.norm(T - T.mean(1, keepdims=True), axis=2).max())
+    V = V + away * V.max()
+    lo, hi = V.min(0), V.max(0)
+    N = np.minimum(np.ceil((hi - lo) / h).astype(np.int64) + 14, 40)
+    o = 0.5 * (lo + hi) - 0.5 * h * N + 0.123 * h
+    ctx.set_mesh(V, F)
+    ref, _, _ = oracle.distances(V, F, o, h, N, mode=mode)
+    d, _ = ctx.distances(o, h, N, mode, want_xp=want_xp)
+    assert np.array_equal(d, ref)
+    return ctx.stats()
+
+
+H = [5e9, 1e10, 1.0000000001e10, 3e10, 1e12]
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("h", H)
+@pytest.mark.parametrize("cells", [0.01, 0.4, 1.4])
+def test_scatter(gpu_ctx, h, cells, mode):
+    assert check(gpu_ctx, h, cells, mode, False)["band_nodes"] > 0
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("h", H)
+@pytest.mark.parametrize("away", [0.0, 100.0])  # the scatter takes meshes near the origin
+def test_tiles(gpu_ctx, h, mode, away):
+    assert check(gpu_ctx, h, 0.01, mode, away == 0.0, away)["band_nodes"] == 0
+
+
+@pytest.mark.parametrize("h", H)
+def test_unbounded(gpu_ctx, h):
+    check(gpu_ctx, h, 0.4, 2, True)
