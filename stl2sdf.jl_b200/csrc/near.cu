@@ -547,13 +547,15 @@ __global__ void __launch_bounds__(128) k_hard_replay(const __grid_constant__ Nea
 // Whether near_distances takes this call: triangles of at most 1.5 (reference rule) or 4 cells from their
 // centroid, the mesh near the coordinate origin (see unb_mesh), mesh and grid within 1e5 cells of the mesh's
 // centre (FP32 node indices within half a cell, and a box's rows within a mask), and few and small triangles
-// unfit for FP32 decisions, each of which sends the nodes nearest to it to the replay.
+// unfit for FP32 decisions, each of which sends the nodes nearest to it to the replay.  And cells whose squares
+// FP32 holds with all their digits: from 1e-15 the error of a square of a few cells by underflow, at most
+// sqrt(16 * 2^-149) = 1.5e-22 of distance, is below a tenth of eD, and up to 1e15 nothing overflows.
 bool near_applies(const sdfgpu_ctx* ctx, const GridP& g, int mode) {
   const MeshDev& M = ctx->mesh;
   double off = 0.0;
   for (int a = 0; a < 3; ++a) off = std::max(off, std::fabs(M.center[a]));
   const double rho = M.rho_max * (1.0 + 1e-9) + 1e-6 * g.E;
-  return off <= 64.0 * M.E && g.E <= 1e5 * g.h && rho < (mode == SDFGPU_MODE_REF_RULE ? 1.5 : 4.0) * g.h && M.rho_weak <= 1.5 * g.h &&
+  return off <= 64.0 * M.E && g.h >= 1e-15 && g.h <= 1e15 && g.E <= 1e5 * g.h && rho < (mode == SDFGPU_MODE_REF_RULE ? 1.5 : 4.0) * g.h && M.rho_weak <= 1.5 * g.h &&
          M.n_weak <= M.nel / 64;
 }
 

@@ -1,6 +1,7 @@
-"""Every distance mode at cell sizes around 1e10, the reference's initial minimum (abs(-1.0e10),
-src/SignedDistances/dfOnTriangularMesh.jl:31), every node against the FP64 oracle, bit for bit: above it a node
-that no triangle comes closer to keeps that minimum, whether or not it has candidates."""
+"""Every distance mode at the ends of the range of cell sizes, every node against the FP64 oracle, bit for bit.
+Around 1e10, the reference's initial minimum (abs(-1.0e10), src/SignedDistances/dfOnTriangularMesh.jl:31): above
+it a node that no triangle comes closer to keeps that minimum, whether or not it has candidates.  And where
+the squares of FP32 distances lose digits by underflow."""
 
 from __future__ import annotations
 
@@ -14,9 +15,9 @@ pytestmark = pytest.mark.gpu
 
 
 
-def check(ctx, h, cells, mode, want_xp, away=0.0):
+def check(ctx, h, cells, mode, want_xp, away=0.0, level=3):
     """A sphere whose triangles reach `cells` cells from their centroids, `away` radii from the origin."""
-    V, F = synthetic.icosphere(3, jitter=0.1, seed=5)
+    V, F = synthetic.icosphere(level, jitter=0.1, seed=5)
     T = V[F - 1]
     V = V * (cells * h / np.linalg.norm(T - T.mean(1, keepdims=True), axis=2).max())
     V = V + away * V.max()
@@ -50,3 +51,14 @@ def test_tiles(gpu_ctx, h, mode, away):
 @pytest.mark.parametrize("h", H)
 def test_unbounded(gpu_ctx, h):
     check(gpu_ctx, h, 0.4, 2, True)
+
+
+SMALL = [2e-15, 5e-16, 1e-19, 1e-20, 1e-21, 1e-22, 1e-24]
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("h", SMALL)
+@pytest.mark.parametrize("cells,level", [(0.3, 4), (0.66, 5), (1.4, 3)])
+def test_small_cells(gpu_ctx, h, cells, level, mode):
+    st = check(gpu_ctx, h, cells, mode, False, level=level)
+    assert (st["band_nodes"] > 0) == (h > 1e-15)  # the scatter takes the larger ones
