@@ -74,14 +74,15 @@ inline LeafTris leaf_tris(sdfgpu_ctx* ctx) { return {buf<float4>(ctx, "ltri"), c
 
 // The mesh's arrays of a search beyond its positional fields.  lane_resolve compares plain FP64 distances
 // only while the mesh lies within 64 of its own half-extents of the coordinate origin: far from it the
-// reference's barycentric solve, which works on absolute coordinates, loses the digits it relies on.
+// reference's barycentric solve, which works on absolute coordinates, loses the digits it relies on.  And from
+// 1e-15 on, below which the FP32 root in its tolerance can underflow.
 inline void unb_mesh(sdfgpu_ctx* ctx, UnbArgs& A) {
   const MeshDev& M = ctx->mesh;
   double off = 0.0;
   for (int a = 0; a < 3; ++a) off = M.center[a] > off ? M.center[a] : (-M.center[a] > off ? -M.center[a] : off);
   A.lv32 = buf<float4>(ctx, "lv32");
   A.v32 = buf<float4>(ctx, "v32");
-  A.local = off <= 64.0 * M.E;
+  A.local = off <= 64.0 * M.E && M.E >= 1e-15;
 }
 
 // Error model of the FP32 searches, u = 2^-24.  Coordinates in the mesh-local frame are within E, so
@@ -96,6 +97,8 @@ constexpr float kUnbDistRel = 1.5e-6f;
 // plane and edge lines below 1e-6 E + 1e-6 (d + its edges); with the error of the distance itself,
 // kWidePadRel (E + d) plus the share of the longest edge covers both.
 constexpr float kWidePadRel = 4.0e-6f;
+// What underflow takes from a squared distance of up to 16 terms, 16 * 2^-149, as a distance; it enters both.
+constexpr float kUnbUnderflow = 2.0e-22f;
 // FP32 margin of the box tests of the FP64 re-search, as a multiple of E (per-lane box distances).
 constexpr float kUnbPadRel = 2.2e-5f;
 
@@ -104,9 +107,9 @@ inline void unb_errors(const MeshDev& M, double E, UnbArgs& A) {
   A.E = (float)E;
   A.pad = kUnbPadRel * (float)E;
   // edges are at most 2 rho_max long
-  A.eD_abs = kUnbDistRel * (float)E + 2.0e-6f * (float)M.rho_max;
+  A.eD_abs = kUnbDistRel * (float)E + 2.0e-6f * (float)M.rho_max + kUnbUnderflow;
   A.eD_rel = kUnbDistRel;
-  A.wpad_abs = kWidePadRel * (float)E + 2.0e-6f * (float)M.rho_max;
+  A.wpad_abs = kWidePadRel * (float)E + 2.0e-6f * (float)M.rho_max + kUnbUnderflow;
 }
 
 // Squared lower bound on the distance from p to the child `side` of an LBVH node: the larger of its

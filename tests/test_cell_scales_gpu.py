@@ -53,7 +53,7 @@ def test_unbounded(gpu_ctx, h):
     check(gpu_ctx, h, 0.4, 2, True)
 
 
-SMALL = [2e-15, 5e-16, 1e-19, 1e-20, 1e-21, 1e-22, 1e-24]
+SMALL = [2e-15, 5e-16, 1e-20, 1e-22, 1e-24]
 
 
 @pytest.mark.parametrize("mode", [0, 1])
@@ -62,3 +62,10 @@ SMALL = [2e-15, 5e-16, 1e-19, 1e-20, 1e-21, 1e-22, 1e-24]
 def test_small_cells(gpu_ctx, h, cells, level, mode):
     st = check(gpu_ctx, h, cells, mode, False, level=level)
     assert (st["band_nodes"] > 0) == (h > 1e-15)  # the scatter takes the larger ones
+
+
+@pytest.mark.parametrize("mode", [0, 2])  # with closest points: the nearest-vertex fallback, the search
+@pytest.mark.parametrize("h", SMALL)
+@pytest.mark.parametrize("cells,level", [(0.3, 4), (0.66, 5), (1.4, 3)])
+def test_searches_of_small_cells(gpu_ctx, h, cells, level, mode):
+    check(gpu_ctx, h, cells, mode, True, level=level)
