@@ -54,7 +54,10 @@ __device__ __forceinline__ void make_cand(const float3 a, const float3 e1, const
   const float L0 = len3(e1), L1 = len3(ed1), L2 = len3(e2);
   const float3 n = cross3f(e1, e2);
   const float nn = len3(n);
-  const bool fine = ok && nn > 0.f && L0 > 0.f && L1 > 0.f && L2 > 0.f;
+  const float size = len3(a) + L0 + L2;
+  // products of up to four lengths (n . n, and n . (edge x offset)): FP32 holds them, and their digits, in this
+  // range; beyond it the candidate is decided in FP64
+  const bool fine = ok && nn > 2.0e-19f && size < 1.0e9f && L0 > 0.f && L1 > 0.f && L2 > 0.f;
   const float inn = fine ? 1.0f / nn : 0.f;
   c.a = make_float4(a.x, a.y, a.z, fine ? L0 * L2 * inn : INFINITY);
   c.e1 = make_float4(e1.x, e1.y, e1.z, L0);
@@ -65,7 +68,7 @@ __device__ __forceinline__ void make_cand(const float3 a, const float3 e1, const
   c.u1 = make_float4(ed1.x * r1, ed1.y * r1, ed1.z * r1, r0 * inn);
   c.u2 = make_float4(-e2.x * r2, -e2.y * r2, -e2.z * r2, r1 * inn);
   c.gid = make_int4(g0, g1, g2, tri);
-  c.aux = make_float4(r2 * inn, len3(a) + L0 + L2, 0.f, 0.f);
+  c.aux = make_float4(r2 * inn, size, 0.f, 0.f);
 }
 
 __device__ __forceinline__ float cand_err(const Cand32& c, float plen) {

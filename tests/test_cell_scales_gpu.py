@@ -1,7 +1,7 @@
 """Every distance mode at the ends of the range of cell sizes, every node against the FP64 oracle, bit for bit.
 Around 1e10, the reference's initial minimum (abs(-1.0e10), src/SignedDistances/dfOnTriangularMesh.jl:31): above
 it a node that no triangle comes closer to keeps that minimum, whether or not it has candidates.  And where
-the squares of FP32 distances lose digits by underflow."""
+the squares of FP32 distances, or the tile fold's products of four lengths, overflow or lose digits by underflow."""
 
 from __future__ import annotations
 
@@ -69,3 +69,10 @@ def test_small_cells(gpu_ctx, h, cells, level, mode):
 @pytest.mark.parametrize("cells,level", [(0.3, 4), (0.66, 5), (1.4, 3)])
 def test_searches_of_small_cells(gpu_ctx, h, cells, level, mode):
     check(gpu_ctx, h, cells, mode, True, level=level)
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("h", H + [1e8, 1e16, 1e-9, 1e-10, 3e-11, 1e-11, 1e-12])
+@pytest.mark.parametrize("cells", [0.4, 2.5, 6.0])
+def test_tiles_where_products_of_four_lengths_leave_fp32(gpu_ctx, h, cells, mode):
+    check(gpu_ctx, h, cells, mode, True)
