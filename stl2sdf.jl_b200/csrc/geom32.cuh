@@ -29,19 +29,23 @@ __device__ __forceinline__ float seg_d2(float3 p, float3 a, float3 e) {
 }
 
 // Squared distance from p to triangle (a, b, c): minimum of the three edge distances and, when
-// p projects inside, the plane distance.  Degenerate triangles reduce to their edges.
+// p projects inside, the plane distance.  Degenerate triangles reduce to their edges.  The normal is formed
+// from edges scaled to about 1: products of all the lengths would leave FP32 from some 1e6 on.
 __device__ __forceinline__ float pt_tri_d2(float3 p, float3 a, float3 b, float3 c) {
   const float3 ab = b - a, bc = c - b, ca = a - c;
   float d2 = fminf(seg_d2(p, a, ab), fminf(seg_d2(p, b, bc), seg_d2(p, c, ca)));
-  const float3 n = cross3f(ab, c - a);
+  const float size = fmaxf(fmaxf(fmaxf(fabsf(ab.x), fabsf(ab.y)), fmaxf(fabsf(ab.z), fabsf(ca.x))),
+                           fmaxf(fabsf(ca.y), fabsf(ca.z)));
+  const float inv = 1.f / size;
+  const float3 u = ab * inv, v = bc * inv, w = ca * inv, n = cross3f(w, u);
   const float nn = dot3f(n, n);
   if (nn > 0.f) {
-    const float s1 = dot3f(cross3f(ab, p - a), n);
-    const float s2 = dot3f(cross3f(bc, p - b), n);
-    const float s3 = dot3f(cross3f(ca, p - c), n);
+    const float s1 = dot3f(cross3f(u, p - a), n);
+    const float s2 = dot3f(cross3f(v, p - b), n);
+    const float s3 = dot3f(cross3f(w, p - c), n);
     if (s1 >= 0.f && s2 >= 0.f && s3 >= 0.f) {
-      const float pd = dot3f(p - a, n);
-      d2 = fminf(d2, pd * pd / nn);
+      const float pd = dot3f(p - a, n) / sqrtf(nn);
+      d2 = fminf(d2, pd * pd);
     }
   }
   return d2;

@@ -1,7 +1,8 @@
 """Every distance mode at the ends of the range of cell sizes, every node against the FP64 oracle, bit for bit.
 Around 1e10, the reference's initial minimum (abs(-1.0e10), src/SignedDistances/dfOnTriangularMesh.jl:31): above
 it a node that no triangle comes closer to keeps that minimum, whether or not it has candidates.  And where
-the squares of FP32 distances, or the tile fold's products of four lengths, overflow or lose digits by underflow."""
+the squares of FP32 distances, or the tile fold's products of four lengths, overflow or lose digits by
+underflow."""
 
 from __future__ import annotations
 
@@ -15,9 +16,10 @@ pytestmark = pytest.mark.gpu
 
 
 
-def check(ctx, h, cells, mode, want_xp, away=0.0, level=3):
+def check(ctx, h, cells, mode, want_xp, away=0.0, level=3, copies=1):
     """A sphere whose triangles reach `cells` cells from their centroids, `away` radii from the origin."""
     V, F = synthetic.icosphere(level, jitter=0.1, seed=5)
+    F = np.repeat(F, copies, axis=0)
     T = V[F - 1]
     V = V * (cells * h / np.linalg.norm(T - T.mean(1, keepdims=True), axis=2).max())
     V = V + away * V.max()
@@ -76,3 +78,15 @@ def test_searches_of_small_cells(gpu_ctx, h, cells, level, mode):
 @pytest.mark.parametrize("cells", [0.4, 2.5, 6.0])
 def test_tiles_where_products_of_four_lengths_leave_fp32(gpu_ctx, h, cells, mode):
     check(gpu_ctx, h, cells, mode, True)
+
+
+@pytest.mark.parametrize("h", [1e8, 1e7, 1e6, 1e5, 1.0, 1e-6, 1e-8, 1e-12, 1e-16])
+@pytest.mark.parametrize("cells,level", [(6.0, 1), (8.1, 2)])
+def test_large_triangles_off_the_candidates(gpu_ctx, h, cells, level):
+    """The nodes within a cell of a triangle whose centroid is far take the nearest-vertex fallback."""
+    assert check(gpu_ctx, h, cells, 0, False, level=level)["knn_fallback_nodes"] > 0
+
+
+@pytest.mark.parametrize("h", [1e8, 1e7, 1e6, 1e5, 1.0, 1e-6, 1e-8, 1e-12, 1e-16])
+def test_more_coincident_triangles_than_a_node_keeps(gpu_ctx, h):
+    check(gpu_ctx, h, 6.0, 2, True, level=0, copies=20)
