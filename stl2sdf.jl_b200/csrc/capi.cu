@@ -321,6 +321,14 @@ int run_all(sdfgpu_ctx* ctx, const GridP& g, bool want_dist, bool want_sign, int
     return rc;
   }
   SDF_TRY(finish_counters(ctx, g));
+  if (ctx->h_counters[C_HARD_LEFT]) {
+    SDF_CUDA(ctx, cudaMemsetAsync(ctx->d_counters + C_HARD_LEFT, 0, sizeof(int64_t), ctx->stream));
+    ctx->h_counters[C_BAND] = 0;
+    SDF_TRY(run_tiles(ctx, g, mode, d_dist, d_xp));
+    SDF_MARK(ctx, T_DIST1);
+    if (want_sign && d_sdf) SDF_TRY(run_combine(ctx, g, d_dist, d_sign, d_sdf));
+    SDF_TRY(finish_counters(ctx, g));
+  }
   auto span = [&](int a, int b, double* out) -> int {
     float ms = 0.f;
     SDF_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->tev[a], ctx->tev[b]));

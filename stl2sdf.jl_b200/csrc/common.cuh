@@ -53,6 +53,7 @@ enum Counter : int {
   C_CERTIFIED,      // learned radius: nodes certified by the bounded search
   C_VISITS,         // LBVH nodes visited by the unbounded search
   C_SIGN_BAND,      // ray-triangle decisions inside the FP32 band, replayed in FP64
+  C_HARD_LEFT,      // nodes whose fold the scatter could not replay: the tile fold takes the call
   C_NUM = 32
 };
 
@@ -265,6 +266,9 @@ int ensure_tree(sdfgpu_ctx* ctx, bool boxes);
 // enqueued, or after an unbounded search has been.
 int run_distances(sdfgpu_ctx* ctx, const GridP& g, int mode, int use_learned, double* d_dist, double* d_xp,
                   const std::function<int()>& between = {});
+// The reference-rule / h-bounded stage by tile lists and folds.
+int run_tiles(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, double* d_xp,
+              const std::function<int()>& between = {});
 // Exact unbounded distances of a sparse grid's nodes, one thread per node (learned.cu).
 int run_nearest_points(sdfgpu_ctx* ctx, const GridP& g, double* d_dist);
 
@@ -293,7 +297,8 @@ struct DistPlan {
 int dist_prepare(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, double* d_xp, DistPlan& P,
                  int use_learned = 0);
 int dist_fold(sdfgpu_ctx* ctx, const DistPlan& P);
-// The same stage as a scatter from the triangles to the nodes near them (near.cu).
+// The same stage as a scatter from the triangles to the nodes near them (near.cu).  Where it leaves nodes open
+// (C_HARD_LEFT) the caller runs the tile fold.
 bool near_applies(const sdfgpu_ctx* ctx, const GridP& g, int mode);
 int near_prepare(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, DistPlan& P);
 int near_run(sdfgpu_ctx* ctx, const DistPlan& P);

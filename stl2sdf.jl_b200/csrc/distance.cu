@@ -681,8 +681,8 @@ int run_distances(sdfgpu_ctx* ctx, const GridP& g, int mode, int use_learned, do
     return between ? between() : 0;
   }
 
-  DistPlan P;
   if (!d_xp && !ctx->tune_tiles && near_applies(ctx, g, mode)) {
+    DistPlan P;
     SDF_TRY(near_prepare(ctx, g, mode, d_dist, P));
     SDF_MARK(ctx, T_TILES);
     if (between) SDF_TRY(between());
@@ -690,12 +690,18 @@ int run_distances(sdfgpu_ctx* ctx, const GridP& g, int mode, int use_learned, do
     SDF_MARK(ctx, T_FOLD);
     return 0;
   }
+  return run_tiles(ctx, g, mode, d_dist, d_xp, between);
+}
+
+int run_tiles(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, double* d_xp,
+              const std::function<int()>& between) {
+  DistPlan P;
   SDF_TRY(dist_prepare(ctx, g, mode, d_dist, d_xp, P));
   SDF_MARK(ctx, T_TILES);
   if (between) SDF_TRY(between());
   SDF_TRY(dist_fold(ctx, P));
   SDF_MARK(ctx, T_FOLD);
-  if (P.knn) SDF_TRY(dist_knn(ctx, P, st, true));
+  if (P.knn) SDF_TRY(dist_knn(ctx, P, ctx->stream, true));
   return 0;
 }
 

@@ -14,7 +14,9 @@
 // whenever no value depends on m, or those that do cannot go below the others -- or when they share
 // one V and, in index order, some F is not below the F before it: after the earlier one m is at most its
 // F, so the later one's feet do not improve it and V is taken.  Nodes for which none of this holds, and
-// nodes next to a triangle unfit for FP32 decisions, replay the whole fold (k_hard_*).
+// nodes next to a triangle unfit for FP32 decisions, replay the whole fold (k_hard_*); when their candidates do
+// not fit the lists (hundreds of coincident triangles, a fan of a thousand in a large mesh), the tile fold takes
+// the call, whose work is bounded by the candidates' number.
 // SDFGPU_MODE_EXACT takes the true minimum, so its ties' smallest value is the result.
 //
 // A triangle within h of a node has its centroid within h + rho of it (rho the mesh's largest
@@ -38,7 +40,12 @@ namespace {
 
 constexpr int kSlots = 16;        // triangles kept per near node
 constexpr int kHardCap = 1024;    // candidates listed per hard node (more: the mesh is scanned)
-constexpr int64_t kHardPool = 16 << 20;  // candidates listed in all
+constexpr int64_t kHardPool = 16 << 20;  // candidates listed in all (likewise)
+// A scan is a warp's walk of the mesh, 20 ns a triangle by its latency, for as many nodes as there are resident
+// warps; the tile fold with its lists takes 0.3 ms and 4.5 ns a triangle for the whole call (2.1M triangles of
+// which 2000 meet in one point, B200: 43.7 ms with scans, 10.2 ms handed over).  They meet at about 19k triangles.
+constexpr int64_t kScanTriangles = 16384;
+constexpr int kScanNodes = 4096;
 constexpr int kTileShift = 2;     // flags of 4 x 4 x 4 node tiles with hard nodes
 
 struct NearArgs {
@@ -71,6 +78,8 @@ struct NearArgs {
   int32_t* hard_n;
   int32_t* hard;        // near indices of hard nodes
   int32_t* unbounded_n; // hard nodes whose hbound is not known from their slots
+  int32_t* scan_n;      // hard nodes without a list
+  int32_t scan_max;     // how many of them are scanned for; with more the tile fold takes the call
   uint8_t* tflag;       // tiles with hard nodes
   uint8_t* tcand;       // tiles in which a candidate of a hard node can have its centroid
   int64_t tn[3];
@@ -411,6 +420,7 @@ __global__ void __launch_bounds__(128) k_hard_collect(const __grid_constant__ Ne
   if (*A.hard_n == 0) return;
   if (kPhase == 0 && *A.unbounded_n == 0) return;
   if (kPhase == 1 && hard_uniform(*A.hard_n)) return;
+  if (kPhase == 2 && *A.scan_n > A.scan_max) return;
   const GridP& g = A.g;
   const double tol = 1e-9 * (double)A.E;
   for (int64_t el = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; el < A.nel; el += (int64_t)gridDim.x * blockDim.x) {
@@ -462,6 +472,7 @@ __global__ void __launch_bounds__(128) k_hard_collect(const __grid_constant__ Ne
                   atomicAdd(A.hcnt + hq, 1);
                 } else if (A.hoff[hq] >= 0) {
                   const int c = atomicAdd(A.hcnt + hq, 1);
+                  if (c == kHardCap) atomicAdd(A.scan_n, 1);
                   if (c < kHardCap) A.pool[A.hoff[hq] + c] = (int32_t)el;
                 }
               }
@@ -481,6 +492,7 @@ __global__ void k_hard_place(const __grid_constant__ NearArgs A) {
       off = (int64_t)atomicAdd(A.pool_n, (unsigned long long)c);
       if (off + c > kHardPool) off = -1;
     }
+    if (off < 0) atomicAdd(A.scan_n, 1);
     A.hoff[hq] = off;
     A.hcnt[hq] = 0;
   }
@@ -489,11 +501,15 @@ __global__ void k_hard_place(const __grid_constant__ NearArgs A) {
 // Replays the fold of a hard node, one warp each: the candidates in ascending index 32 at a time, a lane
 // per candidate bounding its distance from below (near64; 0 where that is not certain), and the
 // reference step on those that the running minimum does not exclude (every value a step can assign is at
-// least the true distance).  The few nodes whose list is too long scan the mesh instead.
+// least the true distance).  Nodes without a list scan the mesh instead, where that is the cheaper way.
 __global__ void __launch_bounds__(128) k_hard_replay(const __grid_constant__ NearArgs A) {
   __shared__ int s_list[4][kHardCap];
   const GridP& g = A.g;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (*A.scan_n > A.scan_max) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) count_add(A.counters, C_HARD_LEFT, *A.scan_n);
+    return;
+  }
   const int n_hard = *A.hard_n;
   const double tol = 1e-9 * (double)A.E;
   uint32_t fp64 = 0;
@@ -544,7 +560,7 @@ __global__ void __launch_bounds__(128) k_hard_replay(const __grid_constant__ Nea
 
 }  // namespace
 
-// Whether near_distances takes this call: triangles of at most 1.5 (reference rule) or 4 cells from their
+// Whether near_prepare and near_run take this call: triangles of at most 1.5 (reference rule) or 4 cells from their
 // centroid, the mesh near the coordinate origin (see unb_mesh), mesh and grid within 1e5 cells of the mesh's
 // centre (FP32 node indices within half a cell, and a box's rows within a mask), and few and small triangles
 // unfit for FP32 decisions, each of which sends the nodes nearest to it to the replay.  And cells whose squares
@@ -605,7 +621,7 @@ int near_prepare(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, Dist
     A.tn[a] = (g.n[a] >> kTileShift) + 1;
     tiles *= A.tn[a];
   }
-  int32_t* counts;  // near nodes, hard nodes, hard nodes without a bound; the pool's length
+  int32_t* counts;  // near nodes, hard nodes, hard nodes without a bound, without a list; the pool's length
   SDF_TRY(scratch_t(ctx, "near_m2", (size_t)g.ngp, &A.m2));
   SDF_TRY(scratch_t(ctx, "near_map", (size_t)g.ngp, &A.map));
   SDF_TRY(scratch_t(ctx, "near_node", (size_t)g.ngp, &A.node));
@@ -616,6 +632,8 @@ int near_prepare(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, Dist
   A.near_n = counts;
   A.hard_n = counts + 1;
   A.unbounded_n = counts + 2;
+  A.scan_n = counts + 3;
+  A.scan_max = M.nel <= kScanTriangles ? kScanNodes : 0;
   A.pool_n = reinterpret_cast<unsigned long long*>(counts + 4);
   SDF_CUDA(ctx, cudaMemsetAsync(A.m2, 0x7f, sizeof(uint32_t) * g.ngp, st));  // 3.39e38
   SDF_CUDA(ctx, cudaMemsetAsync(counts, 0, 6 * sizeof(int32_t), st));
