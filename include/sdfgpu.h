@@ -227,7 +227,8 @@ typedef struct sdfgpu_batch_item {
  * `streams` worker contexts on the device of ctx (0 = 8), each with its own stream and host thread,
  * take meshes from a shared queue, largest estimated work (ngp * log2(nel)) first, so small and
  * large meshes overlap on the GPU.  With autotune = 1 each size class (log4 of ngp, log4 of nel)
- * gets its tile from sdfgpu_autotune the first time it appears; the choice is kept in ctx for later
+ * gets its tile from sdfgpu_autotune the first time it appears with an item whose distances the tile
+ * fold (or, in the unbounded modes, the brick search) computes; the choice is kept in ctx for later
  * calls.  Results equal per-mesh sdfgpu_sdf calls.  ctx's own mesh is left as it was; ctx's stats
  * become the sums over the items (rho_max: the maximum; ms_*: summed per-item device times).
  * Returns the first failure; its message names the item. */
@@ -256,10 +257,12 @@ int sdfgpu_sdf_batch_ex(sdfgpu_ctx* ctx, sdfgpu_batch_item* items, int64_t count
                         int32_t max_rays, double confidence_threshold, int32_t use_winding_fallback, int32_t streams,
                         int32_t autotune, int32_t persistent);
 
-/* Tile autotuner for the distance stage (the reference has no counterpart).  Times the current mesh
- * on the grid (origin, h, N) in `mode` with each built-in tile shape (nodes per CTA along x, y, z:
- * 4x4x4, 8x4x2, 4x4x2, 8x4x4, 4x4x8, 8x8x4), keeps the fastest as ctx's tile and writes it to
- * tile_out and its device time to ms_out (either may be NULL).  In SDFGPU_MODE_UNBOUNDED, which
+/* Tile autotuner for the distance stage (the reference has no counterpart).  Times the tile fold of
+ * the current mesh on the grid (origin, h, N) in `mode` with each built-in tile shape (nodes per CTA
+ * along x, y, z: 4x4x4, 8x4x2, 4x4x2, 8x4x4, 4x4x8, 8x8x4), keeps the fastest as ctx's tile and writes
+ * it to tile_out and its device time to ms_out (either may be NULL).  The tile fold serves closest
+ * points, persistent batches, and meshes whose triangles are large against the cell or that lie far
+ * from the coordinate origin; other truncated distances scatter from the triangles and have no tile.  In SDFGPU_MODE_UNBOUNDED, which
  * has no tiles, it times the warp bricks instead (the 32 nodes one warp searches together:
  * 4x2x4, 4x4x2, 2x4x4, 8x4x1, 4x8x1, 32x1x1) and keeps the fastest as ctx's brick.  Neither shape
  * changes a result, only how the work is split. */

@@ -109,8 +109,8 @@ struct BatchJob {
 
 }  // namespace
 
-// Times the distance stage of the current mesh on grid (origin, h, N) with every tile of kTiles, or,
-// in the unbounded mode (which has no tiles), with every warp brick of kBricks.
+// Times the distance stage of the current mesh on grid (origin, h, N) as a tile fold with every tile of
+// kTiles, or, in the unbounded mode (which has no tiles), with every warp brick of kBricks.
 int autotune_tile(sdfgpu_ctx* ctx, const double origin[3], double h, const int64_t N[3], int mode, int32_t best[3],
                   double* best_ms) {
   const bool bricks = mode == SDFGPU_MODE_UNBOUNDED || mode == SDFGPU_MODE_LEARNED;
@@ -205,7 +205,13 @@ void worker_main(BatchJob& J, sdfgpu_ctx* w) {
     int rc = sdfgpu_set_mesh(w, it.X, it.nnp, it.IEN, it.nel);
     sdfgpu_stats ms = w->stats;
     if (rc == 0 && J.mode == SDFGPU_MODE_LEARNED) rc = train_item(J, w, it, ms);
-    if (rc == 0 && J.autotune) rc = pick_tile(J, w, it);
+    if (rc == 0 && J.autotune) {
+      GridP g;
+      rc = make_grid(w, it.origin, it.h, it.N, g);
+      // the scatter, where it takes the item, has no tiles to tune (a persistent batch folds every item)
+      const bool tiles = J.mode == SDFGPU_MODE_REF_RULE || J.mode == SDFGPU_MODE_EXACT;
+      if (rc == 0 && !(tiles && near_applies(w, g, J.mode))) rc = pick_tile(J, w, it);
+    }
     if (rc == 0)
       rc = sdfgpu_sdf(w, it.origin, it.h, it.N, J.mode, J.min_rays, J.max_rays, J.conf, J.use_winding, it.sdf, it.dist,
                       it.sign, it.conf);
