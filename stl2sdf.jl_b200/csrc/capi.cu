@@ -18,39 +18,31 @@ int fail(sdfgpu_ctx* ctx, int code, const std::string& msg) {
   return code;
 }
 
-// Batch workers take whatever items come up, so each would grow its buffers several times a call for as
-// long as new sizes reach it, and every cudaFree waits for all of them: with 32 meshes and 8 workers 82 frees
-// a call and 33 to 56 ms, against 16 to 29 (B200).  A worker's buffer that has to grow therefore
-// grows to the largest size that any worker has asked for, up to kHintMax and a share of the free memory.
-constexpr size_t kHintMax = (size_t)128 << 20;
-
 int scratch(sdfgpu_ctx* ctx, const char* name, size_t bytes, void** out) {
   DevBuf& b = ctx->ns.empty() ? ctx->bufs[name] : ctx->bufs[ctx->ns + name];
   if (b.cap < bytes) {
-    size_t hint = 0;
-    if (ctx->hints && ctx->ns.empty()) {
-      std::lock_guard<std::mutex> lk(ctx->hints->mu);
-      size_t& most = ctx->hints->bytes[name];
-      most = std::max(most, bytes);
-      hint = std::min(most, kHintMax);
-    }
+    ScratchHints* hints = ctx->ns.empty() ? ctx->hints.get() : nullptr;
     if (b.p) {
       cudaError_t e = cudaFree(b.p);
       b.p = nullptr;
       b.cap = 0;
+      if (b.slack) ctx->hints->give_back(b.slack);
+      b.slack = 0;
       if (e != cudaSuccess) return fail(ctx, SDFGPU_ERR_CUDA, std::string("cudaFree: ") + cudaGetErrorString(e));
     }
     size_t want = bytes + bytes / 8;  // headroom for slowly growing sizes
+    const size_t hint = hints ? hints->grant(name, bytes, want) : want;
     if (hint > want) {
       size_t free_b = 0, total_b = 0;
-      hint += hint / 8;
       if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && hint < free_b / 16 && cudaMalloc(&b.p, hint) == cudaSuccess) {
         b.cap = hint;
+        b.slack = hint - want;
         *out = b.p;
         return 0;
       }
       b.p = nullptr;
       cudaGetLastError();
+      hints->give_back(hint - want);
     }
     cudaError_t e = cudaMalloc(&b.p, want);
     if (e != cudaSuccess) {

@@ -14,6 +14,7 @@
 
 #include "exact64.cuh"
 #include "geom32.cuh"
+#include "hints.hpp"
 #include "radius.cuh"
 #include "sdfgpu.h"
 
@@ -105,12 +106,7 @@ struct MeshDev {
 struct DevBuf {
   void* p = nullptr;
   size_t cap = 0;
-};
-
-// The largest size that any worker of a batch has asked for, per scratch buffer (see scratch()).
-struct ScratchHints {
-  std::mutex mu;
-  std::unordered_map<std::string, size_t> bytes;
+  size_t slack = 0;  // what a hint added to it
 };
 
 }  // namespace sdfgpu
