@@ -650,7 +650,7 @@ __global__ void k_ine_fill(const int64_t* __restrict__ IEN, int64_t nel, const i
 // axis rays do not.  (Building them for every mesh took a third of a reference-rule call on 1.4M
 // triangles.)  set_mesh enqueues at once what the last mesh's calls used (ctx->tree_used), so that a
 // program of unbounded calls overlaps the build as before.
-int ensure_tree(sdfgpu_ctx* ctx, bool boxes) {
+static int build_tree(sdfgpu_ctx* ctx, bool boxes) {
   MeshDev& M = ctx->mesh;
   ctx->tree_used = std::max(ctx->tree_used, boxes ? 2 : 1);
   const int64_t nel = M.nel;
@@ -726,6 +726,13 @@ int ensure_tree(sdfgpu_ctx* ctx, bool boxes) {
     M.tree = 2;
   }
   return 0;
+}
+
+int ensure_tree(sdfgpu_ctx* ctx, bool boxes) {
+  const int rc = build_tree(ctx, boxes);
+  // no event covers what a failed build has enqueued: wait, so that nothing rewrites its inputs under it
+  if (rc != 0) cudaStreamSynchronize(ctx->bvh_stream);
+  return rc;
 }
 
 int mesh_upload_and_build(sdfgpu_ctx* ctx, const double* X, int64_t nnp, const int64_t* IEN, int64_t nel,
