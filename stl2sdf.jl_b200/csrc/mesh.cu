@@ -807,7 +807,11 @@ int mesh_upload_and_build(sdfgpu_ctx* ctx, const double* X, int64_t nnp, const i
   M.rho_max = ord_dbl(hbb[7]);
   M.n_weak = (int64_t)hbb[9];
   M.rho_weak = M.n_weak ? ord_dbl(hbb[8]) : 0.0;
-  if (eager) SDF_TRY(ensure_tree(ctx, eager > 1));
+  if (eager) {
+    const int rc = ensure_tree(ctx, eager > 1);
+    if (rc == SDFGPU_ERR_OUT_OF_MEMORY) ctx->err.clear();  // this mesh's calls may not need it; those that do report it
+    else SDF_TRY(rc);
+  }
   ctx->tree_used = 0;
   float ms = 0.f;
   SDF_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev[4], ctx->ev[5]));
