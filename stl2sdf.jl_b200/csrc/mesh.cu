@@ -139,6 +139,13 @@ __device__ __forceinline__ LeafTri leaf_record(const TriRec64& r, int id, double
 constexpr int kPrepThreads = 128;
 constexpr int kRecDoubles = sizeof(TriRec64) / 8, kRecStride = kRecDoubles + 1;
 static_assert(sizeof(TriRec64) % 16 == 0 && kRecStride % 2 == 1, "records are copied 16 bytes at a time");
+// A warp's stage: 32 records, or the FP32 copies as float4.
+struct __align__(16) PrepStage {
+  double d[32 * kRecStride];
+};
+static_assert(sizeof(PrepStage) % sizeof(float4) == 0 && alignof(PrepStage) >= alignof(float4) &&
+                  sizeof(PrepStage) >= 5 * 32 * sizeof(float4),
+              "the stage holds five float4 a triangle");
 __global__ void __launch_bounds__(kPrepThreads) k_prep(const double* __restrict__ X, int64_t nnp,
                                                        const int64_t* __restrict__ IEN, int64_t nel,
                                                        const unsigned long long* __restrict__ bb,
@@ -146,9 +153,9 @@ __global__ void __launch_bounds__(kPrepThreads) k_prep(const double* __restrict_
                                                        float4* __restrict__ v32, float4* __restrict__ c32,
                                                        float4* __restrict__ box32, float4* __restrict__ tri32,
                                                        unsigned long long* bad, unsigned long long* rho_ord) {
-  __shared__ double s_rec[kPrepThreads / 32][32 * kRecStride];
+  __shared__ PrepStage s_rec[kPrepThreads / 32];
   const int lane = threadIdx.x & 31;
-  double* stage = s_rec[threadIdx.x >> 5];
+  double* stage = s_rec[threadIdx.x >> 5].d;
   double ctr[3], E = 0.0;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
