@@ -218,13 +218,19 @@ __device__ __forceinline__ void bary_solve(const TriRec64& r, const d3& x, doubl
   }
 }
 
+// The box test that starts a candidate's step: whether it is passed over at the running minimum m.  Its bounds
+// are rounded at the coordinates' scale, so it can pass over a candidate that is nearer than m by less than
+// that.
+__device__ __forceinline__ bool step_skips(const TriRec64& r, const d3& p, double m) {
+  return p.x < ds(r.bmin[0], m) || p.x > da(r.bmax[0], m) || p.y < ds(r.bmin[1], m) || p.y > da(r.bmax[1], m) ||
+         p.z < ds(r.bmin[2], m) || p.z > da(r.bmax[2], m);
+}
+
 // One candidate of the reference's per-node loop (dfOnTriangularMesh.jl:104-176).  quirk = true
 // keeps the reference rule (vertices only when no edge foot improved the running minimum);
 // quirk = false evaluates the true point-triangle minimum with the same arithmetic.
 __device__ inline void tri_step64(const TriRec64& r, const d3& p, double& m, d3& proj, bool quirk) {
-  if (p.x < ds(r.bmin[0], m) || p.x > da(r.bmax[0], m)) return;
-  if (p.y < ds(r.bmin[1], m) || p.y > da(r.bmax[1], m)) return;
-  if (p.z < ds(r.bmin[2], m) || p.z > da(r.bmax[2], m)) return;
+  if (step_skips(r, p, m)) return;
   double lam[3];
   bary_solve(r, p, lam);
   const d3 v0 = rec_v(r, 0), v1 = rec_v(r, 1), v2 = rec_v(r, 2);

@@ -13,7 +13,8 @@
 // triangles whose distance can equal D (the "ties") the fold's result is the smallest of their values
 // whenever no value depends on m, or those that do cannot go below the others -- or when they share
 // one V and, in index order, some F is not below the F before it: after the earlier one m is at most its
-// F, so the later one's feet do not improve it and V is taken.  Nodes for which none of this holds, and
+// F, so the later one's feet do not improve it and V is taken.  (The ties are taken in index order with the box
+// test of the step, which decides between values a few roundings apart.)  Nodes for which none of this holds, and
 // nodes next to a triangle unfit for FP32 decisions, replay the whole fold (k_hard_*); when their candidates do
 // not fit the lists (hundreds of coincident triangles, a fan of a thousand in a large mesh), the tile fold takes
 // the call, whose work is bounded by the candidates' number.
@@ -319,7 +320,7 @@ __global__ void __launch_bounds__(128, 6) k_near_resolve(const __grid_constant__
       }
       nearest = best;
       // in ascending triangle index
-      double Vc = INFINITY, Fprev = INFINITY;
+      double Vc = INFINITY, Fprev = INFINITY, Fmin = INFINITY;
       int dependent = 0, last = -1;
       bool sure = false, one_v = true;
 #pragma unroll 1
@@ -333,6 +334,7 @@ __global__ void __launch_bounds__(128, 6) k_near_resolve(const __grid_constant__
         }
         last = tri;
         const int feat = (int)(pick >> kFeatShift);
+        if (m < kBig && step_skips(A.rec[tri], p, m)) continue;
         ++fp64;
         if (feat <= F_EDGE2 || (feat != 7 && !A.ref)) {  // face or edge: whatever m
           double d;
@@ -352,12 +354,22 @@ __global__ void __launch_bounds__(128, 6) k_near_resolve(const __grid_constant__
             sure = sure || F >= Fprev;
           }
           if (V < Vc) Vc = V;
+          Fmin = fmin(Fmin, F);
           Fprev = F;
         }
       }
-      if (dependent && m > Vc) {  // the values that depend on m can go below the others
-        if (one_v && sure) m = Vc;
-        else hard = true;
+      if (dependent) {
+        // the values that depend on m can go below the others; and where values lie closer together than the
+        // box test resolves, which of them are taken depends on the order (tol is far above that)
+        const bool apart = Fmin - Vc > tol;
+        if (m == Vc) {
+          hard = !apart;
+        } else if (m < Vc) {
+          hard = Vc - m <= tol;
+        } else {
+          hard = !(one_v && sure && apart && m - Vc > tol);
+          m = Vc;
+        }
       }
     }
     A.hidx[q] = -1;
