@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(kUnbThreads, 4) k_nearest_points(const __grid_
                                                 [&] { lane_prune<kUnbThreads>(A, L, p); });
     const bool over = mine && L.n > kKeep;
     if (ok && __any_sync(0xffffffffu, over))
-      ok = exact_search(A, s_wide[w].queue, lane, 0, p, p32, over, band_of(A, L.m), m64, proj, fp64, visits);
+      ok = exact_search(A, s_wide[w].queue, spill, lane, 0, p, p32, over, band_of(A, L.m), m64, proj, fp64, visits);
     if (mine) {
       if (!over) lane_resolve<kUnbThreads>(A, L, p, m64, proj, fp64);
       if (!ok) ++errs;

@@ -709,13 +709,26 @@ __device__ __forceinline__ bool wide_search(const P& A, WideShared& W, int* spil
   return ok;
 }
 
-// The FP64 re-search of lanes whose band overflowed (rare): a packet traversal, one LBVH node per
-// step with its two children tested per lane, where every leaf triangle within a lane's bound --
-// r0 = band of its FP32 minimum, then its FP64 minimum -- runs the FP64 step at once.
+// The FP64 re-search of lanes whose band overflowed (rare): a packet traversal, one LBVH node per step with
+// its two children tested per lane, where every leaf triangle within a lane's bound -- r0 = band of its FP32
+// minimum, then its FP64 minimum -- runs the FP64 step at once.
+//
+// It finds the smallest value, its lowest triangle index, and the next larger value.  When that is farther off
+// than roundings can matter, this is what the steps in ascending index come to.  Else (equally far triangles
+// whose values differ by a few roundings, as two beside one edge: the steps' box test decides between them by
+// their order) the steps of the triangles within tol of the smallest value are replayed in ascending index from
+// the lane's share of the warp's spilled queue, which the FP32 pass has done with.  Where there are more of them
+// than it holds (a node on the axis of a fan), the smallest value stays, which the box test could have kept from
+// being reached by a few roundings.
+constexpr int kTies = kWideSpill / 32;
 template <class P>
-__device__ __noinline__ bool exact_search(const P& A, int* stack, int lane, int rep, const d3& p, const float3& p32,
-                                          bool active, float r0, double& m64, d3& proj, uint32_t& fp64,
-                                          uint32_t& visits_out) {
+__device__ __noinline__ bool exact_search(const P& A, int* stack, int* spill, int lane, int rep, const d3& p,
+                                          const float3& p32, bool active, float r0, double& m64, d3& proj,
+                                          uint32_t& fp64, uint32_t& visits_out) {
+  int* ties = spill + lane;
+  const double tol = 1e-9 * (double)A.E + 1e-14 * (fabs(p.x) + fabs(p.y) + fabs(p.z));
+  double next = INFINITY;
+  int at = -1, n = 0;  // the triangle of m64; triangles in `ties`
   int sp = 1;
   if (lane == 0) stack[0] = 0;
   __syncwarp();
@@ -753,9 +766,24 @@ __device__ __noinline__ bool exact_search(const P& A, int* stack, int lane, int 
       const float4* v = A.lv32 + 3 * l;
       const float D = sqrtf(pt_tri_d2(p32, f3(v[0]), f3(v[1]), f3(v[2])));
       const float mq = (float)m64;
-      if (want && !(D > fminf(r0, mq + A.eD_abs + A.eD_rel * mq) + A.pad)) {
-        step64_call(A.rec, __float_as_int(A.ltri.at(0, (int)l).w) & ~kWeakTri, p, m64, proj);
-        ++fp64;
+      if (!want || D > fminf(r0, mq + A.eD_abs + A.eD_rel * mq) + A.pad) continue;
+      const int prim = __float_as_int(A.ltri.at(0, (int)l).w) & ~kWeakTri;
+      const double from = fmin(m64 + 2.0 * tol, kBig);
+      double m = from;
+      d3 x;
+      step64_call(A.rec, prim, p, m, x);
+      ++fp64;
+      if (!(m < from)) continue;
+      if (m < m64 - tol) n = 0;  // what was kept is farther
+      if (n < kTies) ties[n * 32] = prim;
+      ++n;
+      if (m < m64 || (m == m64 && prim < at)) {
+        if (m < m64) next = at < 0 ? INFINITY : m64;
+        m64 = m;
+        at = prim;
+        proj = x;
+      } else if (m > m64) {
+        next = fmin(next, m);
       }
     }
     // inner children, the far one pushed first so the near one is popped next
@@ -773,6 +801,18 @@ __device__ __noinline__ bool exact_search(const P& A, int* stack, int lane, int 
   }
   __syncwarp();
   visits_out += visits;
+  if (active && next <= m64 + tol && n <= kTies) {
+    m64 = fmin(m64 + 2.0 * tol, kBig);
+    int last = -1;
+#pragma unroll 1
+    for (int it = 0; it < n; ++it) {
+      int t = 0x7fffffff;
+      for (int q = 0; q < n; ++q)
+        if (ties[q * 32] > last && ties[q * 32] < t) t = ties[q * 32];
+      last = t;
+      step64_call(A.rec, t, p, m64, proj);
+    }
+  }
   return ok;
 }
 

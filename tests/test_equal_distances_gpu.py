@@ -40,3 +40,15 @@ def test_symmetric_grids_about_boxes(gpu_ctx, pieces, mode):
         if not np.array_equal(d, ref):
             bad.append((seed, int((d != ref).sum()), float(np.abs(d - ref).max() / h)))
     assert not bad
+
+
+@pytest.mark.parametrize("level,copies", [(0, 1), (1, 1), (2, 1), (3, 1), (0, 17), (1, 5), (2, 20)])
+def test_closest_points_of_more_ties_than_a_node_keeps(gpu_ctx, level, copies):
+    """The centre of a sphere, and the nodes around meshes of coincident triangles: the lowest index has it."""
+    V, F = synthetic.icosphere(level, jitter=0.0 if copies == 1 else 0.1, seed=level)
+    F = np.repeat(F, copies, axis=0)[np.random.default_rng(copies).permutation(copies * len(F))]
+    N = np.array([12, 12, 12])
+    gpu_ctx.set_mesh(V, F)
+    d, x = gpu_ctx.distances(np.full(3, -1.5), 0.25, N, 2, want_xp=True)
+    ref, xr, _ = oracle.distances(V, F, np.full(3, -1.5), 0.25, N, mode=2, want_xp=True)
+    assert np.array_equal(d, ref) and np.array_equal(x, xr)
