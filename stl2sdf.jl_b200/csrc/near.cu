@@ -334,19 +334,22 @@ __global__ void __launch_bounds__(128, 6) k_near_resolve(const __grid_constant__
         }
         last = tri;
         const int feat = (int)(pick >> kFeatShift);
-        if (m < kBig && step_skips(A.rec[tri], p, m)) continue;
         ++fp64;
+        // a value that the triangle's step takes unless its box test passes it over at m (never at kBig)
+        auto take = [&](double v) {
+          if (v < m && !(m < kBig && step_skips(A.rec[tri], p, m))) m = v;
+        };
         if (feat <= F_EDGE2 || (feat != 7 && !A.ref)) {  // face or edge: whatever m
           double d;
           d3 x;
           feature64(A.rec[tri], p, feat, d, x);
-          m = fmin(m, d);
+          take(d);
           continue;
         }
         double face, F, V;
         step_values(A.rec, tri, p, face, F, V);
-        if (face == face) m = fmin(m, face);
-        else if (!A.ref || !(V < F) || isinf(F)) m = fmin(m, fmin(F, V));
+        if (face == face) take(face);
+        else if (!A.ref || !(V < F) || isinf(F)) take(fmin(F, V));
         else {  // V < F: depends on m
           if (dependent++ == 0) Vc = V;
           else {
@@ -360,12 +363,14 @@ __global__ void __launch_bounds__(128, 6) k_near_resolve(const __grid_constant__
       }
       if (dependent) {
         // the values that depend on m can go below the others; and where values lie closer together than the
-        // box test resolves, which of them are taken depends on the order (tol is far above that)
+        // box test resolves, which of them are taken depends on the order (tol is far above that).  Below Vc
+        // it does not when the test passes over none of the ties at Vc: then all of them are taken as here.
         const bool apart = Fmin - Vc > tol;
         if (m == Vc) {
           hard = !apart;
         } else if (m < Vc) {
-          hard = Vc - m <= tol;
+          if (Vc - m <= tol)
+            for (int s = 0; s < left && !hard; ++s) hard = step_skips(A.rec[(unsigned)slot[s] & kTriMask], p, Vc);
         } else {
           hard = !(one_v && sure && apart && m - Vc > tol);
           m = Vc;

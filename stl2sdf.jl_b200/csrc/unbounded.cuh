@@ -158,12 +158,10 @@ __device__ __noinline__ void step64_call(const TriRec64* rec, int prim, const d3
     tri_step64(rec[prim], p, m64, proj, false);
     return;
   }
-  // (no value below kBig is skipped at kBig; the record's box need not be read then)
-  if (m64 < kBig && step_skips(rec[prim], p, m64)) return;
   double d;
   d3 x;
   feature64(rec[prim], p, feat, d, x);
-  if (d < m64) {
+  if (d < m64 && !(m64 < kBig && step_skips(rec[prim], p, m64))) {  // (no value below kBig is skipped at kBig)
     m64 = d;
     proj = x;
   }
