@@ -90,7 +90,8 @@ typedef struct sdfgpu_opts {
 typedef struct sdfgpu_stats {
   int64_t ngp;                    /* grid nodes of the call */
   int64_t nel;                    /* triangles of the mesh */
-  int64_t tile_pairs;             /* (tile, triangle) candidate pairs (0 where the scatter took the call) */
+  int64_t tile_pairs;             /* (tile, triangle) candidate pairs (0 where the scatter took the call; a batch
+                                     sums over its items, whichever way each went) */
   int64_t active_tiles;           /* tiles with at least one candidate */
   int64_t candidate_nodes;        /* nodes whose candidate set was non-empty (0 where the scatter took it) */
   int64_t fp64_evals;             /* FP64 point-triangle evaluations (near-tie band) */
@@ -106,13 +107,15 @@ typedef struct sdfgpu_stats {
   double ms_distance;             /* device time of the distance stage (ms) */
   double ms_sign;                 /* device time of the sign stage (ms) */
   double ms_mesh;                 /* device time of the last set_mesh up to the triangle records (ms); the LBVH
-                                     build runs beside the next call's distance stage */
+                                     is built when a call first needs it, or ahead beside the next call when
+                                     the last mesh's calls did */
   int64_t launches;               /* kernels of this library launched by the last call (CUB excluded) */
   int64_t mesh_launches;          /* same, for the last set_mesh */
   double ms_tiles;                /* nearest distances and near nodes of the scatter, or (tile, triangle) pair build + sort */
   double ms_fold;                 /* the near nodes' results, the tile fold kernel or the unbounded search */
   double ms_rows;                 /* axis-row hit lists (count, fill) and their flags */
-  double ms_parity;               /* the rows' parity masks and the vote */
+  double ms_parity;               /* the rows' parity masks and the vote (in the unbounded modes with their wait
+                                     for the search, which holds the GPU; likewise ms_sign) */
   double ms_vote;                 /* adaptive rays + winding */
   int64_t certified_nodes;        /* learned radius: nodes whose bounded search certified the result */
   double radius_loss;             /* final training loss of the radius network */

@@ -267,7 +267,8 @@ int run_all(sdfgpu_ctx* ctx, const GridP& g, bool want_dist, bool want_sign, int
   // The sign stage runs on its own stream, forked after the counters are cleared: its row counting
   // is enqueued first, the distance stage's lists next (its one host wait covers the row count too),
   // then the rest of the sign stage up to the vote, whose chain of small kernels is the longer one on small
-  // meshes, and the distance fold beside it.  The join precedes the combine.
+  // meshes, and the distance stage's second half beside it.  (An unbounded search is enqueued before that; its
+  // resident warps fill the GPU, so the vote then waits for them.)  The join precedes the combine.
   cudaStream_t ss = ctx->sign_stream;
   SignPlan P;
   bool forked = false;

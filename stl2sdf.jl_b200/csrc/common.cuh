@@ -259,13 +259,13 @@ int mesh_upload_and_build(sdfgpu_ctx* ctx, const double* X, int64_t nnp, const i
 int ensure_ine(sdfgpu_ctx* ctx);
 int ensure_tree(sdfgpu_ctx* ctx, bool boxes);
 // `between` (may be empty) runs once the host has waited for the stage's lists and before their use is
-// enqueued, or after an unbounded search has been.
+// enqueued, or after an unbounded search has been (whose resident warps leave it the GPU when they are done).
 int run_distances(sdfgpu_ctx* ctx, const GridP& g, int mode, int use_learned, double* d_dist, double* d_xp,
                   const std::function<int()>& between = {});
 // The reference-rule / h-bounded stage by tile lists and folds.
 int run_tiles(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, double* d_xp,
               const std::function<int()>& between = {});
-// Exact unbounded distances of a sparse grid's nodes, one thread per node (learned.cu).
+// Exact unbounded distances of a sparse grid's nodes, one warp per node (learned.cu).
 int run_nearest_points(sdfgpu_ctx* ctx, const GridP& g, double* d_dist);
 
 // The reference-rule / h-bounded distance stage in parts (distance.cu), so a batch can run the folds

@@ -25,7 +25,9 @@
 //      fallback on the LBVH.  Every other node with empty C(p) has a result > h, so it is h.
 //
 // SDFGPU_MODE_EXACT uses the same tiles with lists of the triangles whose box lies within h of
-// the tile; SDFGPU_MODE_UNBOUNDED is a per-node LBVH nearest-triangle search without the clamp.
+// the tile; SDFGPU_MODE_UNBOUNDED is the nearest-triangle search of a warp per brick of nodes over the LBVH
+// (unbounded.cuh), without the clamp.  Calls of both clamped modes whose triangles are small against the cell
+// go to the scatter (near.cu), which hands back those that it cannot finish.
 #include <cub/cub.cuh>
 #include <cuda_fp16.h>
 
@@ -350,7 +352,6 @@ __global__ void __launch_bounds__(256) k_tile_fold_multi(const FoldArgs* __restr
   }
 }
 
-// Sort keys of the tile order: list length saturated to 16 bits, and the tile index.
 // The nodes of tiles without candidates: a node with an empty candidate set clamps to h
 // (dfOnTriangularMesh.jl:202-206; the 3-nearest-vertex fallback, when the mesh needs it, runs after
 // and finds these nodes by their status 0).  One coalesced pass over the nodes instead of a fold
@@ -372,6 +373,7 @@ __global__ void k_fill_empty(GridP g, const int32_t* __restrict__ tile_cnt, doub
   }
 }
 
+// Sort keys of the tile order: list length saturated to 16 bits, and the tile index.
 __global__ void k_tile_keys(const int32_t* __restrict__ cnt, int64_t n, uint16_t* __restrict__ key,
                             int32_t* __restrict__ idx) {
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
@@ -621,8 +623,8 @@ void unb_tree(sdfgpu_ctx* ctx, const GridP& g, const int32_t b[3], double* d_dis
   }
 }
 
-// The unbounded search's arguments for grid g on the current mesh, with the learned radius of every brick when use_learned and the network's bound
-// is on; the context stream waits for the LBVH and its oriented boxes.
+// The unbounded search's arguments for grid g on the current mesh, with the learned radius of every brick when
+// use_learned and the network's bound is on; the context stream waits for the LBVH and its oriented boxes.
 int unb_setup(sdfgpu_ctx* ctx, const GridP& g, int use_learned, double* d_dist, double* d_xp, UnbArgs& A) {
   SDF_TRY(ensure_tree(ctx, true));
   SDF_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->ev_obb, 0));  // the search walks the LBVH and its oriented boxes
@@ -705,8 +707,6 @@ int run_tiles(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, double*
   return 0;
 }
 
-// Tile lists of the reference rule (or the h-bounded exact mode) and the fold's arguments; when the
-// mesh needs the 3-nearest-vertex fallback, its incidence lists, band flags and arguments too.
 // A batch item's unbounded (or learned) search, prepared for the multi-mesh launch: its arguments
 // and, in the learned mode, the radius of every brick, in the item's own buffers.
 int unb_prepare(sdfgpu_ctx* ctx, const GridP& g, int use_learned, double* d_dist, double* d_xp, DistPlan& Pl) {
@@ -722,6 +722,8 @@ int unb_prepare(sdfgpu_ctx* ctx, const GridP& g, int use_learned, double* d_dist
   return 0;
 }
 
+// Tile lists of the reference rule (or the h-bounded exact mode) and the fold's arguments; when the
+// mesh needs the 3-nearest-vertex fallback, its incidence lists, band flags and arguments too.
 int dist_prepare(sdfgpu_ctx* ctx, const GridP& g, int mode, double* d_dist, double* d_xp, DistPlan& Pl,
                  int use_learned) {
   if (mode == SDFGPU_MODE_UNBOUNDED) return unb_prepare(ctx, g, use_learned, d_dist, d_xp, Pl);

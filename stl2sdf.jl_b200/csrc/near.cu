@@ -118,10 +118,10 @@ __device__ __forceinline__ float node32(const NearArgs& A, int a, float x, float
 // largest count, about half of the box's nodes.  The first scatter keeps the bits of the pairs that were
 // within the band of the node's minimum at that time; it only falls, so the second needs no others: about
 // two pairs a triangle instead of thirty.  Triangles of more than 64 nodes go through 64 at a time, both
-// times.  Bound: instruction issue, about 70 a pair.  Both scatters, 1.4M triangles of which a third of a
-// node is near, and 5.8M: 0.43 -> 0.27 and 1.9 -> 1.11 ms (B200) against all
-// nodes of the box in both.
-// 64 registers (8 blocks an SM) for the latency of the triangles' reads: 10% below the compiler's 80.
+// times.  Bound: instruction issue, about 70 a pair, and the latency of the triangles' reads, for which the
+// registers are limited to 64 (8 blocks an SM).  Both scatters of 1.4M and of 5.8M triangles (B200): 0.43 and
+// 1.9 ms when each took all nodes of the boxes, 0.30 and 1.22 ms with the masks, 0.27 and 1.11 ms at 64 registers
+// instead of the compiler's 80.
 template <bool kFill>
 __global__ void __launch_bounds__(128, 8) k_near_scatter(const __grid_constant__ NearArgs A) {
   const GridP& g = A.g;

@@ -620,7 +620,7 @@ int train_radius(sdfgpu_ctx* ctx, int coarse_n, int steps, int batch, float lr, 
   SDF_TRY(make_grid(ctx, o, h, N, g));
   double* dd;
   SDF_TRY(scratch_t(ctx, "mlp_dist", (size_t)ngp, &dd));
-  // the exact unbounded distances of the coarse grid (sparse nodes: one nearest-first walk per node)
+  // the exact unbounded distances of the coarse grid (sparse nodes: a warp per node)
   SDF_TRY(ensure_tree(ctx, true));
   SDF_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_obb, 0));
   SDF_TRY(run_nearest_points(ctx, g, dd));

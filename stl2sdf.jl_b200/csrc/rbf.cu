@@ -129,7 +129,8 @@ __device__ __forceinline__ void cg_reduce(double acc, double* partial, unsigned*
 // farthest offset along an axis with a factor above the cut-off), and a thread walks kMZ nodes along
 // z with its x and y factors in registers; products below the cut-off, and all outside the grid (factor
 // 0), add nothing.  Same terms and order per node as the form that read 2 x 81 values from memory and
-// formed u_new for each: 130 -> 32 us on 590k nodes.  Bound: the FP64 products and their conversion.
+// formed u_new for each: 130 -> 32 us on 590k nodes.  Bound: instruction issue (60% of the slots) and the
+// conversions of the FP64 products (48% of their pipe); FP64 29%, shared memory 22%.
 template <int RE>
 __global__ void __launch_bounds__(kRbfThreads) k_rbf_matvec(Axis3 ax, const double* __restrict__ kt, int R,
                                                             double thr, const float* __restrict__ r,
