@@ -82,6 +82,20 @@ def test_fans(gpu_ctx, fan, rest, mode):
     assert (st["band_nodes"] > 0) == (st["tile_pairs"] == 0)
 
 
+def test_slabs_that_the_tile_fold_takes_over(gpu_ctx):
+    V, F, h = sphere(4, 4 * SLOTS)
+    o = V.min(0) - 2.9 * h
+    N = np.ceil((V.max(0) - o) / h).astype(np.int64) + 2
+    gpu_ctx.set_mesh(V, F)
+    whole, dist, sign, _ = gpu_ctx.sdf(o, h, N, 0, want_parts=True)
+    assert gpu_ctx.stats()["tile_pairs"] > 0
+    n = int((N[0] + 1) * (N[1] + 1))
+    for k0, k1 in ((0, 4), (5, 20), (21, int(N[2]))):
+        part = gpu_ctx.sdf_slab(o, h, N, k0, k1, 0, want_parts=True)
+        for a, b in zip(part, (whole, dist, sign)):
+            assert np.array_equal(a, b[n * k0:n * (k1 + 1)])
+
+
 def test_the_call_after_it(gpu_ctx):
     """A call that the tile fold took over leaves nothing behind for the next one."""
     V, F, h = sphere(4, 4 * SLOTS)
