@@ -169,12 +169,15 @@ int make_grid(sdfgpu_ctx* ctx, const double origin[3], double h, const int64_t N
   g.h = h;
   g.ngp = g.n[0] * g.n[1] * g.n[2];
   g.ntiles = g.nt[0] * g.nt[1] * g.nt[2];
-  double E = M.E;
+  double E = M.E, far = 0.0;
   for (int a = 0; a < 3; ++a) {
     const double lo = origin[a], hi = origin[a] + h * (double)N[a];
     E = std::max(E, std::max(std::fabs(lo - M.center[a]), std::fabs(hi - M.center[a])));
+    far = std::max(far, std::max(std::fabs(M.center[a]), std::max(std::fabs(lo), std::fabs(hi))));
   }
-  g.E = E;
+  // coordinates more than 1e9 extents from the origin round at a scale that counts beside the grid's
+  g.E = std::max(E, 1e-9 * far);
+  g.pad = std::max(1e-6, 1e-15 * (far + E) / h);
   return 0;
 }
 

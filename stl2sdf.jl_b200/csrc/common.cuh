@@ -71,6 +71,7 @@ struct GridP {
   int64_t nt[3];    // tiles per axis
   int64_t ntiles;
   int64_t k0 = 0;   // z index of local layer 0 in the full grid (a z-slab call), else 0
+  double pad = 1e-6;  // what covers the roundings of a coordinate's place in cells
 };
 
 // Node (i, j, k) of the call in FP64, k local to the slab: origin + h * (global index), the

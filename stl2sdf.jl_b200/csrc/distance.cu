@@ -55,7 +55,7 @@ __device__ __forceinline__ void node_ijk(const GridP& g, int64_t lin, int64_t& i
 // Index range [lo, hi] of the nodes whose coordinate along axis a can lie in [x0, x1].
 __device__ __forceinline__ bool axis_range(const GridP& g, int a, double x0, double x1, int64_t& lo, int64_t& hi) {
   const double shift = (double)gidx(g, a, 0);
-  double f0 = (x0 - g.o[a]) / g.h - shift - 1e-6, f1 = (x1 - g.o[a]) / g.h - shift + 1e-6;
+  double f0 = (x0 - g.o[a]) / g.h - shift - g.pad, f1 = (x1 - g.o[a]) / g.h - shift + g.pad;
   f0 = fmax(f0, -1.0);
   f1 = fmin(f1, (double)g.N[a] + 1.0);
   if (!(f0 <= f1)) return false;

@@ -93,12 +93,12 @@ struct NearArgs {
   int64_t* counters;
 };
 
-// Nodes of axis a with coordinate in [x0, x1] (grown by 1e-6 cells), as in the tile lists.
+// Nodes of axis a with coordinate in [x0, x1] (grown by the grid's pad), as in the tile lists.
 __device__ __forceinline__ bool near_range(const NearArgs& A, int a, double x0, double x1, int& lo, int& hi) {
   const GridP& g = A.g;
   const double shift = (double)gidx(g, a, 0);
-  const double f0 = fmax((x0 - g.o[a]) * A.ih - shift - 1e-6, -1.0);
-  const double f1 = fmin((x1 - g.o[a]) * A.ih - shift + 1e-6, (double)g.N[a] + 1.0);
+  const double f0 = fmax((x0 - g.o[a]) * A.ih - shift - g.pad, -1.0);
+  const double f1 = fmin((x1 - g.o[a]) * A.ih - shift + g.pad, (double)g.N[a] + 1.0);
   if (!(f0 <= f1)) return false;
   lo = max((int)ceil(f0), 0);
   hi = (int)min((int64_t)floor(f1), g.N[a]);

@@ -159,7 +159,7 @@ __device__ __forceinline__ int row_test32(const TriRec64& r, double ob, double o
 
 __device__ __forceinline__ bool axis_range2(const GridP& g, int a, double x0, double x1, int64_t& lo, int64_t& hi) {
   const double shift = (double)gidx(g, a, 0);
-  double f0 = (x0 - g.o[a]) / g.h - shift - 1e-6, f1 = (x1 - g.o[a]) / g.h - shift + 1e-6;
+  double f0 = (x0 - g.o[a]) / g.h - shift - g.pad, f1 = (x1 - g.o[a]) / g.h - shift + g.pad;
   f0 = fmax(f0, -1.0);
   f1 = fmin(f1, (double)g.N[a] + 1.0);
   if (!(f0 <= f1)) return false;
