@@ -37,8 +37,6 @@ class TriangularMesh:
         self.nen = 3
         self.nel = self._IENrows.shape[0]
         self._INE = None
-        # what a context knows its resident mesh by; it keeps this object, so no other mesh's can equal it
-        self._key = object()
 
     @property
     def X(self):
@@ -142,10 +140,9 @@ def mesh_edge_statistics(mesh: TriangularMesh, device: int = 0) -> dict:
     """Edge-length statistics of the mesh (calculate_edge_distances + analyze_mesh,
     Grid_setup.jl:28-102), computed on the GPU: shortest, longest, mean and median edge, and the mean
     edge of the triangles with the smallest / largest edge sum (smallest_index / largest_index,
-    0-based, the first on ties).  Uploads the mesh to the device's default context, where the
-    distance and sign calls that follow find it."""
+    0-based, the first on ties).  Uploads the mesh to the device's default context."""
     ctx = _native.default_context(device)
-    ctx.set_mesh(mesh.vertex_rows(), mesh.triangle_rows(), key=mesh._key)
+    ctx.set_mesh(mesh.vertex_rows(), mesh.triangle_rows())
     return ctx.mesh_edge_stats()
 
 

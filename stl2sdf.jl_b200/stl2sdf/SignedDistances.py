@@ -33,8 +33,10 @@ def _check_points(grid: Grid, points) -> None:
 
 
 def _ctx(mesh: TriangularMesh, device: int = 0):
+    # uploaded by every call, so that changes of the arrays count: 0.08 ms for 14k triangles and 3 ms for 1.4M (B200),
+    # as long as comparing them with a copy of what was uploaded last would take
     ctx = _native.default_context(device)
-    ctx.set_mesh(mesh.vertex_rows(), mesh.triangle_rows(), key=mesh._key)
+    ctx.set_mesh(mesh.vertex_rows(), mesh.triangle_rows())
     return ctx
 
 

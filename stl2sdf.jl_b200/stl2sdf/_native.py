@@ -214,7 +214,7 @@ class Context:
 
     def set_mesh(self, X, IEN, key=None):
         """X: (nnp, 3) float64; IEN: (nel, 3) int64 1-based (vertex-major = 3 x n column-major).
-        key: returns at once when it is the resident mesh's."""
+        key: returns at once when it is the resident mesh's (the caller vouches for the arrays)."""
         if key is not None and key == self._mesh_key:
             return
         X = np.ascontiguousarray(X, np.float64).reshape(-1, 3)
